@@ -9,11 +9,25 @@
 // toward the smaller index).  Ranking the roots into labels by rows
 // (core/passes.py:933-950) is bookkeeping done by the caller.
 //
+// Unions alone are latency-bound: every thread walks parent chains that the
+// others are still building and retries on the roots that all of them want
+// (243 us for the 300k unions of a 400k-worker panel, 281 us on the 5M-worker
+// one; a year dimension's ten roots see three million unions).  So the trees
+// are first grown by rounds without walks or retries -- every pair hooks the
+// larger of its two roots under the smaller by one atomicMin, then all trees
+// are flattened -- over a sample of the groups, enough for the giant component
+// to close (three rounds; a sample of one window in four still leaves a firm
+// about four neighbours); the last pass unites what is left, and nearly every
+// pair finds one common root with two loads.  One cooperative launch does all
+// of it, grid barriers between the phases.
 // Normalisation: core/solve.py:383-399 `_normalize`.  The first dimension's
 // effects get obs-weighted mean zero within each component, every further
 // dimension obs-weighted mean zero overall.  Within-component sums are
-// combined per warp (lanes with the same root, __match_any_sync) before one
-// atomic per root, so the giant component does not see 500k atomics.
+// carried along each thread's walk and combined per warp (lanes with the same
+// root) before one atomic per root: the giant component of 500k levels sees
+// about a thousand atomics a column.
+#include <atomic>
+
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -49,13 +63,6 @@ __device__ __forceinline__ int32_t root_of(const int32_t *parent, int32_t x)
     return x;
 }
 
-__global__ void __launch_bounds__(kThreads) k_init(int32_t *parent, int64_t n)
-{
-    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * kThreads)
-        parent[i] = (int32_t)i;
-}
-
 // link a and b: the larger root under the smaller (bounded retries)
 __device__ __forceinline__ void unite(int32_t *parent, int32_t a, int32_t b, unsigned *status)
 {
@@ -67,91 +74,135 @@ __device__ __forceinline__ void unite(int32_t *parent, int32_t a, int32_t b, uns
         const int32_t hi = a > b ? a : b, lo = a > b ? b : a;
         const int32_t old = atomicCAS(parent + hi, hi, lo);
         if (old == hi) return;
-        a = hi;         // hi gained a parent meanwhile: retry from there
+        a = old;        // hi gained this parent meanwhile: retry from there
         b = lo;
     }
 }
 
+// hook the larger level under the smaller where that lowers its parent
+__device__ __forceinline__ void hook(int32_t *parent, int32_t a, int32_t b)
+{
+    const int32_t hi = a > b ? a : b, lo = a > b ? b : a;
+    if (parent[hi] > lo) atomicMin(parent + hi, lo);
+}
+
+struct CompArgs {
+    const int64_t *starts;
+    int64_t G;
+    const uint32_t *codes;
+    int D, col;
+    int64_t nlev;
+    int32_t *parent;
+    unsigned *status;
+    unsigned long long *n_roots;
+    GridBarrier bar;
+    int sample;             // the rounds take every sample-th window
+};
+
+constexpr int kCompThreads = 512;
+constexpr int kRounds = 3;
+
 // The levels (dimension col) of each group joined into one component: a
-// warp takes 32 groups, reads their cells coalesced (one per lane, 32 at a
-// time) and joins each cell's level with the previous cell's of the same
-// group where they differ -- a chain over the group, which connects what the
-// reference's star over the group's first level connects (every root is the
-// component's smallest level either way).
-__global__ void __launch_bounds__(kThreads) k_union(const int64_t *starts, int64_t G,
-                                                    const uint32_t *codes, int D, int col,
-                                                    int64_t nlev, int32_t *parent,
-                                                    unsigned *status)
+// warp takes a window of 32 groups, reads their cells coalesced (one per lane,
+// 32 at a time, the next 32 in flight) and calls join(prev, c) for each cell's
+// level and the previous cell's of the same group where they differ -- a chain
+// over the group, which connects what the reference's star over the group's
+// first level connects (every root is the component's smallest level either
+// way).
+template <typename F>
+__device__ __forceinline__ void walk_pairs(const CompArgs &a, int sample, F join)
 {
     const int lane = threadIdx.x & 31;
-    const int64_t wid = ((int64_t)blockIdx.x * kThreads + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * kThreads) >> 5;
-    for (int64_t g0 = wid * 32; g0 < G; g0 += nw * 32) {
-        const int ng = (int)min((int64_t)32, G - g0);
-        const int64_t gend = starts[g0 + ng];
-        const int64_t st = lane < ng ? starts[g0 + lane] : gend;   // this lane's group start
-        for (int64_t base = starts[g0]; base < gend; base += 32) {
+    const int64_t wid = ((int64_t)blockIdx.x * kCompThreads + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * kCompThreads) >> 5;
+    for (int64_t g0 = wid * 32 * sample; g0 < a.G; g0 += nw * 32 * sample) {
+        const int ng = (int)min((int64_t)32, a.G - g0);
+        const int64_t gend = a.starts[g0 + ng];
+        const int64_t st = lane < ng ? a.starts[g0 + lane] : gend;   // this lane's group start
+        int64_t base = __shfl_sync(0xffffffffu, st, 0);
+        uint32_t next = base + lane < gend ? a.codes[(base + lane) * a.D + a.col] : 0u;
+        uint32_t last = 0;                  // the code before the chunk
+        for (; base < gend; base += 32) {
+            const uint32_t c = next;
+            const int64_t i = base + lane;
+            if (i + 32 < gend) next = a.codes[(i + 32) * a.D + a.col];
             const bool in = lane < ng && st >= base && st < base + 32;
             const unsigned heads = __reduce_or_sync(0xffffffffu, in ? 1u << (int)(st - base) : 0u);
-            const int64_t i = base + lane;
             const bool valid = i < gend;
-            uint32_t c = valid ? codes[i * D + col] : 0u;
             uint32_t prev = __shfl_up_sync(0xffffffffu, c, 1);
-            if (lane == 0 && valid && i > 0) prev = codes[(i - 1) * D + col];
+            if (lane == 0) prev = last;     // a window begins with a head
+            last = __shfl_sync(0xffffffffu, c, 31);
             const bool head = (heads >> lane) & 1u;
-            if (valid && (int64_t)c >= nlev) atomicCAS(status, 0u, (unsigned)HDFE_ERR_BAD_CODE);
-            if (!valid || head || c == prev || (int64_t)c >= nlev || (int64_t)prev >= nlev)
+            if (valid && (int64_t)c >= a.nlev) atomicCAS(a.status, 0u, (unsigned)HDFE_ERR_BAD_CODE);
+            if (!valid || head || c == prev || (int64_t)c >= a.nlev || (int64_t)prev >= a.nlev)
                 continue;
-            unite(parent, (int32_t)prev, (int32_t)c, status);
+            join((int32_t)prev, (int32_t)c);
         }
     }
 }
 
-__global__ void __launch_bounds__(kThreads) k_flatten(int32_t *parent, int64_t n,
-                                                      unsigned long long *n_roots)
+__global__ void __launch_bounds__(kCompThreads, 2) k_components(CompArgs a)
 {
+    const int64_t t0 = (int64_t)blockIdx.x * kCompThreads + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * kCompThreads;
+    int32_t *parent = a.parent;
+    for (int64_t i = t0; i < a.nlev; i += step) parent[i] = (int32_t)i;
+    if (!a.bar.sync()) return;
+    for (int r = 0; r < kRounds; r++) {
+        walk_pairs(a, a.sample, [&](int32_t x, int32_t y) {
+            const int32_t px = parent[x], py = parent[y];
+            if (px != py) hook(parent, px, py);
+        });
+        if (!a.bar.sync()) return;
+        for (int64_t i = t0; i < a.nlev; i += step) parent[i] = root_of(parent, (int32_t)i);
+        if (!a.bar.sync()) return;
+    }
+    walk_pairs(a, 1, [&](int32_t x, int32_t y) {
+        if (parent[x] != parent[y]) unite(parent, x, y, a.status);
+    });
+    if (!a.bar.sync()) return;
     unsigned long long roots = 0;
-    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * kThreads) {
+    for (int64_t i = t0; i < a.nlev; i += step) {
         const int32_t r = root_of(parent, (int32_t)i);
         parent[i] = r;
         roots += (r == (int32_t)i);
     }
     roots = warp_sum(roots);
-    if ((threadIdx.x & 31) == 0 && roots) atomicAdd(n_roots, roots);
+    if ((threadIdx.x & 31) == 0 && roots) atomicAdd(a.n_roots, roots);
 }
 
 // ------------------------------------------------------------ normalise
 
-// sums per root: cw[root] += w, cs[root, j] += w * Gamma[l, j]
+// Sums per root: column j of the grid's second dimension, cw[root] += w (j 0)
+// or cs[root, j - 1] += w * Gamma[l, j - 1].
 __global__ void __launch_bounds__(kThreads) k_comp_sums(const int32_t *root, const double *w,
                                                         const double *gamma, int64_t nl, int m,
                                                         double *cw, double *cs)
 {
-    __shared__ double s_stage[kThreads];
-    const int lane = threadIdx.x & 31;
-    double *stage = s_stage + (threadIdx.x & ~31);
-    for (int64_t base = (int64_t)blockIdx.x * kThreads; base < nl;
-         base += (int64_t)gridDim.x * kThreads) {
-        const int64_t l = base + threadIdx.x;
-        const bool valid = l < nl;
-        const int32_t r = valid ? root[l] : -1;
-        const unsigned peers = __match_any_sync(0xffffffffu, r);
-        const bool leader = valid && lane == __ffs(peers) - 1;
-        const double wl = valid ? w[l] : 0.0;
-        // the peers' values summed in lane order by their leader
-        for (int j = -1; j < m; j++) {
-            stage[lane] = j < 0 ? wl : (valid ? wl * gamma[l * m + j] : 0.0);
-            __syncwarp();
-            if (leader) {
-                double acc = 0.0;
-                for (unsigned p = peers; p; p &= p - 1) acc += stage[__ffs(p) - 1];
-                if (j < 0) atomicAdd(cw + r, acc);
-                else atomicAdd(cs + (int64_t)r * m + j, acc);
-            }
-            __syncwarp();
+    const int j = (int)blockIdx.y - 1;
+    auto add = [&](int32_t r, double v) {
+        atomicAdd(j < 0 ? cw + r : cs + (int64_t)r * m + j, v);
+    };
+    int32_t at = -1;                // the root of the carried sum
+    double sum = 0.0;
+    for (int64_t l = (int64_t)blockIdx.x * kThreads + threadIdx.x; l < nl;
+         l += (int64_t)gridDim.x * kThreads) {
+        const int32_t r = root[l];
+        if (r != at) {
+            if (at >= 0) add(at, sum);
+            at = r;
+            sum = 0.0;
         }
+        sum += j < 0 ? w[l] : w[l] * gamma[l * m + j];
     }
+    // the peers' sums added in lane order
+    const unsigned peers = __match_any_sync(0xffffffffu, at);
+    double total = 0.0;
+    for (int q = 0; q < 32; q++) {
+        const double v = __shfl_sync(0xffffffffu, sum, q);
+        if ((peers >> q) & 1u) total += v;
+    }
+    if (at >= 0 && (int)(threadIdx.x & 31) == __ffs(peers) - 1) add(at, total);
 }
 
 __global__ void __launch_bounds__(kThreads) k_comp_apply(const int32_t *root, const double *cw,
@@ -208,6 +259,26 @@ __global__ void __launch_bounds__(kThreads) k_dim_apply(const double *part, int 
         for (int j = 0; j < m; j++) gamma[l * m + j] -= s_mean[j];
 }
 
+// From this many windows of 32 groups the rounds take one in four: below, a
+// window a warp is one wave and sampling saves nothing.
+constexpr int64_t kSampleFrom = 16384;
+
+// CTAs of k_components that the current device holds at once (0: an error)
+int64_t resident_ctas()
+{
+    static std::atomic<int> known[64];
+    int dev = 0, per = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
+    if (dev >= 0 && dev < 64 && (per = known[dev].load()) > 0) return per;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_components, kCompThreads, 0) !=
+            cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return 0;
+    per *= sms;
+    if (dev >= 0 && dev < 64) known[dev].store(per);
+    return per;
+}
+
 inline unsigned grid_for(int64_t n)
 {
     int64_t b = (n + kThreads - 1) / kThreads;
@@ -232,15 +303,28 @@ extern "C" int hdfe_components(const int64_t *starts, int64_t n_groups, const ui
         !n_components || !workspace || workspace_bytes < 256)
         return hdfe_set_arg_error("hdfe_components: bad argument");
     cudaStream_t s = (cudaStream_t)stream;
-    unsigned *status = (unsigned *)workspace;
+    // status, the barrier's three words (its error word is the status) and the count
+    unsigned *status = (unsigned *)workspace + 2;
     unsigned long long *roots = (unsigned long long *)((char *)workspace + 64);
     HDFE_CUDA_TRY(cudaMemsetAsync(workspace, 0, 128, s));
-    graph::k_init<<<graph::grid_for(n_levels), graph::kThreads, 0, s>>>(root, n_levels);
-    graph::k_union<<<graph::grid_for(n_groups), graph::kThreads, 0, s>>>(
-        starts, n_groups, codes, D, col, n_levels, root, status);
-    graph::k_flatten<<<graph::grid_for(n_levels), graph::kThreads, 0, s>>>(root, n_levels, roots);
+    graph::CompArgs a{starts, n_groups, codes, D, col, n_levels, root, status, roots,
+                      GridBarrier{(unsigned *)workspace}, 1};
+    const int64_t windows = (n_groups + 31) / 32;
+    if (windows >= graph::kSampleFrom) a.sample = 4;
+    const int64_t most = graph::resident_ctas();
+    if (most < 1) return hdfe_set_cuda_error(cudaGetLastError());
+    // a warp per window and eight levels a thread fill the grid of small panels,
+    // whose barriers then wait for fewer CTAs
+    int64_t need = (windows * 32 + graph::kCompThreads - 1) / graph::kCompThreads;
+    const int64_t by_level = (n_levels + 8 * graph::kCompThreads - 1) / (8 * graph::kCompThreads);
+    if (need < by_level) need = by_level;
+    if (need < 1) need = 1;
+    void *args[] = {&a};
+    HDFE_CUDA_TRY(cudaLaunchCooperativeKernel((const void *)graph::k_components,
+                                              dim3((unsigned)(need < most ? need : most)),
+                                              dim3(graph::kCompThreads), args, 0, s));
     HDFE_CUDA_TRY(cudaGetLastError());
-    hdfe_add_launches(3);
+    hdfe_add_launches(1);
     // n_components[0] = roots, n_components[1] = status
     HDFE_CUDA_TRY(cudaMemcpyAsync(n_components, roots, 8, cudaMemcpyDeviceToDevice, s));
     HDFE_CUDA_TRY(cudaMemsetAsync(n_components + 1, 0, 8, s));
@@ -269,8 +353,9 @@ extern "C" int hdfe_normalize(double *gamma, int32_t m, int32_t D, const int64_t
     double *cs = cw + n0;
     double *part = cs + n0 * m;
     HDFE_CUDA_TRY(cudaMemsetAsync(cw, 0, n0 * (1 + (int64_t)m) * 8, s));
-    graph::k_comp_sums<<<graph::grid_for(n0), graph::kThreads, 0, s>>>(root, obs, gamma, n0, m,
-                                                                       cw, cs);
+    const unsigned nc = graph::grid_for(n0) < 148 ? graph::grid_for(n0) : 148;
+    graph::k_comp_sums<<<dim3(nc, 1 + m), graph::kThreads, 0, s>>>(root, obs, gamma, n0, m, cw,
+                                                                   cs);
     graph::k_comp_apply<<<graph::grid_for(n0), graph::kThreads, 0, s>>>(root, cw, cs, n0, m,
                                                                         gamma);
     int64_t off = n0;
