@@ -7,13 +7,13 @@
 //
 // The vectors being projected are Rademacher draws regenerated from (seed,
 // row ordinal, draw index) by splitmix64 in registers -- bit-identical to
-// `_nb_rademacher`, never stored -- or explicit row vectors (the covariates
-// themselves, for the Schur border).  Rows come grouped by the streamed
-// dimension; a sub-warp of Bp lanes (Bp = the draw count rounded up to 8, 16
-// or 32) takes one group, lane j one draw.  The group's rows are staged 32 at
-// a time in shared memory (codes, covariates; weights in registers), loaded
-// lane-parallel; the draws' signs of a group's first chunk are kept as bits
-// between its two passes.
+// `_nb_rademacher`, never stored (draws.cuh: the kernels of every leave-out
+// block) -- or explicit row vectors (the covariates themselves, for the Schur
+// border: the kernels here).  Rows come grouped by the streamed dimension; a
+// sub-warp of Bp lanes (Bp = the vector count rounded up to 8, 16 or 32) takes
+// one group, lane j one vector.  The group's rows are staged 32 at a time in
+// shared memory (codes, covariates; weights in registers), loaded
+// lane-parallel.
 //   center   acc[level, j] += w_i (R_ij - Rbar_gj)  over the group's rows, for
 //            each non-streamed dimension, summed over each run of rows with
 //            equal codes and added once per run; acc_x[c, j] += X_ic w_i (R_ij
@@ -27,66 +27,12 @@
 //            shared-memory transpose: lane t sums row t).
 #include <cuda_runtime.h>
 
-#include "common.cuh"
+#include "rows.cuh"
 
 namespace hdfe {
 namespace rows {
 
 constexpr int kThreads = 256;
-constexpr int kMaxCov = 8;
-
-__device__ __forceinline__ double rademacher(uint64_t seed, int64_t row, int64_t draw)
-{
-    uint64_t x = seed ^ ((uint64_t)row * 0x9E3779B97F4A7C15ull) ^
-                 ((uint64_t)draw * 0xBF58476D1CE4E5B9ull);
-    x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
-    x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
-    x = x ^ (x >> 31);
-    return (x >> 63) == 0 ? 1.0 : -1.0;
-}
-
-struct Args {
-    const int64_t *starts;      // (G+1) row boundaries of the groups
-    int64_t G;
-    const uint32_t *codes;      // (N, D)
-    int D;
-    int64_t offs[HDFE_MAX_DIMS];
-    int64_t nlev[HDFE_MAX_DIMS];
-    int small[HDFE_MAX_DIMS];
-    int64_t soff[HDFE_MAX_DIMS];
-    int64_t n_small;
-    int64_t L;
-    const double *w;            // (N) or null (ones)
-    const double *X;            // (N, c) covariates or null
-    int c;
-    const double *R;            // (N, B) explicit vectors, or null: Rademacher
-    uint64_t seed;
-    int64_t first_draw, ordinal0;
-    int B, Bp;
-    int sqrt_weights;
-    // center
-    double *acc, *acc_x, *squares;
-    // project
-    const double *U, *C;        // (L, B), (c, B)
-    double *out;                // (N, B) or null
-    double *moments;            // (5, N) or null
-    int64_t N;
-    unsigned *status;
-};
-
-// The sign of `rademacher` from precomputed row and draw terms: the last
-// step of splitmix64 (x ^= x >> 31) leaves bit 63 alone, so the draw is -1
-// exactly when bit 63 is set before it.
-__device__ __forceinline__ bool rad_negative(uint64_t seed, uint64_t rterm, uint64_t dterm)
-{
-    uint64_t x = seed ^ rterm ^ dterm;
-    x = (x ^ (x >> 30)) * 0xBF58476D1CE4E5B9ull;
-    x = (x ^ (x >> 27)) * 0x94D049BB133111EBull;
-    return (x >> 63) != 0;
-}
-
-constexpr uint64_t kRowMul = 0x9E3779B97F4A7C15ull, kDrawMul = 0xBF58476D1CE4E5B9ull;
-constexpr int kPassThreads = 128;
 
 // Per sub-warp staging of a chunk of up to BP rows: codes (BP x D) and
 // covariates (BP x c), loaded lane-parallel (lane t: row i0 + t) and read by
@@ -96,22 +42,6 @@ struct Chunk {
     static constexpr int kBytes = BP * (HDFE_MAX_DIMS * 4 + kMaxCov * 8);
     uint32_t *codes;    // [BP][D]
     double *x;          // [BP][c]
-};
-
-// a sub-warp of BP lanes: lane j holds draw j of the block (on: j < B)
-template <int BP>
-struct Lanes {
-    int lane, j, sub;
-    unsigned mask;
-    bool on;
-    __device__ Lanes(int B)
-    {
-        lane = threadIdx.x & 31;
-        j = lane % BP;
-        sub = lane / BP;
-        mask = BP == 32 ? 0xffffffffu : (((1u << BP) - 1u) << (sub * BP));
-        on = j < B;
-    }
 };
 
 // Load rows [i0, i0 + n) of the group into the chunk (lane t: row i0 + t):
@@ -162,17 +92,11 @@ __device__ __forceinline__ void take_codes(const Args &a, const uint32_t *codes,
     }
 }
 
-__device__ __forceinline__ double inv_root(const Args &a, double w)
-{
-    return a.sqrt_weights ? (w > 0.0 ? 1.0 / sqrt(w) : 0.0) : 1.0;
-}
-
-// `_nb_center_rows` for one sub-warp of BP lanes per group (lane j: draw j).
-// Pass 1 over the group's rows: sum w, sum w r, sum w r^2, with the draws'
-// signs kept as bits for the group's first chunk; pass 2: v = w (r - mean)
-// summed over each run of rows with equal codes and added once per run to
-// every dimension's level (shared-memory copies for small dimensions), and
-// the covariate block per row.
+// `_nb_center_rows` for explicit vectors R, one sub-warp of BP lanes per group
+// (lane j: vector j).  Pass 1 over the group's rows: sum w, sum w r, sum w
+// r^2; pass 2: v = w (r - mean) summed over each run of rows with equal codes
+// and added once per run to every dimension's level (shared-memory copies for
+// small dimensions), and the covariate block per row.
 template <int BP>
 __global__ void __launch_bounds__(kPassThreads) k_center(Args a)
 {
@@ -187,7 +111,6 @@ __global__ void __launch_bounds__(kPassThreads) k_center(Args a)
     ch.x = reinterpret_cast<double *>(s_chunks + subw * Chunk<BP>::kBytes + BP * HDFE_MAX_DIMS * 4);
     for (int64_t k = threadIdx.x; k < a.n_small * a.B; k += kPassThreads) s_acc[k] = 0.0;
     __syncthreads();
-    const uint64_t dterm = (uint64_t)(a.first_draw + ln.j) * kDrawMul;
     double sq = 0.0;
     double ax[kMaxCov];
 #pragma unroll
@@ -207,7 +130,6 @@ __global__ void __launch_bounds__(kPassThreads) k_center(Args a)
         const int n = (int)(e - s);
         // pass 1
         double sw = 0.0, tot = 0.0;
-        uint32_t bits = 0;
         double wl = 1.0, irl = 1.0;
         for (int c0 = 0; c0 < n; c0 += BP) {
             const int m = min(BP, n - c0);
@@ -218,16 +140,7 @@ __global__ void __launch_bounds__(kPassThreads) k_center(Args a)
                 const double ir = __shfl_sync(ln.mask, irl, q, BP);
                 sw += wi;
                 if (ln.on) {
-                    double r;
-                    const int64_t i = s + c0 + q;
-                    if (a.R) {
-                        r = a.R[i * a.B + ln.j] * ir;
-                    } else {
-                        const bool neg =
-                            rad_negative(a.seed, (uint64_t)(a.ordinal0 + i) * kRowMul, dterm);
-                        if (c0 == 0 && neg) bits |= 1u << q;
-                        r = neg ? -ir : ir;
-                    }
+                    const double r = a.R[(s + c0 + q) * a.B + ln.j] * ir;
                     tot += wi * r;
                     sq += wi * r * r;
                 }
@@ -257,17 +170,7 @@ __global__ void __launch_bounds__(kPassThreads) k_center(Args a)
                 take_codes(a, ch.codes, q, prev);
                 have = true;
                 if (!ln.on) continue;
-                const int64_t i = s + c0 + q;
-                double r;
-                if (a.R) {
-                    r = a.R[i * a.B + ln.j] * ir;
-                } else {
-                    const bool neg =
-                        c0 == 0 ? ((bits >> q) & 1u) != 0
-                                : rad_negative(a.seed, (uint64_t)(a.ordinal0 + i) * kRowMul, dterm);
-                    r = neg ? -ir : ir;
-                }
-                const double v = wi * (r - mean);
+                const double v = wi * (a.R[(s + c0 + q) * a.B + ln.j] * ir - mean);
                 run += v;
 #pragma unroll
                 for (int c = 0; c < kMaxCov; c++) {
@@ -298,7 +201,8 @@ __global__ void __launch_bounds__(kPassThreads) k_center(Args a)
     }
 }
 
-// `_nb_project_rows` and the JLA sink, one sub-warp of BP lanes per group.
+// `_nb_project_rows` and the JLA sink for explicit vectors R, one sub-warp of
+// BP lanes per group.
 // h_ij = sum_d U[level_d(i), j] (loaded once per run of equal codes) +
 // X_i . C[:, j]; pass 1: the weighted group mean of r - h; pass 2: the
 // projection o_ij (times sqrt(w_i) in the square-root weight metric), written
@@ -322,7 +226,6 @@ __global__ void __launch_bounds__(kPassThreads) k_project(Args a)
     ch.x = reinterpret_cast<double *>(s_chunks + subw * Chunk<BP>::kBytes + BP * HDFE_MAX_DIMS * 4);
     for (int k = threadIdx.x; k < a.c * a.B; k += kPassThreads) s_C[k] = a.C[k];
     __syncthreads();
-    const uint64_t dterm = (uint64_t)(a.first_draw + ln.j) * kDrawMul;
     double *pp_buf = s_mom, *mm_buf = s_mom + MR * (BP + 1);
     auto hU_of = [&](const uint32_t (&codes)[HDFE_MAX_DIMS]) {
         double h = 0.0;
@@ -369,7 +272,6 @@ __global__ void __launch_bounds__(kPassThreads) k_project(Args a)
         const int n = (int)(e - s);
         // pass 1
         double sw = 0.0, tot = 0.0;
-        uint32_t bits = 0;
         double wl = 1.0, irl = 1.0;
         uint32_t prev[HDFE_MAX_DIMS] = {0, 0, 0, 0};
         bool have = false;
@@ -388,15 +290,7 @@ __global__ void __launch_bounds__(kPassThreads) k_project(Args a)
                     have = true;
                 }
                 if (!ln.on) continue;
-                const int64_t i = s + c0 + q;
-                double r;
-                if (a.R) {
-                    r = a.R[i * a.B + ln.j] * ir;
-                } else {
-                    const bool neg = rad_negative(a.seed, (uint64_t)(a.ordinal0 + i) * kRowMul, dterm);
-                    if (c0 == 0 && neg) bits |= 1u << q;
-                    r = neg ? -ir : ir;
-                }
+                const double r = a.R[(s + c0 + q) * a.B + ln.j] * ir;
                 tot += wi * (r - (hU + h_cov(q)));
             }
             if (c0 + BP < n) __syncwarp(ln.mask);
@@ -425,15 +319,7 @@ __global__ void __launch_bounds__(kPassThreads) k_project(Args a)
                     double o = hU + h_cov(q) + mean;
                     if (a.sqrt_weights) o *= sqrt(wi);
                     if (a.out) a.out[i * a.B + ln.j] = o;
-                    double rr;       // the sink's unscaled draw
-                    if (a.R) {
-                        rr = a.R[i * a.B + ln.j];
-                    } else {
-                        const bool neg =
-                            c0 == 0 ? ((bits >> q) & 1u) != 0
-                                    : rad_negative(a.seed, (uint64_t)(a.ordinal0 + i) * kRowMul, dterm);
-                        rr = neg ? -1.0 : 1.0;
-                    }
+                    const double rr = a.R[i * a.B + ln.j];   // the sink's unscaled vector
                     P = o * o;
                     M = (rr - o) * (rr - o);
                 }
@@ -580,7 +466,8 @@ constexpr int center_chunk_smem() { return (kPassThreads / BP) * Chunk<BP>::kByt
 
 constexpr int kSmallBytes = 40 * 1024;    // small dimensions' level x draw sums per CTA
 
-// the dynamic shared memory limits, raised once per device
+// the dynamic shared memory limits of the explicit-vector passes, raised once
+// per device
 bool set_smem_limits()
 {
     static bool done[64] = {};
@@ -660,6 +547,13 @@ extern "C" int hdfe_rows_center(const int64_t *starts, int64_t n_groups, const u
     HDFE_CUDA_TRY(cudaMemsetAsync(acc, 0, a.L * B * 8, s));
     if (c > 0) HDFE_CUDA_TRY(cudaMemsetAsync(acc_x, 0, (int64_t)c * B * 8, s));
     if (squares) HDFE_CUDA_TRY(cudaMemsetAsync(squares, 0, B * 8, s));
+    if (!R) {
+        st = rows::launch_center_draws(a, s);
+        if (st != HDFE_OK) return st;
+        HDFE_CUDA_TRY(cudaGetLastError());
+        hdfe_add_launches(1);
+        return HDFE_OK;
+    }
     if (!rows::set_smem_limits()) return hdfe_set_cuda_error(cudaGetLastError());
     const unsigned grid = rows::grid_for(n_groups, a.Bp);
     if (a.Bp == 8)
@@ -692,6 +586,13 @@ extern "C" int hdfe_rows_project(const int64_t *starts, int64_t n_groups, const 
     a.moments = moments;
     a.N = n_rows;
     cudaStream_t s = (cudaStream_t)stream;
+    if (!R) {
+        st = rows::launch_project_draws(a, s);
+        if (st != HDFE_OK) return st;
+        HDFE_CUDA_TRY(cudaGetLastError());
+        hdfe_add_launches(1);
+        return HDFE_OK;
+    }
     if (!rows::set_smem_limits()) return hdfe_set_cuda_error(cudaGetLastError());
     const unsigned grid = rows::grid_for(n_groups, a.Bp);
     if (a.Bp == 8)
