@@ -7,14 +7,11 @@
 // kernels_inverse.py:192-231 `_nb_trace_moments`; the coefficient-space
 // Rademacher vectors of `_trace_block` (core/kernels_groups.py:53-76).
 //
-// One sub-warp of Bp lanes (Bp = the block width rounded up to 8, 16 or 32)
-// per group of rows, lane j holding vector j:
 //   reduce        acc[level, j] += w_i R_ij over the rows (no centring), where
 //                 R is either explicit rows or the streamed block spread over
 //                 its group (R_ij = streamed[g, j] / s_g, s_g = the group's
 //                 weight); acc_x[c, j] += X_ic w_i R_ij; optionally the group
-//                 sums of w_i R_ij.  Sums over a run of rows with equal codes
-//                 are added once per run.
+//                 sums of w_i R_ij.
 //   project_coef  h_ij = sum_d U[level_d(i), j] + X_i . C[:, j]; u0[g, j] =
 //                 weighted group mean of (rho - h); rows (A u)_ij = h + u0 and
 //                 the groups' u0; optionally the collect sink in the same pass:
@@ -22,9 +19,29 @@
 //   trace         per vector j the eight weighted sums of the psi-dimension
 //                 values (a) and streamed values (b) of Z and U over rows, per
 //                 CTA in a fixed order and then over CTAs in a fixed order.
+//
+// Blocks of vectors (more than four) take windows of up to 32 rows made of
+// whole groups, a sub-warp of Bp lanes (the width rounded up to 8, 16 or 32),
+// lane j vector j.  Within a run of rows with equal codes the values h differ
+// by the covariates only, so everything but the rows' own output is linear in
+// sums over the run that no vector enters: w, w omega and w omega X.  Those
+// are made once a window by lane (run, sum), and a vector's work is per run
+// (1.75 a worker rather than 8.5 rows): one gather of U's row, the window's
+// first eight in flight, and a few FMAs.  The covariates' own block X' omega X
+// C of the sink is per pass: each lane sums omega X X' over the rows it staged.
+// 1M-worker panel, 32 vectors, 2 covariates: reduce 1.34 -> 0.45 ms,
+// project_coef with the sink 3.23 -> 1.58 ms.
+//
+// Narrow blocks (one to four vectors, the adjoint's) have too few lanes for
+// that: there a thread (or 2, 4) takes a group and walks its rows, 32 (16, 8)
+// groups a warp.  Dimensions with few levels (the years) are added into a
+// CTA's own copy in shared memory: ten addresses otherwise see every row's
+// atomic (3.4M rows, one vector: reduce 2.37 -> 0.09 ms, project_coef
+// 1.22 -> 0.13 ms).
 #include <cuda_runtime.h>
 
 #include "common.cuh"
+#include "windows.cuh"
 
 namespace hdfe {
 namespace coef {
@@ -55,6 +72,11 @@ struct Args {
     double *acc, *acc_x;        // (L, B), (c, B): added into
     double *gsum;               // (G, B) or null
     unsigned *status;
+    int64_t chunk;              // groups a sub-warp takes at a time (windows)
+    // narrow passes: dimensions summed in shared memory first
+    int small[HDFE_MAX_DIMS];
+    int64_t soff[HDFE_MAX_DIMS];
+    int64_t n_small;
 };
 
 template <int BP>
@@ -113,20 +135,41 @@ struct Runs {
     bool have;
 };
 
-__device__ __forceinline__ void run_flush(const Args &a, const Runs &run, int j)
+__device__ __forceinline__ void run_flush(const Args &a, const Runs &run, int j, double *s_acc)
 {
 #pragma unroll
     for (int d = 0; d < HDFE_MAX_DIMS; d++) {
         if (d >= a.D) break;
-        atomicAdd(a.acc + (a.offs[d] + run.codes[d]) * a.B + j, run.v);
+        if (a.small[d]) atomicAdd(s_acc + (a.soff[d] + run.codes[d]) * a.B + j, run.v);
+        else atomicAdd(a.acc + (a.offs[d] + run.codes[d]) * a.B + j, run.v);
+    }
+}
+
+// the shared sums of the small dimensions: cleared, and added to acc at the end
+__device__ __forceinline__ void small_clear(const Args &a, double *s_acc)
+{
+    for (int64_t k = threadIdx.x; k < a.n_small * a.B; k += kThreads) s_acc[k] = 0.0;
+    __syncthreads();
+}
+
+__device__ __forceinline__ void small_flush(const Args &a, const double *s_acc)
+{
+    if (a.n_small == 0) return;
+    __syncthreads();
+    for (int d = 0; d < a.D; d++) {
+        if (!a.small[d]) continue;
+        for (int64_t q = threadIdx.x; q < a.nlev[d] * a.B; q += kThreads) {
+            const double v = s_acc[a.soff[d] * a.B + q];
+            if (v != 0.0) atomicAdd(a.acc + a.offs[d] * a.B + q, v);
+        }
     }
 }
 
 __device__ __forceinline__ void run_add(const Args &a, Runs &run, const uint32_t (&c)[HDFE_MAX_DIMS],
-                                        double v, int j, bool on)
+                                        double v, int j, bool on, double *s_acc)
 {
     if (run.have && !same(a, run.codes, c)) {
-        if (on) run_flush(a, run, j);
+        if (on) run_flush(a, run, j, s_acc);
         run.v = 0.0;
     }
 #pragma unroll
@@ -138,18 +181,21 @@ __device__ __forceinline__ void run_add(const Args &a, Runs &run, const uint32_t
     run.v += v;
 }
 
-// the covariate block: per thread, then per CTA, then one add per entry
+// the covariate block: per lane of equal j in the warp, then per CTA, then one
+// add per entry
+template <int BP>
 __device__ __forceinline__ void flush_cov(const Args &a, const double (&ax)[kMaxCov], double *s_ax,
                                           int j, bool on)
 {
     for (int k = threadIdx.x; k < a.c * a.B; k += kThreads) s_ax[k] = 0.0;
     __syncthreads();
-    if (on) {
 #pragma unroll
-        for (int c = 0; c < kMaxCov; c++) {
-            if (c >= a.c) break;
-            atomicAdd(s_ax + c * a.B + j, ax[c]);
-        }
+    for (int c = 0; c < kMaxCov; c++) {
+        if (c >= a.c) break;
+        double v = ax[c];
+#pragma unroll
+        for (int o = 16; o >= BP; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+        if (on && (threadIdx.x & 31) < BP) atomicAdd(s_ax + c * a.B + j, v);
     }
     __syncthreads();
     for (int k = threadIdx.x; k < a.c * a.B; k += kThreads)
@@ -160,8 +206,10 @@ template <int BP>
 __global__ void __launch_bounds__(kThreads) k_reduce(Args a)
 {
     constexpr int SUBS = kThreads / BP;
+    extern __shared__ __align__(16) double s_acc[];
     __shared__ double s_ax[kMaxCov * 32];
     const Lanes<BP> ln(a.B);
+    small_clear(a, s_acc);
     const int64_t g0 = (int64_t)blockIdx.x * SUBS + threadIdx.x / BP;
     const int64_t gstep = (int64_t)gridDim.x * SUBS;
     double ax[kMaxCov];
@@ -182,7 +230,7 @@ __global__ void __launch_bounds__(kThreads) k_reduce(Args a)
             const double wi = a.w ? __ldg(a.w + i) : 1.0;
             const double r = a.streamed ? rho : (ln.on ? a.R[i * a.B + ln.j] : 0.0);
             const double v = wi * r;
-            run_add(a, run, c, v, ln.j, ln.on);
+            run_add(a, run, c, v, ln.j, ln.on, s_acc);
             gs += v;
 #pragma unroll
             for (int cc = 0; cc < kMaxCov; cc++) {
@@ -190,10 +238,11 @@ __global__ void __launch_bounds__(kThreads) k_reduce(Args a)
                 ax[cc] += __ldg(a.X + i * a.c + cc) * v;
             }
         }
-        if (run.have && ln.on) run_flush(a, run, ln.j);
+        if (run.have && ln.on) run_flush(a, run, ln.j, s_acc);
         if (a.gsum && ln.on) a.gsum[g * a.B + ln.j] = gs;
     }
-    if (a.acc_x && a.c > 0) flush_cov(a, ax, s_ax, ln.j, ln.on);
+    small_flush(a, s_acc);
+    if (a.acc_x && a.c > 0) flush_cov<BP>(a, ax, s_ax, ln.j, ln.on);
 }
 
 template <int BP>
@@ -202,9 +251,10 @@ __global__ void __launch_bounds__(kThreads) k_project_coef(Args a)
     constexpr int SUBS = kThreads / BP;
     __shared__ double s_ax[kMaxCov * 32];
     __shared__ double s_C[kMaxCov * 32];
+    extern __shared__ __align__(16) double s_acc[];
     const Lanes<BP> ln(a.B);
     for (int k = threadIdx.x; k < a.c * a.B; k += kThreads) s_C[k] = a.C[k];
-    __syncthreads();
+    small_clear(a, s_acc);
     const int64_t g0 = (int64_t)blockIdx.x * SUBS + threadIdx.x / BP;
     const int64_t gstep = (int64_t)gridDim.x * SUBS;
     double ax[kMaxCov];
@@ -261,7 +311,7 @@ __global__ void __launch_bounds__(kThreads) k_project_coef(Args a)
             if (a.collect) {
                 const double wi = a.w ? __ldg(a.w + i) : 1.0;
                 const double v = wi * (a.omega ? __ldg(a.omega + i) : 1.0) * o;
-                run_add(a, run, c, v, ln.j, ln.on);
+                run_add(a, run, c, v, ln.j, ln.on, s_acc);
                 gs += v;
 #pragma unroll
                 for (int cc = 0; cc < kMaxCov; cc++) {
@@ -271,11 +321,425 @@ __global__ void __launch_bounds__(kThreads) k_project_coef(Args a)
             }
         }
         if (a.collect) {
-            if (run.have && ln.on) run_flush(a, run, ln.j);
+            if (run.have && ln.on) run_flush(a, run, ln.j, s_acc);
             if (a.gsum && ln.on) a.gsum[g * a.B + ln.j] = gs;
         }
     }
-    if (a.collect && a.acc_x && a.c > 0) flush_cov(a, ax, s_ax, ln.j, ln.on);
+    if (a.collect) small_flush(a, s_acc);
+    if (a.collect && a.acc_x && a.c > 0) flush_cov<BP>(a, ax, s_ax, ln.j, ln.on);
+}
+
+// ------------------------------------------------------ windows (wide blocks)
+
+// one sub-warp's staging: rows (codes, covariates, weights, w omega), group
+// sums, run sums, the groups' streamed values and U's rows of the runs
+constexpr int kAhead = 8;               // runs and groups whose values are loaded ahead
+
+template <int BP>
+struct Win {
+    static __host__ __device__ int bytes(int c, int D, bool weights, bool project, bool collect)
+    {
+        const int d = kWin * c + kWin * (c + 2) + (weights ? 2 * kWin : 0) +
+                      (collect ? kWin + kWin * (c + 1) : 0) + kAhead * BP +
+                      (project ? kWin * BP : 0);
+        return (d * 8 + kWin * D * 4 + 15) / 16 * 16;
+    }
+    double *x, *gx, *w, *rw, *om, *ro, *st, *hu;
+    uint32_t *codes;
+    __device__ Win(char *p, int c, int D, bool weights, bool project, bool collect)
+    {
+        double *q = reinterpret_cast<double *>(p);
+        auto take = [&](int n) { double *at = q; q += n; return at; };
+        x = take(kWin * c);
+        gx = take(kWin * (c + 2));                  // sums of w x, w; 1 / sum of w
+        w = take(weights ? kWin : 0);
+        rw = take(weights ? kWin : 0);              // by run head
+        om = take(collect ? kWin : 0);
+        ro = take(collect ? kWin * (c + 1) : 0);    // by run: sums of w omega, w omega x
+        st = take(kAhead * BP);
+        hu = take(project ? kWin * BP : 0);         // by run head
+        codes = reinterpret_cast<uint32_t *>(q);
+    }
+};
+
+// rows [i0, i0 + n) into the window; returns the run heads' mask.  xx: this
+// lane's sums of w omega x_k x_l (k <= l) over the rows it staged.
+template <int BP, int C, bool COLLECT>
+__device__ __forceinline__ unsigned load_window(const Args &a, const Lanes<BP> &ln, Win<BP> &wn,
+                                                int64_t i0, int n, double *xx)
+{
+    const int c = C < 0 ? a.c : C;
+    const bool W = a.w != nullptr;
+    constexpr int CM = C < 0 ? kMaxCov : (C > 0 ? C : 1);
+    for (int t = ln.j; t < n; t += BP) {
+        const int64_t i = i0 + t;
+        uint32_t code[HDFE_MAX_DIMS];
+        row_codes(a, i, code);
+#pragma unroll
+        for (int d = 0; d < HDFE_MAX_DIMS; d++) {
+            if (d >= a.D) break;
+            wn.codes[t * a.D + d] = code[d];
+        }
+        double x[CM];
+#pragma unroll
+        for (int k = 0; k < CM; k++) {
+            if (k >= c) break;
+            x[k] = __ldg(a.X + i * a.c + k);
+            wn.x[t * c + k] = x[k];
+        }
+        const double w = W ? __ldg(a.w + i) : 1.0;
+        if (W) wn.w[t] = w;
+        if (COLLECT) {
+            const double o = w * (a.omega ? __ldg(a.omega + i) : 1.0);
+            wn.om[t] = o;
+            if (xx) {
+#pragma unroll
+                for (int k = 0; k < CM; k++) {
+                    if (k >= c) break;
+#pragma unroll
+                    for (int l = 0; l < CM; l++) {
+                        if (l < k) continue;
+                        if (l >= c) break;
+                        xx[k * CM + l] += o * x[k] * x[l];
+                    }
+                }
+            }
+        }
+    }
+    __syncwarp(ln.mask);
+    unsigned heads = 0;
+    for (int t = ln.j; t < n; t += BP) {
+        bool head = t == 0;
+        if (t > 0)
+            for (int d = 0; d < a.D; d++)
+                head |= wn.codes[t * a.D + d] != wn.codes[(t - 1) * a.D + d];
+        heads |= (unsigned)head << t;
+    }
+    return __reduce_or_sync(ln.mask, heads);
+}
+
+// the groups' sums of w x and w with the reciprocal weight, and the runs' sums
+// of w, w omega and w omega x, each by one lane
+template <int BP, int C, bool COLLECT>
+__device__ __forceinline__ void window_sums(const Args &a, const Lanes<BP> &ln, Win<BP> &wn,
+                                            unsigned gheads, int ng, unsigned heads, int n)
+{
+    const int c = C < 0 ? a.c : C;
+    const bool W = a.w != nullptr;
+    for (int t = ln.j; t < ng * (c + 1); t += BP) {
+        const int g = t / (c + 1), k = t - g * (c + 1);
+        const int q0 = nth_bit(gheads, g), q1 = next_bit(gheads, q0, n);
+        double v = 0.0;
+        if (k == c && !W) {
+            v = (double)(q1 - q0);
+        } else {
+            for (int q = q0; q < q1; q++) {
+                const double xq = k < c ? wn.x[q * c + k] : 1.0;
+                v += W ? wn.w[q] * xq : xq;
+            }
+        }
+        wn.gx[g * (c + 2) + k] = v;
+        if (k == c) wn.gx[g * (c + 2) + c + 1] = v > 0.0 ? 1.0 / v : 0.0;
+    }
+    if (W || COLLECT) {
+        const int nr = __popc(heads), per = (W ? 1 : 0) + (COLLECT ? c + 1 : 0);
+        for (int t = ln.j; t < nr * per; t += BP) {
+            const int r = t / per, k = t - r * per - (W ? 1 : 0);      // -1: the run's weight
+            const int q0 = nth_bit(heads, r), q1 = next_bit(heads, q0, n);
+            double v = 0.0;
+            for (int q = q0; q < q1; q++)
+                v += k < 0 ? wn.w[q] : (k == 0 ? wn.om[q] : wn.om[q] * wn.x[q * c + k - 1]);
+            if (k < 0) wn.rw[q0] = v;
+            else wn.ro[r * (c + 1) + k] = v;
+        }
+    }
+    __syncwarp(ln.mask);
+}
+
+// the streamed values of the window's first groups (the rest is loaded when
+// its turn comes)
+template <int BP>
+__device__ __forceinline__ void load_streamed(const Args &a, const Lanes<BP> &ln, Win<BP> &wn,
+                                              int64_t g, int ng)
+{
+    double v[kAhead];
+#pragma unroll
+    for (int f = 0; f < kAhead; f++)
+        v[f] = f < ng && ln.on && a.streamed ? a.streamed[(g + f) * a.B + ln.j] : 0.0;
+#pragma unroll
+    for (int f = 0; f < kAhead; f++)
+        if (f < ng) wn.st[f * BP + ln.j] = v[f];
+}
+
+template <int BP>
+__device__ __forceinline__ double streamed_of(const Args &a, const Lanes<BP> &ln,
+                                              const Win<BP> &wn, int64_t g, int f)
+{
+    if (f < kAhead) return wn.st[f * BP + ln.j];
+    return ln.on && a.streamed ? a.streamed[(g + f) * a.B + ln.j] : 0.0;
+}
+
+// v to row q's levels
+template <int BP>
+__device__ __forceinline__ void add_levels(const Args &a, const Lanes<BP> &ln, const Win<BP> &wn,
+                                           int q, double v)
+{
+    if (!ln.on) return;
+#pragma unroll
+    for (int d = 0; d < HDFE_MAX_DIMS; d++) {
+        if (d >= a.D) break;
+        atomicAdd(a.acc + (a.offs[d] + wn.codes[q * a.D + d]) * a.B + ln.j, v);
+    }
+}
+
+template <int BP, int CM>
+__device__ __forceinline__ void add_cov(const Args &a, const Lanes<BP> &ln, const double (&ax)[CM],
+                                        int c, double *s_ax)
+{
+    if (!a.acc_x || c == 0) return;
+    for (int k = threadIdx.x; k < c * a.B; k += kThreads) s_ax[k] = 0.0;
+    __syncthreads();
+    if (ln.on) {
+#pragma unroll
+        for (int k = 0; k < CM; k++) {
+            if (k >= c) break;
+            atomicAdd(s_ax + k * a.B + ln.j, ax[k]);
+        }
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < c * a.B; k += kThreads)
+        if (s_ax[k] != 0.0) atomicAdd(a.acc_x + k, s_ax[k]);
+}
+
+template <int BP, typename F, typename H>
+__device__ __forceinline__ void walk(const Args &a, const Lanes<BP> &ln, F window, H lone)
+{
+    constexpr int SUBS = kThreads / BP;
+    walk_windows<BP>(a.starts, a.G, a.chunk, (int64_t)blockIdx.x * SUBS + threadIdx.x / BP,
+                     (int64_t)gridDim.x * SUBS, ln.j, ln.mask, window, lone);
+}
+
+// reduce of the streamed block
+template <int BP, int C>
+__global__ void __launch_bounds__(kThreads) k_spread_win(Args a)
+{
+    extern __shared__ __align__(16) char s_raw[];
+    __shared__ double s_ax[kMaxCov * 32];
+    const Lanes<BP> ln(a.B);
+    const int c = C < 0 ? a.c : C;
+    const bool W = a.w != nullptr;
+    constexpr int CM = C < 0 ? kMaxCov : (C > 0 ? C : 1);
+    Win<BP> wn(s_raw + (threadIdx.x / BP) * Win<BP>::bytes(c, a.D, W, false, false), c, a.D, W,
+               false, false);
+    double ax[CM];
+#pragma unroll
+    for (int k = 0; k < CM; k++) ax[k] = 0.0;
+    // group f of the window, rows [q0, q1), rho its streamed value over its weight
+    auto group = [&](int f, int q0, int q1, unsigned heads, double rho) {
+#pragma unroll
+        for (int k = 0; k < CM; k++) {
+            if (k >= c) break;
+            ax[k] += wn.gx[f * (c + 2) + k] * rho;
+        }
+        for (int p0 = q0; p0 < q1;) {
+            const int p1 = next_bit(heads, p0, q1);
+            add_levels(a, ln, wn, p0, (W ? wn.rw[p0] : (double)(p1 - p0)) * rho);
+            p0 = p1;
+        }
+    };
+    auto window = [&](int64_t g, int64_t i0, int n, unsigned gheads, int ng) {
+        load_streamed(a, ln, wn, g, ng);
+        const unsigned heads =
+            load_window<BP, C, false>(a, ln, wn, i0, n, nullptr) | gheads;
+        window_sums<BP, C, false>(a, ln, wn, gheads, ng, heads, n);
+        int q0 = 0;
+        for (int f = 0; f < ng; f++) {
+            const int q1 = next_bit(gheads, q0, n);
+            group(f, q0, q1, heads, streamed_of(a, ln, wn, g, f) * wn.gx[f * (c + 2) + c + 1]);
+            q0 = q1;
+        }
+    };
+    auto lone = [&](int64_t g, int64_t s, int64_t e) {
+        const double sw = group_weight(a, s, e);
+        const double rho = ln.on && sw > 0.0 ? a.streamed[g * a.B + ln.j] / sw : 0.0;
+        for (int64_t i0 = s; i0 < e; i0 += kWin) {
+            const int n = (int)min((int64_t)kWin, e - i0);
+            const unsigned heads = load_window<BP, C, false>(a, ln, wn, i0, n, nullptr);
+            window_sums<BP, C, false>(a, ln, wn, 1u, 1, heads, n);
+            group(0, 0, n, heads, rho);
+            __syncwarp(ln.mask);
+        }
+    };
+    walk(a, ln, window, lone);
+    add_cov<BP, CM>(a, ln, ax, c, s_ax);
+}
+
+template <int BP, int C, bool COLLECT>
+__global__ void __launch_bounds__(kThreads) k_project_win(Args a)
+{
+    extern __shared__ __align__(16) char s_raw[];
+    __shared__ double s_ax[kMaxCov * 32];
+    const Lanes<BP> ln(a.B);
+    const int c = C < 0 ? a.c : C;
+    const bool W = a.w != nullptr;
+    constexpr int CM = C < 0 ? kMaxCov : (C > 0 ? C : 1);
+    Win<BP> wn(s_raw + (threadIdx.x / BP) * Win<BP>::bytes(c, a.D, W, true, COLLECT), c, a.D, W,
+               true, COLLECT);
+    double ax[CM], xx[COLLECT ? CM * CM : 1], Cj[CM];
+#pragma unroll
+    for (int k = 0; k < CM; k++) {
+        ax[k] = 0.0;
+        Cj[k] = k < c && ln.on ? a.C[k * a.B + ln.j] : 0.0;
+    }
+    if (COLLECT) {
+#pragma unroll
+        for (int k = 0; k < CM * CM; k++) xx[k] = 0.0;
+    }
+    auto gather = [&](int q) {                  // sum_d U[level_d, j] of row q's run
+        double h = 0.0;
+#pragma unroll
+        for (int d = 0; d < HDFE_MAX_DIMS; d++) {
+            if (d >= a.D) break;
+            h += a.U[(a.offs[d] + wn.codes[q * a.D + d]) * a.B + ln.j];
+        }
+        return h;
+    };
+    // U's rows of the runs: the first kAhead loaded together
+    auto load_runs = [&](unsigned heads) {
+        double h[kAhead];
+        unsigned m = heads;
+#pragma unroll
+        for (int f = 0; f < kAhead; f++) {
+            h[f] = m && ln.on ? gather(__ffs(m) - 1) : 0.0;
+            m &= m - 1;
+        }
+        unsigned m2 = heads;
+#pragma unroll
+        for (int f = 0; f < kAhead; f++) {
+            if (m2) wn.hu[(__ffs(m2) - 1) * BP + ln.j] = h[f];
+            m2 &= m2 - 1;
+        }
+        for (; m; m &= m - 1) {
+            const int q = __ffs(m) - 1;
+            wn.hu[q * BP + ln.j] = ln.on ? gather(q) : 0.0;
+        }
+    };
+    // sum over the runs of [q0, q1) of w hU
+    auto sum_h = [&](unsigned heads, int q0, int q1) {
+        double t = 0.0;
+        for (int p0 = q0; p0 < q1;) {
+            const int p1 = next_bit(heads, p0, q1);
+            t += (W ? wn.rw[p0] : (double)(p1 - p0)) * wn.hu[p0 * BP + ln.j];
+            p0 = p1;
+        }
+        return t;
+    };
+    // the rows' output and the sink's sums of rows [q0, q1) of one group whose
+    // first run is the window's r-th; returns the group sum
+    auto emit = [&](unsigned heads, int64_t i0, int q0, int q1, int r, double mean) {
+        double gs = 0.0;
+        for (int p0 = q0; p0 < q1; r++) {
+            const int p1 = next_bit(heads, p0, q1);
+            const double base = wn.hu[p0 * BP + ln.j] + mean;
+            if (a.rows) {
+                for (int q = p0; q < p1; q++) {
+                    double o = base;
+#pragma unroll
+                    for (int k = 0; k < CM; k++) {
+                        if (k >= c) break;
+                        o += wn.x[q * c + k] * Cj[k];
+                    }
+                    if (ln.on) a.rows[(i0 + q) * a.B + ln.j] = o;
+                }
+            }
+            if (COLLECT) {
+                const double *ro = wn.ro + r * (c + 1);
+                double v = ro[0] * base;
+#pragma unroll
+                for (int k = 0; k < CM; k++) {
+                    if (k >= c) break;
+                    v += ro[1 + k] * Cj[k];
+                    ax[k] += ro[1 + k] * base;
+                }
+                add_levels(a, ln, wn, p0, v);
+                gs += v;
+            }
+            p0 = p1;
+        }
+        return gs;
+    };
+    auto window = [&](int64_t g, int64_t i0, int n, unsigned gheads, int ng) {
+        load_streamed(a, ln, wn, g, ng);
+        const unsigned heads = load_window<BP, C, COLLECT>(a, ln, wn, i0, n, xx) | gheads;
+        load_runs(heads);
+        window_sums<BP, C, COLLECT>(a, ln, wn, gheads, ng, heads, n);
+        int q0 = 0, r = 0;
+        for (int f = 0; f < ng; f++) {
+            const int q1 = next_bit(gheads, q0, n);
+            const double *gx = wn.gx + f * (c + 2);
+            // the mean of rho - h, rho = streamed / sum of w
+            double tot = (gx[c] > 0.0 ? streamed_of(a, ln, wn, g, f) : 0.0) - sum_h(heads, q0, q1);
+#pragma unroll
+            for (int k = 0; k < CM; k++) {
+                if (k >= c) break;
+                tot -= gx[k] * Cj[k];
+            }
+            const double mean = tot * gx[c + 1];
+            if (a.groups && ln.on) a.groups[(g + f) * a.B + ln.j] = mean;
+            if (a.rows || COLLECT) {
+                const double gs = emit(heads, i0, q0, q1, r, mean);
+                if (COLLECT && a.gsum && ln.on) a.gsum[(g + f) * a.B + ln.j] = gs;
+            }
+            r += __popc(heads & below(q1) & ~below(q0));
+            q0 = q1;
+        }
+    };
+    auto lone = [&](int64_t g, int64_t s, int64_t e) {
+        const double sw = group_weight(a, s, e);
+        double tot = a.streamed && ln.on && sw > 0.0 ? a.streamed[g * a.B + ln.j] : 0.0, gs = 0.0;
+        for (int64_t i0 = s; i0 < e; i0 += kWin) {
+            const int n = (int)min((int64_t)kWin, e - i0);
+            const unsigned heads = load_window<BP, C, COLLECT>(a, ln, wn, i0, n, nullptr);
+            load_runs(heads);
+            window_sums<BP, C, COLLECT>(a, ln, wn, 1u, 1, heads, n);
+            tot -= sum_h(heads, 0, n);
+#pragma unroll
+            for (int k = 0; k < CM; k++) {
+                if (k >= c) break;
+                tot -= wn.gx[k] * Cj[k];
+            }
+            __syncwarp(ln.mask);
+        }
+        const double mean = sw > 0.0 ? tot / sw : 0.0;
+        if (a.groups && ln.on) a.groups[g * a.B + ln.j] = mean;
+        if (!a.rows && !COLLECT) return;
+        for (int64_t i0 = s; i0 < e; i0 += kWin) {
+            const int n = (int)min((int64_t)kWin, e - i0);
+            const unsigned heads = load_window<BP, C, COLLECT>(a, ln, wn, i0, n, xx);
+            load_runs(heads);
+            window_sums<BP, C, COLLECT>(a, ln, wn, 1u, 1, heads, n);
+            gs += emit(heads, i0, 0, n, 0, mean);
+            __syncwarp(ln.mask);
+        }
+        if (COLLECT && a.gsum && ln.on) a.gsum[g * a.B + ln.j] = gs;
+    };
+    walk(a, ln, window, lone);
+    if (COLLECT) {
+        // the sub-warp's w omega X X' times C
+#pragma unroll
+        for (int k = 0; k < CM; k++) {
+#pragma unroll
+            for (int l = 0; l < CM; l++) {
+                if (l < k || k >= c || l >= c) continue;
+                double v = xx[k * CM + l];
+#pragma unroll
+                for (int o = BP / 2; o > 0; o >>= 1) v += __shfl_xor_sync(ln.mask, v, o, BP);
+                ax[k] += v * Cj[l];
+                if (l != k) ax[l] += v * Cj[k];
+            }
+        }
+        add_cov<BP, CM>(a, ln, ax, c, s_ax);
+    }
 }
 
 // ---------------------------------------------------------- trace moments
@@ -291,37 +755,52 @@ struct TraceArgs {
     int B;
     double *partial;                     // (gridDim, B, 8)
     unsigned *status;
+    int64_t chunk;
 };
 
+// Per run of rows with one psi level, as the passes above (0.60 -> 0.45 ms
+// for 32 vectors on the 1M-worker panel).
 template <int BP>
 __global__ void __launch_bounds__(kThreads) k_trace(TraceArgs a)
 {
     constexpr int SUBS = kThreads / BP;
     __shared__ double s_m[SUBS][BP][8];
+    __shared__ uint32_t s_code[SUBS][kWin];
+    __shared__ double s_w[SUBS][kWin];
     const Lanes<BP> ln(a.B);
     const int sub = threadIdx.x / BP;
-    const int64_t g0 = (int64_t)blockIdx.x * SUBS + sub;
-    const int64_t gstep = (int64_t)gridDim.x * SUBS;
+    uint32_t *code = s_code[sub];
+    double *w = s_w[sub];
     double m[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (int64_t g = g0; g < a.G; g += gstep) {
-        const int64_t s = a.starts[g], e = a.starts[g + 1];
-        const double b1 = ln.on ? a.Zg[g * a.B + ln.j] : 0.0;
-        const double b2 = ln.on ? a.Ug[g * a.B + ln.j] : 0.0;
-        uint32_t prev = 0xffffffffu;
-        double a1 = 0.0, a2 = 0.0;
-        for (int64_t i = s; i < e; i++) {
-            uint32_t code = __ldg(a.codes + i * a.D + a.psi_column);
-            if ((int64_t)code >= a.psi_levels) {
+    // rows [i0, i0 + n): their psi codes and weights; returns the run heads
+    auto load = [&](int64_t i0, int n) {
+        for (int t = ln.j; t < n; t += BP) {
+            uint32_t v = __ldg(a.codes + (i0 + t) * a.D + a.psi_column);
+            if ((int64_t)v >= a.psi_levels) {
                 if (a.status) atomicCAS(a.status, 0u, (unsigned)HDFE_ERR_BAD_CODE);
-                code = 0;
+                v = 0;
             }
-            if (code != prev) {
-                prev = code;
-                const int64_t lv = a.psi_offset + code;
-                a1 = ln.on ? a.Zl[lv * a.B + ln.j] : 0.0;
-                a2 = ln.on ? a.Ul[lv * a.B + ln.j] : 0.0;
+            code[t] = v;
+            if (a.w) w[t] = __ldg(a.w + i0 + t);
+        }
+        __syncwarp(ln.mask);
+        unsigned heads = 0;
+        for (int t = ln.j; t < n; t += BP)
+            heads |= (unsigned)(t == 0 || code[t] != code[t - 1]) << t;
+        return __reduce_or_sync(ln.mask, heads);
+    };
+    // the runs of rows [q0, q1), all of one group
+    auto group = [&](unsigned heads, int q0, int q1, double b1, double b2) {
+        for (int p0 = q0; p0 < q1;) {
+            const int p1 = next_bit(heads, p0, q1);
+            const int64_t lv = a.psi_offset + code[p0];
+            const double a1 = ln.on ? a.Zl[lv * a.B + ln.j] : 0.0;
+            const double a2 = ln.on ? a.Ul[lv * a.B + ln.j] : 0.0;
+            double wt = (double)(p1 - p0);
+            if (a.w) {
+                wt = 0.0;
+                for (int q = p0; q < p1; q++) wt += w[q];
             }
-            const double wt = a.w ? __ldg(a.w + i) : 1.0;
             m[0] += wt;
             m[1] += wt * a1 * a2;
             m[2] += wt * b1 * b2;
@@ -330,8 +809,30 @@ __global__ void __launch_bounds__(kThreads) k_trace(TraceArgs a)
             m[5] += wt * a2;
             m[6] += wt * b1;
             m[7] += wt * b2;
+            p0 = p1;
         }
-    }
+    };
+    auto window = [&](int64_t g, int64_t i0, int n, unsigned gheads, int ng) {
+        const unsigned heads = load(i0, n) | gheads;
+        int q0 = 0;
+        for (int f = 0; f < ng; f++) {
+            const int q1 = next_bit(gheads, q0, n);
+            group(heads, q0, q1, ln.on ? a.Zg[(g + f) * a.B + ln.j] : 0.0,
+                  ln.on ? a.Ug[(g + f) * a.B + ln.j] : 0.0);
+            q0 = q1;
+        }
+    };
+    auto lone = [&](int64_t g, int64_t s, int64_t e) {
+        const double b1 = ln.on && e > s ? a.Zg[g * a.B + ln.j] : 0.0;
+        const double b2 = ln.on && e > s ? a.Ug[g * a.B + ln.j] : 0.0;
+        for (int64_t i0 = s; i0 < e; i0 += kWin) {
+            const int n = (int)min((int64_t)kWin, e - i0);
+            group(load(i0, n), 0, n, b1, b2);
+            __syncwarp(ln.mask);
+        }
+    };
+    walk_windows<BP>(a.starts, a.G, a.chunk, (int64_t)blockIdx.x * SUBS + sub,
+                     (int64_t)gridDim.x * SUBS, ln.j, ln.mask, window, lone);
 #pragma unroll
     for (int k = 0; k < 8; k++) s_m[sub][ln.j][k] = m[k];
     __syncthreads();
@@ -411,6 +912,117 @@ inline unsigned grid_for(int64_t G, int Bp)
     return (unsigned)(b > 0 ? b : 1);
 }
 
+// CTAs of a window pass (sub-warps of Bp lanes), and its chunk of groups
+inline unsigned window_grid(int64_t G, int Bp, int64_t *chunk)
+{
+    const int64_t ctas = 148 * 5, subs = kThreads / Bp;
+    *chunk = window_chunk(G, ctas * subs);
+    int64_t b = (G + *chunk * subs - 1) / (*chunk * subs);
+    if (b > 2 * ctas) b = 2 * ctas;
+    return (unsigned)(b > 0 ? b : 1);
+}
+
+// Blocks up to this many vectors take the narrow passes.
+constexpr int kNarrow = 4;
+constexpr int64_t kSmallBytes = 32 * 1024;      // level sums in shared memory per CTA
+
+// the dimensions a narrow pass sums in shared memory first; returns the bytes
+inline int take_small(Args &a)
+{
+    int64_t slots = 0;
+    for (int d = 0; d < a.D; d++) {
+        if (a.nlev[d] <= 512 && (slots + a.nlev[d]) * a.B * 8 <= kSmallBytes) {
+            a.small[d] = 1;
+            a.soff[d] = slots;
+            slots += a.nlev[d];
+        }
+    }
+    a.n_small = slots;
+    return (int)(slots * a.B * 8);
+}
+
+template <typename K>
+int launch_window(K kernel, Args &a, int smem, cudaStream_t s)
+{
+    if (smem > 48 * 1024)
+        HDFE_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           smem));
+    const unsigned grid = window_grid(a.G, a.Bp, &a.chunk);
+    kernel<<<grid, kThreads, smem, s>>>(a);
+    return HDFE_OK;
+}
+
+template <int BP>
+int launch_spread(Args &a, cudaStream_t s)
+{
+    const int smem = kThreads / BP * Win<BP>::bytes(a.c, a.D, a.w != nullptr, false, false);
+    switch (a.c) {
+    case 0: return launch_window(k_spread_win<BP, 0>, a, smem, s);
+    case 1: return launch_window(k_spread_win<BP, 1>, a, smem, s);
+    case 2: return launch_window(k_spread_win<BP, 2>, a, smem, s);
+    case 3: return launch_window(k_spread_win<BP, 3>, a, smem, s);
+    default: return launch_window(k_spread_win<BP, -1>, a, smem, s);
+    }
+}
+
+template <int BP, bool COLLECT>
+int launch_project(Args &a, cudaStream_t s)
+{
+    const int smem = kThreads / BP * Win<BP>::bytes(a.c, a.D, a.w != nullptr, true, COLLECT);
+    switch (a.c) {
+    case 0: return launch_window(k_project_win<BP, 0, COLLECT>, a, smem, s);
+    case 1: return launch_window(k_project_win<BP, 1, COLLECT>, a, smem, s);
+    case 2: return launch_window(k_project_win<BP, 2, COLLECT>, a, smem, s);
+    case 3: return launch_window(k_project_win<BP, 3, COLLECT>, a, smem, s);
+    default: return launch_window(k_project_win<BP, -1, COLLECT>, a, smem, s);
+    }
+}
+
+template <int BP>
+int launch_project(Args &a, cudaStream_t s)
+{
+    return a.collect ? launch_project<BP, true>(a, s) : launch_project<BP, false>(a, s);
+}
+
+// project_coef: narrow blocks by groups, the others by windows
+int project(Args &a, cudaStream_t s)
+{
+    if (a.B <= kNarrow) {
+        const int smem = a.collect ? take_small(a) : 0;
+        if (a.B == 1) k_project_coef<1><<<grid_for(a.G, 1), kThreads, smem, s>>>(a);
+        else if (a.B == 2) k_project_coef<2><<<grid_for(a.G, 2), kThreads, smem, s>>>(a);
+        else k_project_coef<4><<<grid_for(a.G, 4), kThreads, smem, s>>>(a);
+    } else {
+        const int st = a.Bp == 8 ? launch_project<8>(a, s)
+                                 : (a.Bp == 16 ? launch_project<16>(a, s) : launch_project<32>(a, s));
+        if (st != HDFE_OK) return st;
+    }
+    HDFE_CUDA_TRY(cudaGetLastError());
+    hdfe_add_launches(1);
+    return HDFE_OK;
+}
+
+// reduce: explicit rows and narrow blocks by groups, the others by windows
+int reduce(Args &a, cudaStream_t s)
+{
+    if (a.streamed && a.B > kNarrow) {
+        const int st = a.Bp == 8 ? launch_spread<8>(a, s)
+                                 : (a.Bp == 16 ? launch_spread<16>(a, s) : launch_spread<32>(a, s));
+        if (st != HDFE_OK) return st;
+    } else {
+        const int smem = take_small(a);
+        if (a.B == 1) k_reduce<1><<<grid_for(a.G, 1), kThreads, smem, s>>>(a);
+        else if (a.B == 2) k_reduce<2><<<grid_for(a.G, 2), kThreads, smem, s>>>(a);
+        else if (a.B <= 4) k_reduce<4><<<grid_for(a.G, 4), kThreads, smem, s>>>(a);
+        else if (a.Bp == 8) k_reduce<8><<<grid_for(a.G, 8), kThreads, smem, s>>>(a);
+        else if (a.Bp == 16) k_reduce<16><<<grid_for(a.G, 16), kThreads, smem, s>>>(a);
+        else k_reduce<32><<<grid_for(a.G, 32), kThreads, smem, s>>>(a);
+    }
+    HDFE_CUDA_TRY(cudaGetLastError());
+    hdfe_add_launches(1);
+    return HDFE_OK;
+}
+
 }  // namespace coef
 }  // namespace hdfe
 
@@ -434,14 +1046,7 @@ extern "C" int hdfe_rows_reduce(const int64_t *starts, int64_t n_groups, const u
     a.acc = acc;
     a.acc_x = acc_x;
     a.gsum = group_sums;
-    cudaStream_t s = (cudaStream_t)stream;
-    const unsigned grid = coef::grid_for(n_groups, a.Bp);
-    if (a.Bp == 8) coef::k_reduce<8><<<grid, coef::kThreads, 0, s>>>(a);
-    else if (a.Bp == 16) coef::k_reduce<16><<<grid, coef::kThreads, 0, s>>>(a);
-    else coef::k_reduce<32><<<grid, coef::kThreads, 0, s>>>(a);
-    HDFE_CUDA_TRY(cudaGetLastError());
-    hdfe_add_launches(1);
-    return HDFE_OK;
+    return coef::reduce(a, (cudaStream_t)stream);
 }
 
 extern "C" int hdfe_rows_project_coef(const int64_t *starts, int64_t n_groups,
@@ -467,14 +1072,7 @@ extern "C" int hdfe_rows_project_coef(const int64_t *starts, int64_t n_groups,
     a.acc = acc;
     a.acc_x = acc_x;
     a.gsum = group_sums;
-    cudaStream_t s = (cudaStream_t)stream;
-    const unsigned grid = coef::grid_for(n_groups, a.Bp);
-    if (a.Bp == 8) coef::k_project_coef<8><<<grid, coef::kThreads, 0, s>>>(a);
-    else if (a.Bp == 16) coef::k_project_coef<16><<<grid, coef::kThreads, 0, s>>>(a);
-    else coef::k_project_coef<32><<<grid, coef::kThreads, 0, s>>>(a);
-    HDFE_CUDA_TRY(cudaGetLastError());
-    hdfe_add_launches(1);
-    return HDFE_OK;
+    return coef::project(a, (cudaStream_t)stream);
 }
 
 extern "C" int64_t hdfe_trace_moments_workspace_bytes(int32_t B)
@@ -517,7 +1115,7 @@ extern "C" int hdfe_trace_moments(const int64_t *starts, int64_t n_groups, const
     a.status = (unsigned *)status;
     cudaStream_t s = (cudaStream_t)stream;
     const int Bp = B <= 8 ? 8 : (B <= 16 ? 16 : 32);
-    const unsigned grid = coef::grid_for(n_groups, Bp);
+    const unsigned grid = coef::window_grid(n_groups, Bp, &a.chunk);
     if (Bp == 8) coef::k_trace<8><<<grid, coef::kThreads, 0, s>>>(a);
     else if (Bp == 16) coef::k_trace<16><<<grid, coef::kThreads, 0, s>>>(a);
     else coef::k_trace<32><<<grid, coef::kThreads, 0, s>>>(a);
@@ -562,11 +1160,5 @@ extern "C" int hdfe_stream_matvec(const int64_t *starts, int64_t n_groups, const
     a.acc = out;
     cudaStream_t s = (cudaStream_t)stream;
     HDFE_CUDA_TRY(cudaMemsetAsync(out, 0, a.L * k * 8, s));
-    const unsigned grid = coef::grid_for(n_groups, a.Bp);
-    if (a.Bp == 8) coef::k_project_coef<8><<<grid, coef::kThreads, 0, s>>>(a);
-    else if (a.Bp == 16) coef::k_project_coef<16><<<grid, coef::kThreads, 0, s>>>(a);
-    else coef::k_project_coef<32><<<grid, coef::kThreads, 0, s>>>(a);
-    HDFE_CUDA_TRY(cudaGetLastError());
-    hdfe_add_launches(1);
-    return HDFE_OK;
+    return coef::project(a, s);
 }

@@ -1,6 +1,7 @@
 #pragma once
 
 #include "rows.cuh"
+#include "windows.cuh"
 
 namespace hdfe {
 namespace rows {
@@ -36,9 +37,6 @@ __device__ __forceinline__ bool rad_negative(uint64_t seed, uint64_t rterm, uint
 }
 
 constexpr uint64_t kRowMul = 0x9E3779B97F4A7C15ull, kDrawMul = 0xBF58476D1CE4E5B9ull;
-
-constexpr int kWin = 32;                // rows of a window
-constexpr int kMaxChunk = 64;           // most groups a sub-warp takes at a time
 
 // shared memory of one sub-warp's window
 template <int BP>
@@ -131,15 +129,6 @@ __device__ __forceinline__ uint32_t window_signs(const Args &a, int64_t i0, int 
     return word;
 }
 
-__device__ __forceinline__ unsigned below(int n) { return n >= 32 ? 0xffffffffu : (1u << n) - 1u; }
-
-// the next set bit of m after q, or n
-__device__ __forceinline__ int next_bit(unsigned m, int q, int n)
-{
-    const unsigned r = q >= 31 ? 0u : m & ~below(q + 1);
-    return r ? min(__ffs(r) - 1, n) : n;
-}
-
 // gx[group, k] = the sum of w x_k over the group's rows (k < c) and of w (k =
 // c), by lane (group, k); gheads: the groups' first rows, ng of them
 template <int BP, int C, bool W>
@@ -150,9 +139,7 @@ __device__ __forceinline__ void group_sums(const Args &a, const Lanes<BP> &ln, W
         const int c = C < 0 ? a.c : C, per = W ? c + 1 : c;
         for (int t = ln.j; t < ng * per; t += BP) {
             const int g = t / per, k = t - g * per;
-            unsigned m = gheads;
-            for (int r = 0; r < g; r++) m &= m - 1;
-            const int q0 = __ffs(m) - 1, q1 = next_bit(gheads, q0, n);
+            const int q0 = nth_bit(gheads, g), q1 = next_bit(gheads, q0, n);
             double v = 0.0;
             for (int q = q0; q < q1; q++) {
                 const double xq = k < c ? wn.x[q * c + k] : 1.0;
@@ -164,43 +151,18 @@ __device__ __forceinline__ void group_sums(const Args &a, const Lanes<BP> &ln, W
     }
 }
 
-// A sub-warp's walk over its chunks of groups: window(g, i0, n, gheads, ng) for
-// each window of whole groups, lone(g, s, e) for a group of more than 32 rows.
+// the walk of this sub-warp
 template <int BP, typename F, typename H>
-__device__ __forceinline__ void walk_windows(const Args &a, const Lanes<BP> &ln, F window, H lone)
+__device__ __forceinline__ void walk(const Args &a, const Lanes<BP> &ln, F window, H lone)
 {
     constexpr int SUBS = kPassThreads / BP;
-    const int64_t sub = (int64_t)blockIdx.x * SUBS + threadIdx.x / BP;
-    const int64_t step = (int64_t)gridDim.x * SUBS * a.chunk;
-    for (int64_t ga = sub * a.chunk; ga < a.G; ga += step) {
-        const int64_t gb = min(ga + a.chunk, a.G);
-        for (int64_t g = ga; g < gb;) {
-            const int64_t s0 = a.starts[g];
-            const int64_t e = g + ln.j < gb ? a.starts[g + ln.j + 1] : INT64_MAX;
-            const bool fits = e - s0 <= kWin;
-            unsigned m = __ballot_sync(ln.mask, fits) & ln.mask;
-            m >>= (threadIdx.x & 31) / BP * BP;
-            const int ng = __popc(m);
-            if (ng == 0) {
-                lone(g, s0, a.starts[g + 1]);
-                g++;
-                continue;
-            }
-            const int n = (int)(__shfl_sync(ln.mask, e, ng - 1, BP) - s0);
-            // group t + 1 of the window starts at the end of group t
-            const unsigned mine = ln.j < ng - 1 && e - s0 < kWin ? 1u << (int)(e - s0) : 0u;
-            const unsigned gheads = __reduce_or_sync(ln.mask, mine) | 1u;
-            if (n > 0) window(g, s0, n, gheads, __popc(gheads));
-            g += ng;
-            __syncwarp(ln.mask);            // the next window reuses the staging
-        }
-    }
+    walk_windows<BP>(a.starts, a.G, a.chunk, (int64_t)blockIdx.x * SUBS + threadIdx.x / BP,
+                     (int64_t)gridDim.x * SUBS, ln.j, ln.mask, window, lone);
 }
 
 // One Rademacher pass: the kernel for the block's width, the covariates' count
 // (0 to 3 unrolled, else a loop to 8) and weights or none.  K<BP, C, W>::kernel
-// is the kernel and K::kTile whether its windows have the tile.  A sub-warp's
-// chunk is 64 groups, fewer on panels that would leave sub-warps without one.
+// is the kernel and K::kTile whether its windows have the tile.
 template <template <int, int, bool> class K, int BP, int C, bool W>
 int launch_draws(Args &a, cudaStream_t s)
 {
@@ -212,8 +174,7 @@ int launch_draws(Args &a, cudaStream_t s)
         HDFE_CUDA_TRY(cudaFuncSetAttribute(Pass::kernel(),
                                            cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     const int64_t ctas = 148 * 5;
-    const int64_t chunk = (a.G + 2 * ctas * SUBS - 1) / (2 * ctas * SUBS);
-    a.chunk = chunk < 4 ? 4 : (chunk > kMaxChunk ? kMaxChunk : chunk);
+    a.chunk = window_chunk(a.G, ctas * SUBS);
     int64_t b = (a.G + a.chunk * SUBS - 1) / (a.chunk * SUBS);
     if (b > 2 * ctas) b = 2 * ctas;
     Pass::kernel()<<<(unsigned)(b > 0 ? b : 1), kPassThreads, smem, s>>>(a);

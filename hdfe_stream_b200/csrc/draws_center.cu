@@ -117,7 +117,7 @@ __global__ void __launch_bounds__(kPassThreads) k_center_draws(Args a)
             __syncwarp(ln.mask);
         }
     };
-    walk_windows<BP>(a, ln, window, lone);
+    walk(a, ln, window, lone);
     // the covariate block and the sums of squares (the same for every draw)
     if (a.acc_x && ln.on) {
 #pragma unroll

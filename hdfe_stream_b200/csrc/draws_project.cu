@@ -163,7 +163,7 @@ __global__ void __launch_bounds__(kPassThreads) k_project_draws(Args a)
             __syncwarp(ln.mask);
         }
     };
-    walk_windows<BP>(a, ln, window, lone);
+    walk(a, ln, window, lone);
 }
 
 template <int BP, int C, bool W>
