@@ -73,6 +73,9 @@ SIGNATURES = {
                                     _vp, _vp, _vp, _vp, _vp]),
     "hdfe_rows_project_coef": (_c.c_int, [_vp, _i64, _vp, _i32, _vp, _vp, _vp, _i32, _vp, _vp,
                                           _vp, _i32, _vp, _vp, _vp, _vp, _vp, _vp, _vp, _vp]),
+    "hdfe_drop_null_workspace_bytes": (_i64, [_i64, _i32, _i32]),
+    "hdfe_drop_null": (_c.c_int, [_vp, _vp, _i64, _i32, _i32, _vp, _vp, _vp, _i64, _vp, _vp,
+                                  _vp, _vp, _vp, _vp, _i64, _vp]),
     "hdfe_trace_moments_workspace_bytes": (_i64, [_i32]),
     "hdfe_trace_moments": (_c.c_int, [_vp, _i64, _vp, _i32, _vp, _i32, _vp, _vp, _vp, _vp,
                                       _vp, _i32, _vp, _vp, _i64, _vp, _vp]),

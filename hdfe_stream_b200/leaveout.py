@@ -277,47 +277,90 @@ class InverseOperator:
 
     # ---- coefficient-space right-hand sides (inverse.py:311-460)
 
+    def _null_blocks(self):
+        """S's null space (inverse.py:376-428 `_null_space`) on the blocks of
+        entries where its vectors are constant: a component's groups (block
+        c of K), its levels of the first non-streamed dimension (K + c) and
+        each further dimension (2 K + d - 1).  Returns (component of each
+        group, of each first-dimension level (int32), K, 1 / entries per
+        component (K), the further dimensions' orthonormal vectors
+        (2 K + D - 1, D - 1)).  Built once."""
+        if getattr(self, "_null", None) is None:
+            torch = _torch()
+            from .fit import components
+            D, nl0 = len(self.nlev), int(self.nlev[0])
+            root, out = components(self.cells, 0)
+            root = root.to(torch.int64)
+            number = torch.cumsum(root == torch.arange(nl0, device=self.dev), 0) - 1
+            comp_l = number[root]
+            # inverse.py:430-437 `_group_components`: each group's first row
+            first = self.rows.codes.view(-1, D)[self.starts[:-1], 0]
+            comp_g = comp_l[first.to(torch.int64)]
+            K = int(out[0].item())
+            size = torch.cat([torch.bincount(comp_g, minlength=K),
+                              torch.bincount(comp_l, minlength=K)]).cpu().numpy().astype(float)
+            size = np.concatenate([size, self.nlev[1:].astype(float)])
+            whole = size[:K] + size[K:2 * K]
+            Q = np.zeros((2 * K + D - 1, D - 1))
+            for d in range(1, D):
+                q = np.zeros(len(size))
+                q[K:2 * K] = 1.0
+                q[2 * K + d - 1] = -1.0
+                for _ in range(2):              # Gram-Schmidt, twice for rounding
+                    over = (size[:K] * q[:K] - size[K:2 * K] * q[K:2 * K]) / whole
+                    q[:K] -= over
+                    q[K:2 * K] += over
+                    q -= Q[:, :d - 1] @ (Q[:, :d - 1].T @ (size * q))
+                Q[:, d - 1] = q / np.sqrt(size @ (q * q))
+            up = lambda x: torch.as_tensor(np.ascontiguousarray(x), device=self.dev)
+            self._null = (comp_g.to(torch.int32), comp_l.to(torch.int32), K, up(1.0 / whole),
+                          up(Q))
+        return self._null
+
     def null_space(self):
         """inverse.py:376-428 `_null_space`: an orthonormal basis of S's null
         space as (streamed (G, k), levels (L, k)) device blocks -- per
         connected component, +1 on its groups and -1 on its levels of the
         first non-streamed dimension; per further dimension, +1 across the
-        first and -1 across it.  Built once (host QR of a (G + L) x k matrix
-        of structured columns, as the reference does)."""
-        if getattr(self, "_null", None) is None:
-            torch = _torch()
-            from .fit import components, rank_components
-            cells = self.cells
-            root, _ = components(cells, 0)
-            nl0 = int(self.nlev[0])
-            cnt_first = cells.cnt[:nl0].cpu().numpy()
-            comp, n_comp = rank_components(root.cpu().numpy(), cnt_first)
-            # inverse.py:430-437 `_group_components`: each group's first row
-            first = self.rows.codes.view(-1, len(self.nlev))[self.starts[:-1], 0]
-            gcomp = comp[first.cpu().numpy().astype(np.int64)]
-            offs = np.concatenate(([0], np.cumsum(self.nlev)[:-1]))
-            vecs = []
-            for c in range(n_comp):
-                lv = np.zeros(self.L)
-                lv[offs[0]:offs[0] + nl0] = -(comp == c).astype(float)
-                vecs.append(np.concatenate([(gcomp == c).astype(float), lv]))
-            for d in range(1, len(self.nlev)):
-                lv = np.zeros(self.L)
-                lv[offs[0]:offs[0] + nl0] = 1.0
-                lv[offs[d]:offs[d] + self.nlev[d]] = -1.0
-                vecs.append(np.concatenate([np.zeros(self.G), lv]))
-            q = np.linalg.qr(np.column_stack(vecs))[0] if vecs else np.zeros((self.G + self.L, 0))
-            q = torch.as_tensor(q, device=self.dev)
-            self._null = (q[:self.G].contiguous(), q[self.G:].contiguous())
-        return self._null
+        first and -1 across it."""
+        torch = _torch()
+        comp_g, comp_l, K, inv_size, Q = self._null_blocks()
+        basis = torch.zeros((len(Q), K + Q.shape[1]), dtype=torch.float64, device=self.dev)
+        c = torch.arange(K, device=self.dev)
+        basis[c, c] = torch.sqrt(inv_size)
+        basis[K + c, c] = -torch.sqrt(inv_size)
+        basis[:, K:] = Q
+        further = [torch.full((int(n),), 2 * K + d, device=self.dev)
+                   for d, n in enumerate(self.nlev[1:])]
+        return basis[comp_g.long()], basis[torch.cat([K + comp_l.long()] + further)]
 
     def drop_null(self, levels, streamed):
-        """inverse.py:445-460 `_drop_null_component` (thin GEMMs)."""
-        qs, ql = self.null_space()
-        if ql.shape[1] == 0:
-            return levels, streamed
-        overlap = qs.T @ streamed + ql.T @ levels
-        return (levels - ql @ overlap).contiguous(), (streamed - qs @ overlap).contiguous()
+        """inverse.py:445-460 `_drop_null_component` (`hdfe_drop_null`):
+        (levels, streamed) less their part in the null space, for any number
+        of columns."""
+        torch = _torch()
+        parts = [self._drop_null(levels[:, j:j + MAX_BLOCK], streamed[:, j:j + MAX_BLOCK])
+                 for j in range(0, int(levels.shape[1]), MAX_BLOCK)]
+        return torch.cat([p[0] for p in parts], 1), torch.cat([p[1] for p in parts], 1)
+
+    def _drop_null(self, levels, streamed):
+        """`drop_null`, and the sums of squares (B) of what is left."""
+        torch = _torch()
+        lib = _lib.lib()
+        comp_g, comp_l, K, inv_size, Q = self._null_blocks()
+        levels, streamed = levels.contiguous(), streamed.contiguous()
+        B, D = int(levels.shape[1]), len(self.nlev)
+        out_l, out_s = torch.empty_like(levels), torch.empty_like(streamed)
+        norm2 = torch.empty(B, dtype=torch.float64, device=self.dev)
+        ws = torch.empty(int(lib.hdfe_drop_null_workspace_bytes(K, D, B)), dtype=torch.uint8,
+                         device=self.dev)
+        with self._phase("k_drop_null"):
+            _lib.check(lib.hdfe_drop_null(
+                levels.data_ptr(), streamed.data_ptr(), self.G, B, D, self.nlev.ctypes.data,
+                comp_g.data_ptr(), comp_l.data_ptr(), K, inv_size.data_ptr(),
+                Q.data_ptr() if D > 1 else None, out_l.data_ptr(), out_s.data_ptr(),
+                norm2.data_ptr(), ws.data_ptr(), ws.numel(), _lib.stream_handle()))
+        return out_l, out_s, norm2
 
     def _status(self):
         torch = _torch()
@@ -339,8 +382,8 @@ class InverseOperator:
             raise ValueError(f"apply_inverse: 1 <= B <= {MAX_BLOCK}")
         f64 = dict(dtype=torch.float64, device=self.dev)
         Z, schur_inv = self.border()
-        levels, streamed = self.drop_null(levels.to(**f64), streamed.to(**f64).contiguous())
-        scale = torch.sqrt((levels * levels).sum(dim=0) + (streamed * streamed).sum(dim=0))
+        levels, streamed, norm2 = self._drop_null(levels.to(**f64), streamed.to(**f64))
+        scale = torch.sqrt(norm2)
         acc = torch.zeros((self.L, B), **f64)
         acc_x = torch.zeros((max(self.c, 1), B), **f64)
         st, sh = self._status(), _lib.stream_handle()

@@ -276,6 +276,25 @@ int hdfe_rows_project_coef(const int64_t *starts, int64_t n_groups, const uint32
                            double *acc, double *acc_x, double *group_sums, void *status,
                            void *stream);
 
+/* Coefficient vectors (levels (L, B) and streamed (n_groups, B), B <= 32) less
+ * their part in the normal equations' null space (inverse.py:376-460
+ * `_null_space`, `_drop_null_component`), and the sums of squares norm2 (B) of
+ * what is left.  The null space is constant on blocks of entries: component
+ * c's groups (block c), its levels of the first dimension (n_components + c)
+ * and each further dimension d (2 n_components + d - 1).  comp_groups
+ * (n_groups) and comp_levels (n_levels[0]): components 0 .. n_components - 1;
+ * inv_size (n_components): 1 / (the component's groups + first-dimension
+ * levels); Q (2 n_components + D - 1, D - 1): the further dimensions' vectors
+ * on the blocks, orthonormal (each block weighing its entries) and orthogonal
+ * to the components' (NULL when D = 1). */
+int64_t hdfe_drop_null_workspace_bytes(int64_t n_components, int32_t D, int32_t B);
+
+int hdfe_drop_null(const double *levels, const double *streamed, int64_t n_groups, int32_t B,
+                   int32_t D, const int64_t *n_levels, const int32_t *comp_groups,
+                   const int32_t *comp_levels, int64_t n_components, const double *inv_size,
+                   const double *Q, double *out_levels, double *out_streamed, double *norm2,
+                   void *workspace, int64_t workspace_bytes, void *stream);
+
 int64_t hdfe_trace_moments_workspace_bytes(int32_t B);
 
 int hdfe_trace_moments(const int64_t *starts, int64_t n_groups, const uint32_t *codes, int32_t D,
