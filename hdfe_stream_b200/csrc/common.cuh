@@ -120,6 +120,36 @@ __device__ __forceinline__ T block_sum(T v, T *scratch)
     return total;
 }
 
+// Exclusive scan of v[0 .. n) in place by one CTA of T threads, *total = the
+// sum: each thread takes a consecutive stretch, the stretches' sums are scanned
+// by warps and then over warps.
+template <int T>
+__device__ __forceinline__ void cta_exclusive_scan(int64_t *v, int64_t n, int64_t *total)
+{
+    __shared__ int64_t s_warp[T / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t per = (n + T - 1) / T;
+    const int64_t lo = min((int64_t)threadIdx.x * per, n), hi = min(lo + per, n);
+    int64_t sum = 0;
+    for (int64_t i = lo; i < hi; i++) sum += v[i];
+    int64_t inc = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int64_t y = __shfl_up_sync(0xffffffffu, inc, o);
+        if (lane >= o) inc += y;
+    }
+    if (lane == 31) s_warp[warp] = inc;
+    __syncthreads();
+    int64_t run = inc - sum;
+    for (int k = 0; k < warp; k++) run += s_warp[k];
+    for (int64_t i = lo; i < hi; i++) {
+        const int64_t x = v[i];
+        v[i] = run;
+        run += x;
+    }
+    if (threadIdx.x == T - 1) *total = run;
+}
+
 }  // namespace hdfe
 
 #define HDFE_CUDA_TRY(expr)                                            \

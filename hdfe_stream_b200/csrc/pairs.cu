@@ -82,13 +82,11 @@ __global__ void __launch_bounds__(kThreads) k_heads(const uint32_t *a, const uin
     if (threadIdx.x == 0) tiles[blockIdx.x] = (int64_t)t;
 }
 
-// exclusive scan of the tile counts, one thread (a few thousand tiles)
-__global__ void k_scan(int64_t *tiles, int64_t nt, int64_t *total)
+// exclusive scan of the tile counts, one CTA (one thread took 37 us for the 2,075
+// tiles of 8.5M rows)
+__global__ void __launch_bounds__(1024) k_scan(int64_t *tiles, int64_t nt, int64_t *total)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int64_t run = 0;
-    for (int64_t t = 0; t < nt; t++) { const int64_t v = tiles[t]; tiles[t] = run; run += v; }
-    *total = run;
+    cta_exclusive_scan<1024>(tiles, nt, total);
 }
 
 // each pair's first row, in row order
@@ -799,7 +797,7 @@ struct Ctx {
         HDFE_CUDA_TRY(cudaMemsetAsync(P, 0, 256, s));
         const int64_t rt = (N + kTile - 1) / kTile;
         k_heads<<<(unsigned)rt, kThreads, 0, s>>>(a, b, N, tiles, status);
-        k_scan<<<1, 32, 0, s>>>(tiles, rt, P);
+        k_scan<<<1, 1024, 0, s>>>(tiles, rt, P);
         k_write<<<(unsigned)rt, kThreads, 0, s>>>(a, b, N, tiles, first);
         k_pairs<<<grid_for(N), kThreads, 0, s>>>(a, b, first, P, N, n0, n1, pa, pb, count,
                                                  status);
@@ -831,7 +829,7 @@ struct Ctx {
         k_init<<<grid_for(n), kThreads, 0, s>>>(parent, n);
         k_union<<<grid_for(N), kThreads, 0, s>>>(pa, pb, P, n0, alive, parent, status);
         k_roots<<<(unsigned)vt, kThreads, 0, s>>>(parent, alive, n, tiles);
-        k_scan<<<1, 32, 0, s>>>(tiles, vt, ncomp);
+        k_scan<<<1, 1024, 0, s>>>(tiles, vt, ncomp);
         k_number<<<(unsigned)vt, kThreads, 0, s>>>(parent, alive, n, tiles, labels);
         k_label<<<grid_for(n), kThreads, 0, s>>>(parent, alive, n, labels);
         k_resolve<<<grid_for(n), kThreads, 0, s>>>(labels, n);
@@ -916,7 +914,7 @@ extern "C" int hdfe_leave_one_out(const uint32_t *a, const uint32_t *b, int64_t 
     HDFE_CUDA_TRY(cudaMemsetAsync(c.deg, 0, n * 8, s));
     k_adj_degree<<<grid_for(N), kThreads, 0, s>>>(c.pa, c.pb, c.P, n0, alive, c.deg);
     k_tile_sums<<<(unsigned)vt, kThreads, 0, s>>>(c.deg, n, c.tiles);
-    k_scan<<<1, 32, 0, s>>>(c.tiles, vt, c.removed);
+    k_scan<<<1, 1024, 0, s>>>(c.tiles, vt, c.removed);
     k_tile_scan<<<(unsigned)vt, kThreads, 0, s>>>(c.deg, n, c.tiles, c.removed, indptr);
     HDFE_CUDA_TRY(cudaMemsetAsync(c.deg, 0, n * 8, s));
     k_adj_fill<<<grid_for(N), kThreads, 0, s>>>(c.pa, c.pb, c.P, n0, alive, indptr, c.deg,

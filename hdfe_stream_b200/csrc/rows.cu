@@ -376,12 +376,9 @@ __global__ void __launch_bounds__(kThreads) k_group_count(const uint32_t *gcode,
     if (threadIdx.x == 0) tiles[blockIdx.x] = (int64_t)t;
 }
 
-__global__ void k_group_scan(int64_t *tiles, int64_t nt, int64_t *total)
+__global__ void __launch_bounds__(1024) k_group_scan(int64_t *tiles, int64_t nt, int64_t *total)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    int64_t run = 0;
-    for (int64_t b = 0; b < nt; b++) { const int64_t v = tiles[b]; tiles[b] = run; run += v; }
-    *total = run;
+    cta_exclusive_scan<1024>(tiles, nt, total);
 }
 
 __global__ void __launch_bounds__(kThreads) k_group_write(const uint32_t *gcode, int64_t N,
@@ -507,7 +504,7 @@ extern "C" int hdfe_row_groups(const uint32_t *gcode, int64_t n_rows, int64_t *s
     const int64_t nt = (n_rows + rows::kTile - 1) / rows::kTile;
     int64_t *tiles = (int64_t *)workspace;
     rows::k_group_count<<<(unsigned)nt, rows::kThreads, 0, s>>>(gcode, n_rows, tiles);
-    rows::k_group_scan<<<1, 32, 0, s>>>(tiles, nt, n_groups);
+    rows::k_group_scan<<<1, 1024, 0, s>>>(tiles, nt, n_groups);
     rows::k_group_write<<<(unsigned)nt, rows::kThreads, 0, s>>>(gcode, n_rows, tiles, starts,
                                                                  n_groups);
     HDFE_CUDA_TRY(cudaGetLastError());

@@ -13,7 +13,7 @@ non-streamed dimension; for CRV1 on the streamed dimension its levels, which
 are nested in their own clusters, count as one.  The pairs' components come
 from the device: the streamed dimension against each other one from the
 identifying cells' union-find (`fit.components`), two non-streamed dimensions
-from their distinct code pairs (`connected.pair_components`).
+from their rows' codes (`hdfe_code_components`).
 """
 
 from __future__ import annotations
@@ -21,7 +21,6 @@ from __future__ import annotations
 import numpy as np
 
 from . import _lib
-from .connected import pair_components
 from .fit import DeviceCells, DeviceRows, components
 
 
@@ -57,31 +56,59 @@ def fe_pair_components(rows: DeviceRows, cells: DeviceCells):
     with each other, then the other pairs), as core/passes.py's pass 1
     collects them for the degrees of freedom."""
     torch = _torch()
+    lib = _lib.lib()
+    dev = rows.gcode.device
     D = rows.D
-    counts = []
-    for d in range(D):
-        _, out = components(cells, d)
-        counts.append(int(out[0].item()))
     nl = [int(x) for x in rows.n_levels]
+    outs = [components(cells, d)[1] for d in range(D)]
     for d1 in range(D):
         for d2 in range(d1 + 1, D):
-            c1 = rows.codes[:, d1].to(torch.int64)
-            c2 = rows.codes[:, d2].to(torch.int64)
-            keys = torch.unique(c1 * nl[d2] + c2)
-            a = (keys // nl[d2]).to(torch.int32).contiguous()
-            b = (keys % nl[d2]).to(torch.int32).contiguous()
-            _, _, info = pair_components(a, b, nl[d1], nl[d2])
-            counts.append(int(info["components"]))
-    return counts
+            root = torch.empty(nl[d1] + nl[d2], dtype=torch.int32, device=dev)
+            out = torch.zeros(2, dtype=torch.int64, device=dev)
+            ws = torch.empty(int(lib.hdfe_components_workspace_bytes()), dtype=torch.uint8,
+                             device=dev)
+            _lib.check(lib.hdfe_code_components(
+                rows.codes.data_ptr(), rows.n_rows, D, d1, d2, nl[d1], nl[d2], root.data_ptr(),
+                out.data_ptr(), ws.data_ptr(), ws.numel(), _lib.stream_handle()))
+            outs.append(out)
+    counts = torch.stack(outs).cpu().numpy()
+    bad = counts[counts[:, 1] != _lib.HDFE_OK]
+    if len(bad):
+        raise _lib.HDFEError(int(bad[0, 1]), "components: a level code is out of range or the "
+                             "union-find failed")
+    return [int(c) for c in counts[:, 0]]
 
 
-def row_scores(rows: DeviceRows, cells: DeviceCells, gamma, beta, with_h=False):
-    """The per-row scores w e h (N, m - 1) of pass 2 (`hdfe_row_scores`);
-    with_h: also the residualised covariates h, as (scores, h)."""
+def nested_dims(code, rows: DeviceRows, n_levels):
+    """Per dimension -- the streamed one, then the others --, whether every
+    level has its rows in one cluster of `code` (N int64)
+    (core/inference.py:242-269): `hdfe_levels_nested`, one read for all;
+    n_levels: levels per dimension, or None for one that is not asked for."""
     torch = _torch()
     lib = _lib.lib()
     dev = rows.gcode.device
-    starts, G = row_groups(rows)
+    code = code.contiguous()
+    loose = torch.ones(1 + rows.D, dtype=torch.int32, device=dev)
+    for d, nl in enumerate(n_levels):
+        if not nl:
+            continue
+        first = torch.empty(int(nl), dtype=torch.int64, device=dev)
+        at, stride = (rows.gcode.data_ptr(), 1) if d == 0 else \
+            (rows.codes.data_ptr() + 4 * (d - 1), rows.D)
+        _lib.check(lib.hdfe_levels_nested(code.data_ptr(), rows.n_rows, at, stride, int(nl),
+                                          first.data_ptr(), loose.data_ptr() + 4 * d,
+                                          _lib.stream_handle()))
+    return [v == 0 for v in loose.cpu().tolist()]
+
+
+def row_scores(rows: DeviceRows, cells: DeviceCells, gamma, beta, with_h=False, groups=None):
+    """The per-row scores w e h (N, m - 1) of pass 2 (`hdfe_row_scores`);
+    with_h: also the residualised covariates h, as (scores, h); groups: the
+    rows' `row_groups`, when the caller has them."""
+    torch = _torch()
+    lib = _lib.lib()
+    dev = rows.gcode.device
+    starts, G = groups or row_groups(rows)
     nlev = np.asarray(rows.n_levels, dtype=np.int64)
     gamma = gamma.to(dev, torch.float64).contiguous()
     beta_d = torch.as_tensor(np.asarray(beta, np.float64), device=dev)
@@ -137,7 +164,12 @@ def cluster_vcov(rows: DeviceRows, scores, Binv, k, requests, fe_names, pair_com
         col[fe_names[d + 1]] = rows.codes[:, d].to(torch.int64)
     for name, c in (extra or {}).items():
         col[name] = torch.as_tensor(c, device=dev).to(torch.int64)
-    card = {name: int(c.max().item()) + 1 if N else 0 for name, c in col.items()}
+    cards = {}
+
+    def card(name):
+        if name not in cards:
+            cards[name] = int(col[name].max().item()) + 1 if N else 0
+        return cards[name]
     G_groups = int(rows.gcode[-1].item()) + 1 if N else 0
     fe_params = {g0: G_groups}
     for d in range(D):
@@ -153,16 +185,16 @@ def cluster_vcov(rows: DeviceRows, scores, Binv, k, requests, fe_names, pair_com
         if cs == {g0}:
             kind, code, G = "seg", col[g0], G_groups
         elif len(cols) == 1 and cols[0] in fe_params:
-            kind, code, G = "fe", col[cols[0]], card[cols[0]]
+            kind, code, G = "fe", col[cols[0]], card(cols[0])
         else:
             # compose the clusters column by column, re-coding densely after
             # each step, so the packed key never exceeds (distinct so far) x
             # card[c] < 2^63 whatever the columns' cardinalities
             code, G = None, 1
             for c in cols:
-                if G * max(card[c], 1) >= 2 ** 63:
+                if G * max(card(c), 1) >= 2 ** 63:
                     raise ValueError(f"cluster request {'^'.join(cols)!r}: too many clusters")
-                key = col[c] if code is None else code * card[c] + col[c]
+                key = col[c] if code is None else code * card(c) + col[c]
                 _, code = torch.unique(key, sorted=True, return_inverse=True)
                 G = int(code.max().item()) + 1 if N else 0
             kind = "segsub" if g0 in cs else ("fe" if len(cols) == 1 else "extra")
@@ -172,20 +204,11 @@ def cluster_vcov(rows: DeviceRows, scores, Binv, k, requests, fe_names, pair_com
         else:
             S = torch.zeros((G, k), dtype=torch.float64, device=dev).index_add_(0, code, scores)
             meat = (S.T @ S).cpu().numpy()
-        nested = []
-        for d in fe_dims:
-            if cs <= {d}:
-                nested.append(d)
-                continue
-            if kind == "segsub":
-                continue
-            nl = fe_params[d]
-            lo = torch.full((nl,), N, dtype=torch.int64, device=dev).scatter_reduce_(
-                0, col[d], code, "amin")
-            hi = torch.full((nl,), -1, dtype=torch.int64, device=dev).scatter_reduce_(
-                0, col[d], code, "amax")
-            if bool((lo == hi).all().item()):
-                nested.append(d)
+        within = [False] * len(fe_dims)
+        if kind != "segsub":
+            within = nested_dims(code, rows, [None if cs <= {d} else fe_params[d]
+                                              for d in fe_dims])
+        nested = [d for d, w in zip(fe_dims, within) if w or cs <= {d}]
         cache[key_name] = (G, meat, nested, code, S)
         return cache[key_name]
 
@@ -346,9 +369,9 @@ def estimate(rows: DeviceRows, cells: DeviceCells, gamma, clusters=(), fe_names=
                 pair[(names[d1 + 1], names[d2 + 1])] = pcs[j]
                 j += 1
         if crv3 or bootcluster:
-            scores, h = row_scores(rows, cells, gamma, beta, with_h=True)
+            scores, h = row_scores(rows, cells, gamma, beta, with_h=True, groups=(starts, G))
         else:
-            scores, h = row_scores(rows, cells, gamma, beta), None
+            scores, h = row_scores(rows, cells, gamma, beta, groups=(starts, G)), None
         for req, (V, info) in cluster_vcov(rows, scores, Binv, k, clusters, names, pair,
                                            group_meat=meat_g, extra=extra, crv3=crv3, h=h,
                                            B=B, boot=bootcluster).items():

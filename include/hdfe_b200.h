@@ -190,6 +190,23 @@ int hdfe_components(const int64_t *starts, int64_t n_groups, const uint32_t *cod
                     int32_t col, int64_t n_levels, int32_t *root, int64_t *n_components,
                     void *workspace, int64_t workspace_bytes, void *stream);
 
+/* Components of two dimensions' levels joined by the rows that hold both: codes
+ * (n_rows, D), dimensions col1 (n1 levels) and col2 (n2 levels, vertices n1 +
+ * code); root (n1 + n2) and n_components, workspace as hdfe_components.  A
+ * level without rows is a component of its own. */
+int hdfe_code_components(const uint32_t *codes, int64_t n_rows, int32_t D, int32_t col1,
+                         int32_t col2, int64_t n1, int64_t n2, int32_t *root,
+                         int64_t *n_components, void *workspace, int64_t workspace_bytes,
+                         void *stream);
+
+/* Whether every level of a dimension has its rows in one cluster
+ * (core/inference.py:242-269): clusters (n_rows) >= 0, the level of row i
+ * codes[i * stride]; *loose (device) = 0 when nested, 1 when a level spans
+ * clusters or has no rows.  first (n_levels): scratch. */
+int hdfe_levels_nested(const int64_t *clusters, int64_t n_rows, const uint32_t *codes,
+                       int32_t stride, int64_t n_levels, int64_t *first, int32_t *loose,
+                       void *stream);
+
 int64_t hdfe_normalize_workspace_bytes(int64_t n_first, int32_t m);
 int hdfe_normalize(double *gamma, int32_t m, int32_t D, const int64_t *n_levels,
                    const double *obs, const int32_t *root, void *workspace,
