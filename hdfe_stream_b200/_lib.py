@@ -103,6 +103,12 @@ SIGNATURES = {
     "hdfe_sort_workspace_bytes": (_i64, [_i64]),
     "hdfe_sort_pairs": (_c.c_int, [_vp, _vp, _i64, _i32, _vp, _vp, _vp, _i64, _vp]),
     "hdfe_factorize": (_c.c_int, [_vp, _i64, _i32, _vp, _vp, _vp, _vp, _i64, _vp]),
+    "hdfe_factorize_range_workspace_bytes": (_i64, [_i64]),
+    "hdfe_factorize_range": (_c.c_int, [_vp, _i32, _i64, _i64, _i64, _vp, _vp, _vp, _vp, _i64,
+                                        _vp]),
+    "hdfe_pack_codes": (_c.c_int, [_vp, _vp, _i32, _i64, _vp, _vp]),
+    "hdfe_rows_from_order": (_c.c_int, [_vp, _i32, _i32, _i64, _vp, _vp, _vp, _i32, _vp, _vp,
+                                        _vp, _vp, _vp, _vp, _vp]),
     "hdfe_gram_workspace_bytes": (_i64, [_i64, _i32]),
     "hdfe_gram_bf16x3": (_c.c_int, [_vp, _i64, _i32, _vp, _vp, _vp, _i64, _vp]),
     "hdfe_solver_create": (_c.c_int, [_vp, _vp, _vp, _i64, _i64, _vp, _f64, _i64, _i32, _vp]),

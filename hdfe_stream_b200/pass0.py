@@ -7,14 +7,17 @@ fit keeps its intermediates; n_buckets = 1), the streamed code becoming the
 dense group code.  Here the raw columns are already on the device and both
 steps run on this library's own radix sort (csrc/sort.cu):
 
-* each id column is factorized by `hdfe_factorize` (a stable radix sort of
-  the ids' order-preserving unsigned keys with their positions, run heads,
-  a scan of the heads, the ranks scattered back); integer ids are shifted by
-  their minimum first, so only the bits their range needs are sorted;
+* each id column is factorized: integer ids of a range of at most 32 values
+  an id through a bitmap of the range (`hdfe_factorize_range`), others by
+  `hdfe_factorize` (a stable radix sort of the ids' order-preserving unsigned
+  keys with their positions, run heads, a scan of the heads, the ranks
+  scattered back; integers shifted by their minimum first, so only the bits
+  their range needs are sorted);
 * the codes are packed, most significant first, into one 64-bit key of
   ceil(log2(levels)) bits each (columns that do not fit go in further keys)
   and the rows ordered by a stable `hdfe_sort_pairs` of the keys with the
-  row positions;
+  row positions; with one key, the sorted codes are read back out of the
+  sorted keys and one kernel gathers the rest (`hdfe_rows_from_order`);
 * when two rows share every code, the variables break the tie: the order
   is rebuilt least significant key first (the last variable ... the first,
   then the code keys), each pass stable -- the same order as the host
@@ -22,6 +25,8 @@ steps run on this library's own radix sort (csrc/sort.cu):
 """
 
 from __future__ import annotations
+
+import ctypes
 
 from . import _lib
 from .fit import DeviceRows
@@ -89,34 +94,82 @@ def sort_pairs(keys, vals=None, key_bits: int = 64):
     return k_out, v_out
 
 
+# A range of ids up to this many values an id goes through the bitmap: its words
+# then stay within 4 bytes an id, half of one radix pass's keys, and in the L2.
+RANGE_PER_ID = 32
+RANGE_FREE = 1 << 20
+
+
+def _ranges(cols):
+    """(least, largest) of every integer column, one read for all; None for
+    an empty or a float one."""
+    torch = _torch()
+    at = [i for i, c in enumerate(cols) if c.numel() and not c.dtype.is_floating_point]
+    out = [None] * len(cols)
+    if at:
+        wide = [c if c.dtype in (torch.int32, torch.int64) else c.to(torch.int64)
+                for c in (cols[i] for i in at)]
+        got = torch.stack([torch.stack(torch.aminmax(c)).to(torch.int64) for c in wide])
+        for i, (lo, hi) in zip(at, got.cpu().tolist()):
+            out[i] = (lo, hi)
+    return out
+
+
+def _factorize_all(cols):
+    """[(codes int32, levels)] of id columns (`factorize`), the sizes in two
+    reads for all of them."""
+    torch = _torch()
+    lib = _lib.lib()
+    work = []                               # codes, levels buffer, count, to levels
+    for ids, ends in zip(cols, _ranges(cols)):
+        n = ids.numel()
+        if n == 0:
+            work.append((torch.zeros(0, dtype=torch.int32, device=ids.device), ids.clone(), None,
+                         None))
+            continue
+        if n > 2 ** 31 - 1:
+            raise ValueError("factorize: at most 2^31 - 1 ids")
+        codes = torch.empty(n, dtype=torch.int32, device=ids.device)
+        count = torch.zeros(1, dtype=torch.int64, device=ids.device)
+        span = None if ends is None else ends[1] - ends[0] + 1
+        if span is not None and span <= RANGE_PER_ID * n + RANGE_FREE:
+            x = ids if ids.dtype in (torch.int32, torch.int64) else ids.to(torch.int64)
+            x = x.contiguous()
+            levels = torch.empty(min(n, span), dtype=torch.int64, device=ids.device)
+            size = int(lib.hdfe_factorize_range_workspace_bytes(span))
+            ws = torch.empty(size, dtype=torch.uint8, device=ids.device)
+            _lib.check(lib.hdfe_factorize_range(x.data_ptr(), x.element_size(), n, ends[0], span,
+                                                codes.data_ptr(), levels.data_ptr(),
+                                                count.data_ptr(), ws.data_ptr(), size,
+                                                _lib.stream_handle()))
+            work.append((codes, levels, count, lambda v, t=ids.dtype: v.to(t)))
+            continue
+        if span is None:
+            keys, base, bits = order_key(ids), None, 64
+        elif span <= 2 ** 63:
+            keys, base, bits = ids.to(torch.int64) - ends[0], ends[0], max((span - 1).bit_length(), 1)
+        else:                                   # the range needs the sign bit
+            keys, base, bits = ids.to(torch.int64) ^ SIGN, None, 64
+        keys = keys.contiguous()
+        levels = torch.empty(n, dtype=torch.int64, device=ids.device)
+        ws, size = _workspace(n, ids.device)
+        _lib.check(lib.hdfe_factorize(keys.data_ptr(), n, bits, codes.data_ptr(),
+                                      levels.data_ptr(), count.data_ptr(), ws.data_ptr(),
+                                      size, _lib.stream_handle()))
+        work.append((codes, levels, count,
+                     (lambda v, t=ids.dtype, b=base: (v + b).to(t)) if base is not None
+                     else (lambda v, t=ids.dtype: _from_key(v, t))))
+    counts = [c for _, _, c, _ in work if c is not None]
+    sizes = iter(torch.cat(counts).cpu().tolist() if counts else [])
+    return [(codes, levels if count is None else back(levels[:next(sizes)]))
+            for codes, levels, count, back in work]
+
+
 def factorize(ids):
     """(codes int64, levels): the rank of each id among the sorted distinct
     ids, and those ids in order (ids' dtype)."""
     torch = _torch()
-    n = ids.numel()
-    if n == 0:
-        return torch.zeros(0, dtype=torch.int64, device=ids.device), ids.clone()
-    if n > 2 ** 31 - 1:
-        raise ValueError("factorize: at most 2^31 - 1 ids")
-    if ids.dtype.is_floating_point:
-        keys, base, bits = order_key(ids), None, 64
-    else:
-        x = ids.to(torch.int64)
-        lo, hi = (int(v) for v in torch.aminmax(x))
-        if hi - lo < 2 ** 63:
-            keys, base, bits = x - lo, lo, max((hi - lo).bit_length(), 1)
-        else:                                   # the range needs the sign bit
-            keys, base, bits = x ^ SIGN, None, 64
-    keys = keys.contiguous()
-    codes = torch.empty(n, dtype=torch.int32, device=ids.device)
-    levels = torch.empty(n, dtype=torch.int64, device=ids.device)
-    count = torch.zeros(1, dtype=torch.int64, device=ids.device)
-    ws, size = _workspace(n, ids.device)
-    _lib.check(_lib.lib().hdfe_factorize(keys.data_ptr(), n, bits, codes.data_ptr(),
-                                         levels.data_ptr(), count.data_ptr(), ws.data_ptr(),
-                                         size, _lib.stream_handle()))
-    levels = levels[:int(count.item())]
-    levels = (levels + base).to(ids.dtype) if base is not None else _from_key(levels, ids.dtype)
+    (codes, levels), = _factorize_all([ids])
     return codes.to(torch.int64), levels
 
 
@@ -157,11 +210,16 @@ def pass0(streamed, fixed_effects, V, w=None, sort_only=()):
     effects.  Returns (rows, levels): levels per column, streamed first."""
     torch = _torch()
     N = streamed.numel()
-    g, glev = factorize(streamed)
-    fe = [factorize(c) for c in fixed_effects]
-    extra = [factorize(c) for c in sort_only]
-    cols = [g] + [c for c, _ in fe] + [c for c, _ in extra]
-    sizes = [len(glev)] + [len(l) for _, l in fe] + [len(l) for _, l in extra]
+    ids = [streamed] + list(fixed_effects) + list(sort_only)
+    coded = _factorize_all(ids)
+    sizes = [len(l) for _, l in coded]
+    D = len(fixed_effects)
+    levels = [l for _, l in coded[:1 + D]]
+    rows = _rows_by_one_key(coded, sizes, D, V, w, N)
+    if rows is not None:
+        return rows, levels
+    cols = [c.to(torch.int64) for c, _ in coded]
+    g, fe = cols[0], cols[1:1 + D]
     code_keys = _packed_keys(cols, sizes)
     order = _chain(code_keys, N, g.device)
     # rows sharing every code: neighbours equal in every key after the sort
@@ -172,9 +230,50 @@ def pass0(streamed, fixed_effects, V, w=None, sort_only=()):
     if bool(same.any()):
         var_keys = [(order_key(V[:, j]), 64) for j in range(V.shape[1])]
         order = _chain(code_keys + var_keys, N, g.device)
-    codes = torch.stack([c[order] for c, _ in fe], 1).to(torch.int32).contiguous()
+    codes = torch.stack([c[order] for c in fe], 1).to(torch.int32).contiguous()
     rows = DeviceRows(g[order].to(torch.int32).contiguous(), codes,
                       V[order].T.contiguous().to(torch.float64),
                       None if w is None else w[order].to(torch.float64).contiguous(),
-                      [len(l) for _, l in fe])
-    return rows, [glev] + [l for _, l in fe]
+                      sizes[1:1 + D])
+    return rows, levels
+
+
+def _rows_by_one_key(coded, sizes, D, V, w, N):
+    """The rows when all codes pack into one key and no two rows share it:
+    one sort, the codes out of the sorted keys, one gather.  None for every
+    other form of the input (several keys, ties that the variables break, no
+    rows, columns of different lengths or devices, inputs that record
+    gradients): those take the general path."""
+    torch = _torch()
+    lib = _lib.lib()
+    bits = [_bits(n) for n in sizes]
+    dev = coded[0][0].device
+    if N == 0 or D == 0 or sum(bits) > 64 or max(bits) > 31 or len(bits) > 8:
+        return None
+    if any(c.numel() != N or c.device != dev for c, _ in coded) or V.dim() != 2 or \
+            V.shape[0] != N or V.device != dev or V.requires_grad or V.is_complex():
+        return None
+    if w is not None and (w.dim() != 1 or w.numel() != N or w.device != dev or w.requires_grad
+                          or w.is_complex()):
+        return None
+    m = int(V.shape[1])
+    cols = (ctypes.c_void_p * len(bits))(*[c.data_ptr() for c, _ in coded])
+    width = (ctypes.c_int32 * len(bits))(*bits)
+    keys = torch.empty(N, dtype=torch.int64, device=dev)
+    _lib.check(lib.hdfe_pack_codes(cols, width, len(bits), N, keys.data_ptr(),
+                                   _lib.stream_handle()))
+    keys, order = sort_pairs(keys, None, sum(bits))
+    V = V.to(torch.float64).contiguous()
+    w = None if w is None else w.to(torch.float64).contiguous()
+    gcode = torch.empty(N, dtype=torch.int32, device=dev)
+    codes = torch.empty((N, D), dtype=torch.int32, device=dev)
+    V_out = torch.empty((m, N), dtype=torch.float64, device=dev)
+    w_out = None if w is None else torch.empty(N, dtype=torch.float64, device=dev)
+    ties = torch.empty(1, dtype=torch.int32, device=dev)
+    _lib.check(lib.hdfe_rows_from_order(
+        width, len(bits), D, N, keys.data_ptr(), order.data_ptr(), V.data_ptr(), m, _lib.ptr(w),
+        gcode.data_ptr(), codes.data_ptr(), V_out.data_ptr(), _lib.ptr(w_out), ties.data_ptr(),
+        _lib.stream_handle()))
+    if int(ties.item()):
+        return None
+    return DeviceRows(gcode, codes, V_out, w_out, sizes[1:1 + D])

@@ -704,6 +704,30 @@ int hdfe_factorize(const uint64_t *ids, int64_t n, int32_t key_bits, int32_t *co
                    uint64_t *levels, int64_t *n_levels, void *workspace, int64_t workspace_bytes,
                    void *stream);
 
+/* The same for signed ids (id_bytes 4 or 8) within [lo, lo + range): a bitmap
+ * of the range instead of a sort; levels (min(n, range)) int64.  An id outside
+ * the range gets no code and is recorded in the workspace's first word.
+ *
+ * hdfe_pack_codes: keys[i] = the columns' codes packed most significant first,
+ * bits[c] <= 31 each, 64 in all (cols and bits are HOST arrays, at most 8).
+ * hdfe_rows_from_order: the rows in a sorted order of such keys: gcode and
+ * codes (n, D) out of the keys' first 1 + D columns, V_out (m, n) and w_out (n)
+ * gathered from V (n, m) and w by order; *ties (device) = 1 when two rows have
+ * the same key. */
+int64_t hdfe_factorize_range_workspace_bytes(int64_t range);
+
+int hdfe_factorize_range(const void *ids, int32_t id_bytes, int64_t n, int64_t lo, int64_t range,
+                         int32_t *codes, int64_t *levels, int64_t *n_levels, void *workspace,
+                         int64_t workspace_bytes, void *stream);
+
+int hdfe_pack_codes(const int32_t *const *cols, const int32_t *bits, int32_t n_cols, int64_t n,
+                    uint64_t *keys, void *stream);
+
+int hdfe_rows_from_order(const int32_t *bits, int32_t n_cols, int32_t D, int64_t n,
+                         const uint64_t *keys, const int32_t *order, const double *V, int32_t m,
+                         const double *w, int32_t *gcode, int32_t *codes, double *V_out,
+                         double *w_out, int32_t *ties, void *stream);
+
 /* ------------------------------------------- X' W X of a wide design
  *
  * core/inference.py:109-137 `_assemble` forms the design's cross-products
