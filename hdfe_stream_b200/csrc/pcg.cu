@@ -1020,26 +1020,32 @@ constexpr int kShortLpr = HDFE_PCG_SHORT_LPR;
 __host__ __device__ constexpr int lane_threads(int K) { return K >= 32 ? 256 : 512; }
 __host__ __device__ constexpr int lane_ru(int K) { return K >= 32 ? 4 : 2; }  // vector elements per trip
 constexpr int kLaneStages = 3;          // windows of 32 nonzeros in flight per warp
-// The FP64 block of 32 columns keeps one window in flight: its CTAs (8 warps,
-// at most 128 registers a thread) then fit two to an SM, which hides more of
-// the gathers' latency than two more windows do (the 32-probe block solve of
-// the KSS call: 103 -> 92 ms on the 1M-worker panel).
-__host__ __device__ constexpr int lane_stages(int K) { return K >= 32 ? 1 : kLaneStages; }
-__host__ __device__ constexpr int lane_ctas(int K) { return K >= 32 ? 2 : 1; }
-// its reduce_range: partials a lane (grids up to 32 x this CTAs), quantities
-// a warp at a time
-__host__ __device__ constexpr int lane_red_loads(int K) { return K >= 32 ? 16 : kRedLoads; }
-__host__ __device__ constexpr int lane_red_qw(int K) { return K >= 32 ? 2 : 4; }
+// The FP64 lane kernel's CTA, one an SM: 512 threads, or 1024 from this many
+// values a vector on.  Above, the gathers of P miss the near half of the L2 and
+// the vector phases stream, and twice the warps keep more of both in flight;
+// below, an iteration is barriers, reductions and short phases, which the
+// larger CTA only slows (L x K = 3.2M: 214 us an iteration with 512 threads, 176
+// with 1024; L x K = 0.32M: 38 against 44).
+#ifndef HDFE_PCG_PAIR_WIDE
+#define HDFE_PCG_PAIR_WIDE 1000000
+#endif
+#ifndef HDFE_PCG_PAIR_ROW_COST
+#define HDFE_PCG_PAIR_ROW_COST 8        // a row's fixed cost in the warp split, in nonzeros
+#endif
 constexpr uint8_t kRowCut = 1, kRowEmpty = 2;   // per-row flags
 // dynamic shared memory: per warp, kLaneStages x 32 gathered rows of K values
 // and their 32 matrix values
-inline int lane_smem_bytes(int K, int ns = kLaneStages)
+inline int lane_smem_bytes(int K)
 {
-    return (lane_threads(K) / 32) * ns * 32 * (K + 1) * 8;
+    return (lane_threads(K) / 32) * kLaneStages * 32 * (K + 1) * 8;
 }
 
 inline bool use_lanes(int k) { return k >= HDFE_PCG_LANE_FROM || k > 8; }
 inline int lane_width(int k) { return k <= 8 ? 8 : (k <= 16 ? 16 : 32); }
+inline int pair_threads(int64_t L, int k)
+{
+    return L * lane_width(k) >= HDFE_PCG_PAIR_WIDE ? 1024 : 512;
+}
 
 struct LaneLayout {
     int64_t r, p, ap, x, carry, part, wfirst, wlo, cut, bar, total;
@@ -1050,7 +1056,7 @@ inline LaneLayout lane_layout(int64_t L, int k, int64_t blocks)
 {
     LaneLayout o;
     const int kw = lane_width(k);
-    const int64_t warps = blocks * (lane_threads(kw) / 32);
+    const int64_t warps = blocks * (pair_threads(L, k) / 32);
     int64_t p = 0;
     auto take = [&](int64_t bytes) { int64_t at = p; p += (bytes + 255) / 256 * 256; return at; };
     o.r = take(L * kw * 8);
@@ -1270,25 +1276,200 @@ __device__ __forceinline__ void column_partials(double (&v)[N], double *scratch,
     __syncthreads();
 }
 
-template <int K>
-__global__ void __launch_bounds__(lane_threads(K), lane_ctas(K)) lane_kernel(Params a, LaneArgs x)
+// ---- the FP64 lane kernel: two columns a lane
+//
+// What bounds a wide block is the gathers of P's rows (8 K bytes a nonzero out
+// of the L2) and the instructions spent on each.  A lane holds two columns, so
+// a row of P is one 16-byte load of K / 2 lanes and 64 / K nonzeros go side by
+// side in one load instruction; the loads go straight to registers, eight
+// instructions in flight a warp, with the next chunk's indices and values
+// loaded while this one's gathers are awaited.  (Staging the gathers in shared
+// memory by cp.async, 8 bytes a lane, cost 28 instructions a nonzero and left
+// one window of 32 in flight.)  An iteration took 229 us at 32 columns on the
+// 1M-worker KSS panel (3.1M nonzeros), 41 on the 100k-worker one and 114 at 8
+// columns on the 400k-worker panel with years; now 151, 37 and 61.
+//   A warp walks its range of nonzeros in chunks of up to 32 of one row.  Cut
+// rows leave their partial sums in the carry slots as everywhere here.
+__host__ __device__ constexpr int pair_unroll(int K, int T)
 {
-    constexpr int RU = lane_ru(K);
-    extern __shared__ double s_stage[];
+    return T > 512 ? 4 : (K >= 16 ? 8 : K / 2);
+}
+
+// acc of one row (two columns a lane) summed over the side-by-side groups and
+// written, or left in the carry slots; p'Ap into dot
+template <int K>
+__device__ __forceinline__ void pair_flush(int64_t r, int64_t st, int64_t en, int64_t lo,
+                                           int64_t hi, int64_t gw, double2 acc, double2 vr,
+                                           double *out, double *carry, double2 &dot)
+{
+    constexpr int LPN = K / 2;
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int o = LPN; o < 32; o <<= 1) {
+        acc.x += __shfl_xor_sync(kFull, acc.x, o);
+        acc.y += __shfl_xor_sync(kFull, acc.y, o);
+    }
+    if (lane < LPN) {
+        dot.x += vr.x * acc.x;
+        dot.y += vr.y * acc.y;
+        double *to = st >= lo && en <= hi ? out + r * K
+                                          : carry + (gw * 2 + (st >= lo ? 1 : 0)) * K;
+        reinterpret_cast<double2 *>(to)[lane] = acc;
+    }
+}
+
+// out = S V over this warp's range of nonzeros, cut rows to the carry slots,
+// dot += V[r, col] (S V)[r, col] in lanes < K / 2
+template <int K, int T>
+__device__ void pair_spmm(const Params &a, const double *V, double *out, double *carry,
+                          double2 &dot, bool want_dot)
+{
+    constexpr int LPN = K / 2, H = 32 / LPN, U = pair_unroll(K, T);
+    const int lane = threadIdx.x & 31, cp = lane % LPN, h = lane / LPN;
+    const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    const int64_t lo = a.wlo[gw], hi = a.wlo[gw + 1];
+    if (lo >= hi) return;
+    auto chunk = [&](int64_t e, int n, int32_t &c, double &w) {     // its indices and values
+        c = 0;
+        w = 0.0;
+        if (lane < n) {
+            c = __ldcs(a.indices + e + lane);
+            w = __ldcs(a.data + e + lane);
+            if (c < 0 || c >= a.L) { GridBarrier{a.bar}.fail(HDFE_ERR_BAD_CODE); c = 0; }
+        }
+    };
+    auto own = [&](int64_t r) {                                     // V[r] for p'Ap
+        return want_dot ? reinterpret_cast<const double2 *>(V + r * K)[cp] : make_double2(0.0, 0.0);
+    };
+    int64_t r = a.wfirst[gw];
+    int64_t st = a.indptr[r];
+    int64_t rw = r;     // row-end window: lane i holds indptr[rw + 1 + i]
+    int64_t rend = rw + 1 + lane <= a.L ? a.indptr[rw + 1 + lane] : INT64_MAX;
+    int64_t en = __shfl_sync(kFull, rend, 0);
+    int64_t e = lo;
+    int n = (int)min((int64_t)32, min(en, hi) - e);
+    int32_t c;
+    double w;
+    chunk(e, n, c, w);
+    double2 vr = own(r), acc = make_double2(0.0, 0.0);
+    while (true) {
+        // the chunk after this one, in this row or the next that has nonzeros
+        const int64_t e2 = e + n;
+        int64_t r2 = r, en2 = en;
+        int n2 = 0;
+        int32_t c2 = 0;
+        double w2 = 0.0;
+        double2 vr2 = vr;
+        if (e2 < hi) {
+            while (en2 <= e2) {
+                r2++;
+                if (r2 - rw >= 32) {
+                    rw = r2;
+                    rend = rw + 1 + lane <= a.L ? a.indptr[rw + 1 + lane] : INT64_MAX;
+                }
+                en2 = __shfl_sync(kFull, rend, (int)(r2 - rw));
+            }
+            n2 = (int)min((int64_t)32, min(en2, hi) - e2);
+            chunk(e2, n2, c2, w2);
+            if (r2 != r) vr2 = own(r2);
+        }
+        for (int b = 0; b * H < n; b += U) {
+            double2 g[U];
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                const int t = (b + u) * H + h;
+                const int32_t cc = __shfl_sync(kFull, c, t & 31);
+                g[u] = make_double2(0.0, 0.0);
+                if (t < n) g[u] = reinterpret_cast<const double2 *>(V + (int64_t)cc * K)[cp];
+            }
+#pragma unroll
+            for (int u = 0; u < U; u++) {
+                if ((b + u) * H >= n) break;
+                const double wv = __shfl_sync(kFull, w, ((b + u) * H + h) & 31);
+                acc.x += wv * g[u].x;
+                acc.y += wv * g[u].y;
+            }
+        }
+        if (r2 != r || e2 >= hi) {
+            pair_flush<K>(r, st, en, lo, hi, gw, acc, vr, out, carry, dot);
+            if (e2 >= hi) return;
+            acc = make_double2(0.0, 0.0);
+            st = en;                    // rows between r and r2 are empty
+        }
+        r = r2;
+        en = en2;
+        e = e2;
+        n = n2;
+        c = c2;
+        w = w2;
+        vr = vr2;
+    }
+}
+
+// Per-CTA sums of N quantities per column: v[i] holds this thread's partials
+// of quantity i for its two columns; written as partials (q0 + i) * K + col.
+template <int K, int N>
+__device__ __forceinline__ void pair_partials(double2 (&v)[N], double *scratch, double *part,
+                                              int q0, int nb)
+{
+    constexpr int LPN = K / 2;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+#pragma unroll
+    for (int i = 0; i < N; i++)
+#pragma unroll
+        for (int o = LPN; o < 32; o <<= 1) {
+            v[i].x += __shfl_xor_sync(kFull, v[i].x, o);
+            v[i].y += __shfl_xor_sync(kFull, v[i].y, o);
+        }
+    if (lane < LPN) {
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            reinterpret_cast<double2 *>(scratch + (i * nw + warp) * K)[lane] = v[i];
+    }
+    __syncthreads();
+    for (int t = threadIdx.x; t < N * K; t += blockDim.x) {
+        const int i = t / K, c = t % K;
+        double s = 0.0;
+        for (int w = 0; w < nw; w++) s += scratch[(i * nw + w) * K + c];
+        part[(int64_t)(q0 * K + t) * nb + blockIdx.x] = s;
+    }
+    __syncthreads();
+}
+
+template <int K, int T>
+__global__ void __launch_bounds__(T, 1) lane_kernel(Params a, LaneArgs x)
+{
+    constexpr int LPN = K / 2, RU = T > 512 ? 1 : 2, QW = T > 512 ? 1 : 2;
     __shared__ double s_red[3 * K];
-    __shared__ double s_scratch[(lane_threads(K) / 32) * 3 * K];
-    __shared__ double s_bnorm[K], s_rel[K];
+    __shared__ __align__(16) double s_scratch[(T / 32) * 2 * K];
+    // the columns' scalars live in shared memory between phases: registers are
+    // what the gathers need
+    __shared__ double s_rel[K], s_bn[K], s_rz[K];
     __shared__ int s_active[K];
     GridBarrier gb{a.bar};
-    const int lane = threadIdx.x & 31, col = lane % K;
+    const int lane = threadIdx.x & 31, cp = lane % LPN, c0 = 2 * cp;
     const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t gstride = (int64_t)gridDim.x * blockDim.x;
-    const int64_t L = a.L, LK = a.L * K;
+    const int64_t L = a.L, LP = a.L * LPN;      // pairs of columns
     const int nb = gridDim.x;
     const int kc = x.k;
     double *Xw = x.Xw;
-    const bool zero_c = col >= kc || (a.zero != nullptr && a.zero[col] != 0);
-    double *stage = s_stage + (threadIdx.x >> 5) * lane_stages(K) * 32 * (K + 1);
+    const bool xal = (reinterpret_cast<uintptr_t>(Xw) & 15) == 0;   // the caller's may not be
+    auto loadX = [&](int64_t t) {
+        return xal ? reinterpret_cast<const double2 *>(Xw)[t] : make_double2(Xw[2 * t], Xw[2 * t + 1]);
+    };
+    auto storeX = [&](int64_t t, double2 v) {
+        if (xal) {
+            reinterpret_cast<double2 *>(Xw)[t] = v;
+        } else {
+            Xw[2 * t] = v.x;
+            Xw[2 * t + 1] = v.y;
+        }
+    };
+    double2 *P2 = reinterpret_cast<double2 *>(a.P), *R2 = reinterpret_cast<double2 *>(a.R);
+    const double2 *AP2 = reinterpret_cast<const double2 *>(a.AP);
+    const bool zero0 = c0 >= kc || (a.zero != nullptr && a.zero[c0] != 0);
+    const bool zero1 = c0 + 1 >= kc || (a.zero != nullptr && a.zero[c0 + 1] != 0);
 
     // ---- set-up: each warp's first row and the cut flags
     {
@@ -1302,161 +1483,225 @@ __global__ void __launch_bounds__(lane_threads(K), lane_ctas(K)) lane_kernel(Par
                        (re == rs ? kRowEmpty : 0);
         }
     }
+    // the cut row this warp finishes: its carry slots by the side-by-side groups
+    // in turn (a year's row spans tens of warps, a dependent load each), then
+    // over the groups; two columns a lane, the sum in every group
+    auto finish_cut = [&](int64_t &row, double2 &ap) {
+        const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+        const int64_t lo = a.wlo[gw], hi = a.wlo[gw + 1];
+        if (lo >= hi) return false;
+        const int64_t r = a.wfirst[gw];
+        const int64_t rs = a.indptr[r], re = a.indptr[r + 1];
+        if (!(rs < lo && re <= hi)) return false;
+        const int64_t w0 = warp_of(a, rs);
+        double2 s = make_double2(0.0, 0.0);
+#pragma unroll 4
+        for (int64_t w = w0 + lane / LPN; w <= gw; w += 32 / LPN) {
+            if (a.wlo[w] == a.wlo[w + 1]) continue;
+            const double2 v = __ldcg(
+                reinterpret_cast<const double2 *>(a.carry + (w * 2 + (w == w0 ? 1 : 0)) * K) + cp);
+            s.x += v.x;
+            s.y += v.y;
+        }
+#pragma unroll
+        for (int o = LPN; o < 32; o <<= 1) {
+            s.x += __shfl_xor_sync(kFull, s.x, o);
+            s.y += __shfl_xor_sync(kFull, s.y, o);
+        }
+        ap = s;
+        row = r;
+        return true;
+    };
     // ---- R = B - S X0 (or B), the zero and padding columns, ||B||, rz
-    double dot = 0.0;
+    double2 dot = make_double2(0.0, 0.0);
     if (a.X0 != nullptr) {
-        for (int64_t t = gtid; t < LK; t += gstride)
-            Xw[t] = zero_c ? 0.0 : a.X0[(t / K) * kc + col];
+        // the product runs on a copy in P, whose rows are aligned pairs
+        for (int64_t t = gtid; t < LP; t += gstride) {
+            const int64_t r = t / LPN;
+            const double2 v = make_double2(zero0 ? 0.0 : a.X0[r * kc + c0],
+                                           zero1 ? 0.0 : a.X0[r * kc + c0 + 1]);
+            storeX(t, v);
+            P2[t] = v;
+        }
         if (!gb.sync()) return;
-        lane_spmm<K, double, lane_stages(K)>(a, a.data, Xw, a.AP, a.carry, dot, false, stage);
+        pair_spmm<K, T>(a, a.P, a.AP, a.carry, dot, false);
         if (!gb.sync()) return;
     }
-    double rel_c = 0.0, rz_c, bnorm_c;
-    bool active_c = !zero_c;
+    bool act0 = !zero0, act1 = !zero1;
     {
-        double v[3] = {0.0, 0.0, 0.0};      // b^2, r^2, r^2 dinv
-        auto setup_row = [&](int64_t r, double ap) {
+        double2 v[3] = {};                  // b^2, r^2, r^2 dinv
+        auto setup_row = [&](int64_t r, double2 ap) {
             const double di = a.dinv[r];
-            const double b = col < kc ? a.B[r * kc + col] : 0.0;
-            double xv = 0.0, res = b;
-            if (a.X0 != nullptr) { xv = Xw[r * K + col]; res = b - ap; }
-            if (zero_c) { xv = 0.0; res = 0.0; }
-            Xw[r * K + col] = xv;
-            a.R[r * K + col] = res;
-            a.P[r * K + col] = res * di;
-            v[0] += b * b;
-            v[1] += res * res;
-            v[2] += res * res * di;
+            const int64_t t = r * LPN + cp;
+            const double2 b = make_double2(c0 < kc ? a.B[r * kc + c0] : 0.0,
+                                           c0 + 1 < kc ? a.B[r * kc + c0 + 1] : 0.0);
+            double2 xv = make_double2(0.0, 0.0), res = b;
+            if (a.X0 != nullptr) {
+                xv = loadX(t);
+                res = make_double2(b.x - ap.x, b.y - ap.y);
+            }
+            if (zero0) xv.x = res.x = 0.0;
+            if (zero1) xv.y = res.y = 0.0;
+            storeX(t, xv);
+            R2[t] = res;
+            P2[t] = make_double2(res.x * di, res.y * di);
+            v[0].x += b.x * b.x;
+            v[0].y += b.y * b.y;
+            v[1].x += res.x * res.x;
+            v[1].y += res.y * res.y;
+            v[2].x += res.x * res.x * di;
+            v[2].y += res.y * res.y * di;
         };
-        for (int64_t t = gtid; t < LK; t += gstride) {
-            const int64_t r = t / K;
+        for (int64_t t = gtid; t < LP; t += gstride) {
+            const int64_t r = t / LPN;
             const uint8_t f = a.cut[r];
             if (a.X0 != nullptr && (f & kRowCut)) continue;
-            setup_row(r, (a.X0 != nullptr && !(f & kRowEmpty)) ? a.AP[t] : 0.0);
+            setup_row(r, (a.X0 != nullptr && !(f & kRowEmpty)) ? AP2[t] : make_double2(0.0, 0.0));
         }
         if (a.X0 != nullptr) {
             int64_t r;
-            double ap;
-            if (lane_finish_cut<K>(a, a.carry, r, ap) && lane < K) setup_row(r, ap);
+            double2 ap;
+            if (finish_cut(r, ap) && lane < LPN) setup_row(r, ap);
         }
-        column_partials<K, 3>(v, s_scratch, a.part, 0, nb);
+        double2 first[2] = {v[0], v[1]}, last[1] = {v[2]};
+        pair_partials<K, 2>(first, s_scratch, a.part, 0, nb);
+        pair_partials<K, 1>(last, s_scratch, a.part, 2, nb);
         if (!gb.sync()) return;
-        reduce_range<lane_red_loads(K), lane_red_qw(K)>(a.part, 0, 3 * K, s_red);
-        const double bn = sqrt(s_red[col]);
-        bnorm_c = bn == 0.0 ? 1.0 : bn;
-        rz_c = s_red[2 * K + col];
-        if (a.X0 != nullptr) {
-            rel_c = sqrt(s_red[K + col]) / bnorm_c;
-            active_c = active_c && rel_c > a.tol;
-        }
+        reduce_range<kRedLoads, QW>(a.part, 0, 3 * K, s_red);
         if (threadIdx.x < K) {
-            s_bnorm[col] = bnorm_c;
-            s_rel[col] = rel_c;
-            s_active[col] = active_c ? 1 : 0;
+            const int c = threadIdx.x;
+            const double bn = sqrt(s_red[c]);
+            s_bn[c] = bn == 0.0 ? 1.0 : bn;
+            s_rz[c] = s_red[2 * K + c];
+            const double rel = a.X0 != nullptr ? sqrt(s_red[K + c]) / s_bn[c] : 0.0;
+            s_rel[c] = rel;
+            s_active[c] = !(c >= kc || (a.zero != nullptr && a.zero[c] != 0)) &&
+                          (a.X0 == nullptr || rel > a.tol);
         }
+        __syncthreads();
+        act0 = s_active[c0] != 0;
+        act1 = s_active[c0 + 1] != 0;
     }
-    const bool all_zero = __syncthreads_and(zero_c) != 0;
-    const bool any_active0 = __syncthreads_or(active_c) != 0;
+    const bool all_zero = __syncthreads_and(zero0 && zero1) != 0;
+    const bool any_active0 = __syncthreads_or(act0 || act1) != 0;
     int64_t it = 0;
     const bool done = all_zero || (a.X0 != nullptr && !any_active0);
     if (!done) {
         if (!gb.sync()) return;     // the set-up partials are read before phase A reuses them
         for (it = 1; it <= a.maxiter; it++) {
             // ---- A: AP = S P, p'Ap
-            dot = 0.0;
-            lane_spmm<K, double, lane_stages(K)>(a, a.data, a.P, a.AP, a.carry, dot, true, stage);
+            dot = make_double2(0.0, 0.0);
+            pair_spmm<K, T>(a, a.P, a.AP, a.carry, dot, true);
             {
-                double v[1] = {dot};
-                column_partials<K, 1>(v, s_scratch, a.part, 0, nb);
+                double2 v[1] = {dot};
+                pair_partials<K, 1>(v, s_scratch, a.part, 0, nb);
             }
             if (!gb.sync()) return;
-            reduce_range<lane_red_loads(K), lane_red_qw(K)>(a.part, 0, K, s_red);
-            const double pap = s_red[col];
-            const double alpha = (active_c && pap > 0.0) ? rz_c / pap : 0.0;
-            // ---- B: X += alpha P, R -= alpha AP, sums of R^2, R^2 dinv
-            double v[2] = {0.0, 0.0};
-            auto step_row = [&](int64_t r, double ap) {
-                const double di = a.dinv[r];
-                const int64_t t = r * K + col;
-                Xw[t] += alpha * a.P[t];
-                const double res = a.R[t] - alpha * ap;
-                a.R[t] = res;
-                v[0] += res * res;
-                v[1] += res * res * di;
+            reduce_range<kRedLoads, QW>(a.part, 0, K, s_red);
+            const double al0 = act0 && s_red[c0] > 0.0 ? s_rz[c0] / s_red[c0] : 0.0;
+            const double al1 = act1 && s_red[c0 + 1] > 0.0 ? s_rz[c0 + 1] / s_red[c0 + 1] : 0.0;
+            // ---- B: R -= alpha AP, sums of R^2, R^2 dinv
+            double2 v[2] = {};
+            auto step = [&](int64_t t, double2 rv, double2 ap, double di) {
+                rv.x -= al0 * ap.x;
+                rv.y -= al1 * ap.y;
+                R2[t] = rv;
+                v[0].x += rv.x * rv.x;
+                v[0].y += rv.y * rv.y;
+                v[1].x += rv.x * rv.x * di;
+                v[1].y += rv.y * rv.y * di;
             };
-            // RU elements per thread per trip, all loads first
-            for (int64_t t0 = gtid; t0 < LK; t0 += RU * gstride) {
-                uint8_t f[RU];
-                double ap[RU], pv[RU], xv[RU], rv[RU], di[RU];
+            // 2 RU pairs per thread per trip, all loads first
+            for (int64_t t0 = gtid; t0 < LP; t0 += 2 * RU * gstride) {
+                uint8_t f[2 * RU];
+                double2 ap[2 * RU], rv[2 * RU];
+                double di[2 * RU];
 #pragma unroll
-                for (int u = 0; u < RU; u++) {
+                for (int u = 0; u < 2 * RU; u++) {
                     const int64_t t = t0 + u * gstride;
                     f[u] = kRowCut;
-                    if (t < LK) {
-                        const int64_t r = t / K;
+                    if (t < LP) {
+                        const int64_t r = t / LPN;
                         f[u] = a.cut[r];
-                        ap[u] = a.AP[t];
-                        pv[u] = a.P[t];
-                        xv[u] = Xw[t];
-                        rv[u] = a.R[t];
+                        ap[u] = AP2[t];
+                        rv[u] = R2[t];
                         di[u] = a.dinv[r];
                     }
                 }
 #pragma unroll
-                for (int u = 0; u < RU; u++) {
+                for (int u = 0; u < 2 * RU; u++) {
                     if (f[u] & kRowCut) continue;       // also the slots past the end
-                    const int64_t t = t0 + u * gstride;
-                    Xw[t] = xv[u] + alpha * pv[u];
-                    const double res = rv[u] - alpha * ((f[u] & kRowEmpty) ? 0.0 : ap[u]);
-                    a.R[t] = res;
-                    v[0] += res * res;
-                    v[1] += res * res * di[u];
+                    step(t0 + u * gstride, rv[u],
+                         (f[u] & kRowEmpty) ? make_double2(0.0, 0.0) : ap[u], di[u]);
                 }
             }
             {
                 int64_t r;
-                double ap;
-                if (lane_finish_cut<K>(a, a.carry, r, ap) && lane < K) step_row(r, ap);
+                double2 ap;
+                if (finish_cut(r, ap) && lane < LPN) {
+                    const int64_t t = r * LPN + cp;
+                    step(t, R2[t], ap, a.dinv[r]);
+                }
             }
-            column_partials<K, 2>(v, s_scratch, a.part, 1, nb);
+            pair_partials<K, 2>(v, s_scratch, a.part, 1, nb);
             if (!gb.sync()) return;
-            reduce_range<lane_red_loads(K), lane_red_qw(K)>(a.part, K, 3 * K, s_red);
-            // ---- C: convergence, beta, P = dinv R + beta P
-            rel_c = sqrt(s_red[K + col]) / bnorm_c;
-            active_c = rel_c > a.tol;
-            if (threadIdx.x < K) {
-                s_rel[col] = rel_c;
-                s_active[col] = active_c ? 1 : 0;
+            reduce_range<kRedLoads, QW>(a.part, K, 3 * K, s_red);
+            // ---- C: convergence, beta; X += alpha P, P = dinv R + beta P (the
+            // iterate moves here, where P is read anyway)
+            const double rel0 = sqrt(s_red[K + c0]) / s_bn[c0];
+            const double rel1 = sqrt(s_red[K + c0 + 1]) / s_bn[c0 + 1];
+            act0 = rel0 > a.tol;
+            act1 = rel1 > a.tol;
+            const double rn0 = s_red[2 * K + c0], rn1 = s_red[2 * K + c0 + 1];
+            const double be0 = act0 ? rn0 / (s_rz[c0] != 0.0 ? s_rz[c0] : 1.0) : 0.0;
+            const double be1 = act1 ? rn1 / (s_rz[c0 + 1] != 0.0 ? s_rz[c0 + 1] : 1.0) : 0.0;
+            const bool more = __syncthreads_or(act0 || act1) != 0;
+            if (threadIdx.x < LPN) {        // every thread has read the old ones
+                s_rel[c0] = rel0;
+                s_rel[c0 + 1] = rel1;
+                s_active[c0] = act0 ? 1 : 0;
+                s_active[c0 + 1] = act1 ? 1 : 0;
+                s_rz[c0] = rn0;
+                s_rz[c0 + 1] = rn1;
             }
-            if (!__syncthreads_or(active_c)) break;
-            const double rzn = s_red[2 * K + col];
-            const double beta = active_c ? rzn / (rz_c != 0.0 ? rz_c : 1.0) : 0.0;
-            rz_c = rzn;
-            for (int64_t t0 = gtid; t0 < LK; t0 += RU * gstride) {
-                double rv[RU], pv[RU], di[RU];
+            for (int64_t t0 = gtid; t0 < LP; t0 += RU * gstride) {
+                double2 xv[RU], rv[RU], pv[RU];
+                double di[RU];
 #pragma unroll
                 for (int u = 0; u < RU; u++) {
                     const int64_t t = t0 + u * gstride;
-                    if (t < LK) {
-                        rv[u] = a.R[t];
-                        pv[u] = a.P[t];
-                        di[u] = a.dinv[t / K];
+                    if (t < LP) {
+                        xv[u] = loadX(t);
+                        pv[u] = P2[t];
+                        if (more) {
+                            rv[u] = R2[t];
+                            di[u] = a.dinv[t / LPN];
+                        }
                     }
                 }
 #pragma unroll
                 for (int u = 0; u < RU; u++) {
                     const int64_t t = t0 + u * gstride;
-                    if (t < LK) a.P[t] = rv[u] * di[u] + beta * pv[u];
+                    if (t >= LP) continue;
+                    storeX(t, make_double2(xv[u].x + al0 * pv[u].x, xv[u].y + al1 * pv[u].y));
+                    if (more)
+                        P2[t] = make_double2(rv[u].x * di[u] + be0 * pv[u].x,
+                                             rv[u].y * di[u] + be1 * pv[u].y);
                 }
             }
+            if (!more) break;
             if (!gb.sync()) return;
         }
         if (it > a.maxiter) it = a.maxiter;
     }
     // ---- the iterate to the caller's X (stride k)
     if (Xw != a.X) {
-        for (int64_t t = gtid; t < LK; t += gstride)
-            if (col < kc) a.X[(t / K) * kc + col] = Xw[t];
+        for (int64_t t = gtid; t < LP; t += gstride) {
+            const double2 v = loadX(t);
+            const int64_t r = t / LPN;
+            if (c0 < kc) a.X[r * kc + c0] = v.x;
+            if (c0 + 1 < kc) a.X[r * kc + c0 + 1] = v.y;
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         double mx = 0.0;
@@ -1473,44 +1718,46 @@ __global__ void __launch_bounds__(lane_threads(K), lane_ctas(K)) lane_kernel(Par
     }
 }
 
-template <int K>
+template <int K, int T>
 int lane_grid()
 {
     int dev = 0, sms = 0, per_sm = 0;
     if (cudaGetDevice(&dev) != cudaSuccess) return -1;
     if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) return -1;
-    if (cudaFuncSetAttribute(lane_kernel<K>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             lane_smem_bytes(K, lane_stages(K))) != cudaSuccess)
-        return -1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lane_kernel<K>, lane_threads(K),
-                                                      lane_smem_bytes(K, lane_stages(K))) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, lane_kernel<K, T>, T, 0) !=
         cudaSuccess)
         return -1;
-    // lane_ctas(K) CTAs per SM (fewer if they do not fit), at most as many as
-    // reduce_range sums (32 lanes x lane_red_loads(K) partials each)
-    const int want = sms * (per_sm < lane_ctas(K) ? per_sm : lane_ctas(K));
-    const int most = 32 * lane_red_loads(K);
-    return per_sm < 1 ? -1 : (want < most ? want : most);
+    // one CTA per SM, at most as many as reduce_range sums
+    const int most = 32 * kRedLoads;
+    return per_sm < 1 ? -1 : (sms < most ? sms : most);
 }
 
-int lane_grid_for(int kw)
+int lane_grid_for(int kw, int threads)
 {
-    static int cache[64][3] = {};
+    static int cache[64][6] = {};
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return -1;
-    const int i = kw == 8 ? 0 : (kw == 16 ? 1 : 2);
-    if (cache[dev][i] == 0)
-        cache[dev][i] = kw == 8 ? lane_grid<8>() : (kw == 16 ? lane_grid<16>() : lane_grid<32>());
+    const int i = (kw == 8 ? 0 : (kw == 16 ? 1 : 2)) + (threads > 512 ? 3 : 0);
+    if (cache[dev][i] == 0) {
+        switch (i) {
+        case 0: cache[dev][i] = lane_grid<8, 512>(); break;
+        case 1: cache[dev][i] = lane_grid<16, 512>(); break;
+        case 2: cache[dev][i] = lane_grid<32, 512>(); break;
+        case 3: cache[dev][i] = lane_grid<8, 1024>(); break;
+        case 4: cache[dev][i] = lane_grid<16, 1024>(); break;
+        default: cache[dev][i] = lane_grid<32, 1024>(); break;
+        }
+    }
     return cache[dev][i];
 }
 
 template <int K>
-cudaError_t launch_lanes(Params p, LaneArgs x, int blocks, cudaStream_t s)
+cudaError_t launch_lanes(Params p, LaneArgs x, int blocks, int threads, cudaStream_t s)
 {
     void *args[] = {&p, &x};
-    return cudaLaunchCooperativeKernel((const void *)lane_kernel<K>, dim3(blocks),
-                                       dim3(lane_threads(K)), args,
-                                       lane_smem_bytes(K, lane_stages(K)), s);
+    const void *kernel = threads > 512 ? (const void *)lane_kernel<K, 1024>
+                                       : (const void *)lane_kernel<K, 512>;
+    return cudaLaunchCooperativeKernel(kernel, dim3(blocks), dim3(threads), args, 0, s);
 }
 
 int solve_lanes(const int64_t *indptr, const int32_t *indices, const double *data, int64_t L,
@@ -1519,7 +1766,7 @@ int solve_lanes(const int64_t *indptr, const int32_t *indices, const double *dat
                 int64_t workspace_bytes, hdfe_pcg_info *info, cudaStream_t s)
 {
     const int kw = lane_width(k);
-    const int blocks = lane_grid_for(kw);
+    const int threads = pair_threads(L, k), blocks = lane_grid_for(kw, threads);
     if (blocks < 1) return hdfe_set_cuda_error(cudaGetLastError());
     const LaneLayout lay = lane_layout(L, k, blocks);
     if (workspace_bytes < lay.total)
@@ -1531,7 +1778,7 @@ int solve_lanes(const int64_t *indptr, const int32_t *indices, const double *dat
     p.data = data;
     p.L = L;
     p.nnz = nnz;
-    const int64_t warps = (int64_t)blocks * (lane_threads(kw) / 32);
+    const int64_t warps = (int64_t)blocks * (threads / 32);
     p.nwarps = warps;
     p.dinv = dinv;
     p.B = B;
@@ -1555,10 +1802,11 @@ int solve_lanes(const int64_t *indptr, const int32_t *indices, const double *dat
     x.k = k;
     HDFE_CUDA_TRY(cudaMemsetAsync(p.bar, 0, 16, s));
     pcg::k_partition<<<(unsigned)((p.nwarps + 256) / 256), 256, 0, s>>>(indptr, L, nnz, p.nwarps,
-                                                                      0, (int64_t *)p.wlo);
-    cudaError_t e = kw == 8 ? launch_lanes<8>(p, x, blocks, s)
-                  : kw == 16 ? launch_lanes<16>(p, x, blocks, s)
-                             : launch_lanes<32>(p, x, blocks, s);
+                                                                      HDFE_PCG_PAIR_ROW_COST,
+                                                                      (int64_t *)p.wlo);
+    cudaError_t e = kw == 8 ? launch_lanes<8>(p, x, blocks, threads, s)
+                  : kw == 16 ? launch_lanes<16>(p, x, blocks, threads, s)
+                             : launch_lanes<32>(p, x, blocks, threads, s);
     HDFE_CUDA_TRY(e);
     pcg_status_kernel<<<1, 32, 0, s>>>(p.bar, info);
     HDFE_CUDA_TRY(cudaGetLastError());
@@ -1576,7 +1824,7 @@ extern "C" int64_t hdfe_pcg_workspace_bytes(int64_t L, int64_t nnz, int32_t k)
     (void)nnz;
     if (k < 1 || k > HDFE_PCG_MAX_K || L < 0) return -1;
     if (pcg::use_lanes(k)) {
-        const int blocks = pcg::lane_grid_for(pcg::lane_width(k));
+        const int blocks = pcg::lane_grid_for(pcg::lane_width(k), pcg::pair_threads(L, k));
         return blocks < 1 ? -1 : pcg::lane_layout(L, k, blocks).total;
     }
     int blocks = pcg::grid_blocks_for(k);
