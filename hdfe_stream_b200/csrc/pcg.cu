@@ -32,6 +32,8 @@
 // fixed for a given GPU and build, so repeated solves give identical bits.
 #include <cstdio>
 #include <type_traits>
+#include <atomic>
+
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -185,6 +187,37 @@ __global__ void k_partition(const int64_t *indptr, int64_t L, int64_t nnz, int64
         at = T < first ? indptr[r] : min(indptr[r] + (T - first), indptr[r + 1]);
     }
     wlo[t] = t == nwarps ? nnz : at;
+}
+
+// What a warp knows of its range for the whole solve, kept in shared memory:
+// the nonzeros [lo, hi), the row holding the first, and the cut row that it
+// finishes (-1: none; begun by warp w0).  Found once: the chains of dependent
+// loads behind them (the ranges, the first row, a binary search over the
+// ranges) otherwise stood in every iteration's SpMM and vector phase, about
+// 0.5 and 3 us.
+struct WarpRange {
+    int64_t lo, hi, first, cut, w0;
+};
+
+__device__ __forceinline__ void find_range(const Params &a, WarpRange &wr)
+{
+    const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+    if ((threadIdx.x & 31) == 0) {
+        wr.lo = a.wlo[gw];
+        wr.hi = a.wlo[gw + 1];
+        wr.first = 0;
+        wr.cut = -1;
+        wr.w0 = 0;
+        if (wr.lo < wr.hi) {
+            wr.first = upper_bound(a.indptr, a.L + 1, wr.lo) - 1;
+            const int64_t rs = a.indptr[wr.first], re = a.indptr[wr.first + 1];
+            if (rs < wr.lo && re <= wr.hi) {
+                wr.cut = wr.first;
+                wr.w0 = warp_of(a, rs);
+            }
+        }
+    }
+    __syncwarp();
 }
 
 // Sum of partial q over all CTAs, in fixed order; lane-parallel within one
@@ -384,7 +417,7 @@ __device__ __forceinline__ void finish_row(int64_t row, const T (&acc)[K], int64
 // step order, to this warp's slots s_colw (kSmall x K, zeroed here).  Only
 // the warp holding a row's first nonzero does this for the row.
 template <int K, int VS, int VW, typename T, int LPR = 8, bool DENSE = false>
-__device__ void spmm_range(const Params &a, const T *__restrict__ vals, const T *__restrict__ V,
+__device__ void spmm_range(const Params &a, const WarpRange &wr, const T *__restrict__ vals, const T *__restrict__ V,
                            T *__restrict__ out, T *carry, double (&dot)[K], bool want_dot,
                            const double *s_ps = nullptr, double *s_colw = nullptr)
 {
@@ -394,14 +427,13 @@ __device__ void spmm_range(const Params &a, const T *__restrict__ vals, const T 
     constexpr int JPL = kSmall / LPR;   // a short row's small levels a lane
     const int lane = threadIdx.x & 31, sub = lane / LPR, sl = lane % LPR;
     const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int64_t lo = a.wlo[gw];
-    const int64_t hi = a.wlo[gw + 1];
+    const int64_t lo = wr.lo, hi = wr.hi;
     if constexpr (DENSE) {
         for (int t = lane; t < kSmall * K; t += 32) s_colw[t] = 0.0;
         __syncwarp();
     }
     if (lo >= hi) return;
-    int64_t r0 = a.wfirst[gw];
+    int64_t r0 = wr.first;
     for (;;) {
         // bounds of rows r0 .. r0+31 (lane j: row r0+j)
         const int64_t q = r0 + lane;
@@ -509,17 +541,13 @@ __device__ void spmm_range(const Params &a, const T *__restrict__ vals, const T 
 // slots in a fixed order by the warp holding the row's last nonzero.  Returns
 // true (in all lanes) when this warp finishes such a row, with its AP in ap[].
 template <int K, typename T>
-__device__ bool finish_cut_row(const Params &a, const T *carry, int64_t &row, T (&ap)[K])
+__device__ bool finish_cut_row(const Params &a, const WarpRange &wr, const T *carry, int64_t &row,
+                               T (&ap)[K])
 {
+    if (wr.cut < 0) return false;
     const int lane = threadIdx.x & 31;
     const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int64_t lo = a.wlo[gw];
-    const int64_t hi = a.wlo[gw + 1];
-    if (lo >= hi) return false;
-    const int64_t r = a.wfirst[gw];
-    const int64_t rs = a.indptr[r], re = a.indptr[r + 1];
-    if (!(rs < lo && re <= hi)) return false;
-    const int64_t w0 = warp_of(a, rs);
+    const int64_t r = wr.cut, w0 = wr.w0;
     T s[K];
 #pragma unroll
     for (int k = 0; k < K; k++) s[k] = T(0);
@@ -558,77 +586,170 @@ __device__ __forceinline__ void block_partials(double (&v)[N], double *scratch, 
     __syncthreads();
 }
 
+// ---- how the CTAs of one solve meet (pcg_kernel)
+//
+// The whole GPU: partial sums through global memory and the grid barrier.  A
+// small system: one thread-block cluster of 16 CTAs, whose hardware barrier
+// (under 1 us) replaces the grid's (2.5-3 us with its skew) and whose partial sums are
+// stored straight into every CTA's shared memory before it.  An iteration of a
+// system of a few thousand levels is three barriers, two reductions and next to
+// no work: FIT20_WAS us on the whole GPU, FIT20_NOW us on a cluster (2,010 levels, 38k
+// nonzeros, 3 columns); from about CROSSOVER nonzeros on the 16 SMs take longer than
+// the barriers they save (see kClusterWork).
+//   put(q, v): this CTA's partial of quantity q (one thread); total(q0, q1,
+// dst): after a sync, dst[q - q0] = the sum over the CTAs in a fixed order, in
+// every CTA.  A quantity's slots are written again only after two further
+// syncs, so no CTA still reads them.
+constexpr int kClusterCtas = 16;
+
+template <bool CLUSTER, int NQ>
+struct Team;
+
+template <int NQ>
+struct Team<false, NQ> {
+    struct Slots {};
+    GridBarrier gb;
+    double *part;
+    __device__ Team(const Params &a, Slots &) : gb{a.bar}, part(a.part) {}
+    __device__ __forceinline__ bool begin() const { return true; }
+    __device__ __forceinline__ bool sync() const { return gb.sync(); }
+    __device__ __forceinline__ void put(int q, double v) const
+    {
+        part[(int64_t)q * gridDim.x + blockIdx.x] = v;
+    }
+    __device__ __forceinline__ void total(int q0, int q1, double *dst) const
+    {
+        reduce_range<kRedLoads, 1>(part, q0, q1, dst - q0);
+    }
+};
+
+template <int NQ>
+struct Team<true, NQ> {
+    struct Slots { double v[NQ][kClusterCtas]; };
+    Slots &s;
+    __device__ Team(const Params &, Slots &slots) : s(slots) {}
+    // no store into another CTA's shared memory before it runs
+    __device__ __forceinline__ bool begin() const { return sync(); }
+    __device__ __forceinline__ bool sync() const
+    {
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;\n\t"
+                     "barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        return true;
+    }
+    __device__ __forceinline__ void put(int q, double v) const
+    {
+        const unsigned at = (unsigned)__cvta_generic_to_shared(&s.v[q][blockIdx.x]);
+#pragma unroll
+        for (unsigned c = 0; c < kClusterCtas; c++) {
+            unsigned to;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(at), "r"(c));
+            asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(to), "d"(v) : "memory");
+        }
+    }
+    __device__ __forceinline__ void total(int q0, int q1, double *dst) const
+    {
+        const int l = threadIdx.x % kClusterCtas;
+        for (int b = q0; b < q1; b += blockDim.x / kClusterCtas) {
+            const int q = b + threadIdx.x / kClusterCtas;
+            double t = q < q1 ? s.v[q][l] : 0.0;
+#pragma unroll
+            for (int o = kClusterCtas / 2; o > 0; o >>= 1) t += __shfl_xor_sync(kFull, t, o);
+            if (l == 0 && q < q1) dst[q - q0] = t;
+        }
+        __syncthreads();
+    }
+};
+
+// Per-CTA sums of N values per thread, put as partials q0 .. q0+N-1 of this
+// CTA: warp trees, then one thread per value over the warps in order.
+// One pair of __syncthreads for all N values.
+template <int N, typename TEAM>
+__device__ __forceinline__ void team_partials(const TEAM &team, double (&v)[N], double *scratch,
+                                              int q0)
+{
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < N; i++) v[i] = warp_sum(v[i]);
+    if (lane == 0) {
+#pragma unroll
+        for (int i = 0; i < N; i++) scratch[warp * N + i] = v[i];
+    }
+    __syncthreads();
+    if (threadIdx.x < N) {
+        double t = 0.0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); w++) t += scratch[w * N + threadIdx.x];
+        team.put(q0 + threadIdx.x, t);
+    }
+    __syncthreads();
+}
+
 // ---- the dense small block (see kSmall)
 //
 // s_ps[j * K + k] = V[Lb + j, k]: the small levels' entries of the vector
-// being multiplied, one copy per CTA.
+// being multiplied, and s_sp = small . s_ps, one copy per CTA (s_small: a.small
+// in shared memory; one thread multiplying the whole block out of global memory
+// held the CTA up for 5 us an iteration).
 template <int K, int VS>
-__device__ __forceinline__ void load_small(const Params &a, const double *V, double *s_ps)
+__device__ __forceinline__ void load_small(const Params &a, const double *V, const double *s_small,
+                                           double *s_ps, double *s_sp)
 {
-    if ((int)threadIdx.x < kSmall * K) {        // zeros past the small levels
-        const int j = threadIdx.x / K, k = threadIdx.x % K;
+    const int j = threadIdx.x / K, k = threadIdx.x % K;
+    if ((int)threadIdx.x < kSmall * K)          // zeros past the small levels
         s_ps[threadIdx.x] = j < a.ns ? V[(a.Lb + j) * VS + k] : 0.0;
-    }
     __syncthreads();
+    if ((int)threadIdx.x < kSmall * K) {
+        double q = 0.0;
+#pragma unroll
+        for (int i = 0; i < kSmall; i++) q += s_small[j * kSmall + i] * s_ps[i * K + k];
+        s_sp[threadIdx.x] = q;
+    }
 }
 
 // This CTA's column sums (over its warps, in order) to partials qc .. qc +
 // ns K - 1; with want_dot, thread k adds this CTA's share of the small rows'
 // p'Ap, ps . (its column sums) (CTA 0: also ps . small ps), to dot[k].
-template <int K>
-__device__ __forceinline__ void dense_partials(const Params &a, const double *s_ps,
-                                               double *s_col, double *s_cta, int qc, int nb,
+template <int K, typename TEAM>
+__device__ __forceinline__ void dense_partials(const Params &a, const TEAM &team,
+                                               const double *s_ps, const double *s_sp,
+                                               double *s_col, double *s_cta, int qc,
                                                double (&dot)[K], bool want_dot)
 {
     __syncthreads();
     const int t = threadIdx.x, nw = blockDim.x >> 5;
-    if (t < a.ns * K) {
+    if (t < kSmall * K) {
         double c = 0.0;
-        for (int w = 0; w < nw; w++) c += s_col[w * kSmall * K + t];
-        s_cta[t] = c;
-        a.part[(int64_t)(qc + t) * nb + blockIdx.x] = c;
+        if (t < a.ns * K) {
+            for (int w = 0; w < nw; w++) c += s_col[w * kSmall * K + t];
+            team.put(qc + t, c);
+        }
+        s_cta[t] = c + (blockIdx.x == 0 ? s_sp[t] : 0.0);
     }
     __syncthreads();
     if (want_dot && t < K) {
         double e = 0.0;
-        for (int j = 0; j < a.ns; j++) e += s_ps[j * K + t] * s_cta[j * K + t];
-        if (blockIdx.x == 0) {
-            for (int j = 0; j < a.ns; j++) {
-                double q = 0.0;
-                for (int i = 0; i < a.ns; i++) q += a.small[j * a.ns + i] * s_ps[i * K + t];
-                e += s_ps[j * K + t] * q;
-            }
-        }
+#pragma unroll
+        for (int j = 0; j < kSmall; j++) e += s_ps[j * K + t] * s_cta[j * K + t];
 #pragma unroll
         for (int k = 0; k < K; k++)
             if (t == k) dot[k] += e;
     }
 }
 
-// After the grid barrier: s_aps[j * K + k] = (S V)[Lb + j, k], the column
-// sums over all CTAs (fixed order) plus small . ps, in every CTA.
-template <int K>
-__device__ __forceinline__ void dense_small_rows(const Params &a, const double *s_ps, int qc,
-                                                 double *s_aps)
+// After the sync: s_aps[j * K + k] = (S V)[Lb + j, k], the column sums over all
+// CTAs (fixed order) plus small . ps, in every CTA.
+template <int K, typename TEAM>
+__device__ __forceinline__ void dense_small_rows(const Params &a, const TEAM &team,
+                                                 const double *s_sp, int qc, double *s_aps)
 {
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
-    for (int t = warp; t < a.ns * K; t += nw) {
-        const double v = reduce_part(a.part, qc + t);
-        if (lane == 0) s_aps[t] = v;
-    }
-    __syncthreads();
-    if ((int)threadIdx.x < a.ns * K) {
-        const int j = threadIdx.x / K, k = threadIdx.x % K;
-        double q = 0.0;
-        for (int i = 0; i < a.ns; i++) q += a.small[j * a.ns + i] * s_ps[i * K + k];
-        s_aps[threadIdx.x] += q;
-    }
+    team.total(qc, qc + a.ns * K, s_aps);
+    if ((int)threadIdx.x < a.ns * K) s_aps[threadIdx.x] += s_sp[threadIdx.x];
     __syncthreads();
 }
 
 // SPLIT: S in the split form (a.ns > 0); the kernels for the whole CSR carry
 // none of its code (and none of its registers)
-template <int K, int LPR = 8, bool SPLIT = false>
+template <int K, int LPR = 8, bool SPLIT = false, bool CLUSTER = false>
 __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
 {
     constexpr int KP = Stride<K>::P;
@@ -637,14 +758,18 @@ __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
     // the dense small block: its vector entries, this CTA's column sums, the
     // small rows' products, and the warps' column sums
     __shared__ double s_ps[kSmall * K], s_cta[kSmall * K], s_aps[kSmall * K];
+    __shared__ double s_sp[kSmall * K], s_small[SPLIT ? kSmall * kSmall : 1];
     __shared__ double s_col[kMaxWarps * kSmall * K];
     constexpr int kQc = 4 * K;          // first partial of the column sums
-    GridBarrier gb{a.bar};
+    using TeamK = Team<CLUSTER, (4 + (SPLIT ? kSmall : 0)) * K>;
+    __shared__ typename TeamK::Slots s_slots;
+    const TeamK team(a, s_slots);
+    __shared__ WarpRange s_range[kMaxWarps];
+    WarpRange &wr = s_range[threadIdx.x >> 5];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
     const int64_t gstride = (int64_t)gridDim.x * blockDim.x;
     const int64_t L = a.L;
-    const int nb = gridDim.x;
 
     double bnorm[K], rz[K], rel[K];
     bool active[K], zero[K];
@@ -655,13 +780,16 @@ __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
         rel[k] = 0.0;
     }
 
+    if (!team.begin()) return;
+    if (SPLIT)
+        for (int t = threadIdx.x; t < kSmall * kSmall; t += blockDim.x) {
+            const int j = t / kSmall, i = t % kSmall;
+            s_small[t] = j < a.ns && i < a.ns ? a.small[j * a.ns + i] : 0.0;
+        }
     // ---- set-up: each warp's first row and the cut flags (used by the same
     // warps / threads later, so no barrier is needed for them)
     {
-        const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
-        const int64_t lo = a.wlo[gw];
-        if (lane == 0 && lo < a.nnz) a.wfirst[gw] = upper_bound(a.indptr, L + 1, lo) - 1;
-        __syncwarp();
+        find_range(a, wr);
         for (int64_t r = gtid; r < L; r += gstride) {
             const int64_t rs = a.indptr[r], re = a.indptr[r + 1];
             // bit 0: the row is cut across warps; bit 1: it has no nonzeros
@@ -675,15 +803,15 @@ __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
     for (int k = 0; k < K; k++) dot[k] = 0.0;
     if (a.X0 != nullptr) {
         if ((SPLIT && a.ns > 0)) {
-            load_small<K, K>(a, a.X0, s_ps);
-            spmm_range<K, K, 1, double, LPR, true>(a, a.data, a.X0, a.AP, a.carry, dot, false,
+            load_small<K, K>(a, a.X0, s_small, s_ps, s_sp);
+            spmm_range<K, K, 1, double, LPR, true>(a, wr, a.data, a.X0, a.AP, a.carry, dot, false,
                                                    s_ps, s_col + warp * kSmall * K);
-            dense_partials<K>(a, s_ps, s_col, s_cta, kQc, nb, dot, false);
+            dense_partials<K>(a, team, s_ps, s_sp, s_col, s_cta, kQc, dot, false);
         } else {
-            spmm_range<K, K, 1, double, LPR>(a, a.data, a.X0, a.AP, a.carry, dot, false);
+            spmm_range<K, K, 1, double, LPR>(a, wr, a.data, a.X0, a.AP, a.carry, dot, false);
         }
-        if (!gb.sync()) return;
-        if ((SPLIT && a.ns > 0)) dense_small_rows<K>(a, s_ps, kQc, s_aps);
+        if (!team.sync()) return;
+        if ((SPLIT && a.ns > 0)) dense_small_rows<K>(a, team, s_sp, kQc, s_aps);
     }
     {
         double sb[K], sr[K], sz[K];
@@ -721,22 +849,16 @@ __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
         if (a.X0 != nullptr) {
             int64_t r;
             double ap[K];
-            if (finish_cut_row<K, double>(a, a.carry, r, ap) && lane == 0) setup_row(r, ap);
+            if (finish_cut_row<K, double>(a, wr, a.carry, r, ap) && lane == 0) setup_row(r, ap);
         }
         {
             double v[3 * K];
 #pragma unroll
             for (int k = 0; k < K; k++) { v[k] = sb[k]; v[K + k] = sr[k]; v[2 * K + k] = sz[k]; }
-            block_partials<3 * K>(v, s_scratch, a.part, 0, nb);
+            team_partials<3 * K>(team, v, s_scratch, 0);
         }
-        if (!gb.sync()) return;
-        if (warp < 3) {
-            for (int k = 0; k < K; k++) {
-                double t = reduce_part(a.part, warp * K + k);
-                if (lane == 0) s_red[warp * K + k] = t;
-            }
-        }
-        __syncthreads();
+        if (!team.sync()) return;
+        team.total(0, 3 * K, s_red);
     }
     bool any_active = false, all_zero = true;
 #pragma unroll
@@ -755,7 +877,7 @@ __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
     bool done = all_zero || (a.X0 != nullptr && !any_active);
     __syncthreads();
     if (!done) {
-        if (!gb.sync()) return;     // the set-up partials are read before phase A reuses them
+        if (!team.sync()) return;     // the set-up partials are read before phase A reuses them
         for (it = 1; it <= a.maxiter; it++) {
             // ---- A: AP = S P, p'Ap
 #pragma unroll
@@ -764,23 +886,17 @@ __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
             // rows for k = 3, 4
             constexpr int VWP = (KP == 4) ? 4 : ((KP % 2 == 0) ? 2 : 1);
             if ((SPLIT && a.ns > 0)) {
-                load_small<K, KP>(a, a.P, s_ps);
-                spmm_range<K, KP, VWP, double, LPR, true>(a, a.data, a.P, a.AP, a.carry, dot,
+                load_small<K, KP>(a, a.P, s_small, s_ps, s_sp);
+                spmm_range<K, KP, VWP, double, LPR, true>(a, wr, a.data, a.P, a.AP, a.carry, dot,
                                                           true, s_ps, s_col + warp * kSmall * K);
-                dense_partials<K>(a, s_ps, s_col, s_cta, kQc, nb, dot, true);
+                dense_partials<K>(a, team, s_ps, s_sp, s_col, s_cta, kQc, dot, true);
             } else {
-                spmm_range<K, KP, VWP, double, LPR>(a, a.data, a.P, a.AP, a.carry, dot, true);
+                spmm_range<K, KP, VWP, double, LPR>(a, wr, a.data, a.P, a.AP, a.carry, dot, true);
             }
-            block_partials<K>(dot, s_scratch, a.part, 0, nb);
-            if (!gb.sync()) return;
-            if (warp == 0) {
-                for (int k = 0; k < K; k++) {
-                    double t = reduce_part(a.part, k);
-                    if (lane == 0) s_red[k] = t;
-                }
-            }
-            __syncthreads();
-            if ((SPLIT && a.ns > 0)) dense_small_rows<K>(a, s_ps, kQc, s_aps);
+            team_partials<K>(team, dot, s_scratch, 0);
+            if (!team.sync()) return;
+            team.total(0, K, s_red);
+            if ((SPLIT && a.ns > 0)) dense_small_rows<K>(a, team, s_sp, kQc, s_aps);
             double alpha[K];
 #pragma unroll
             for (int k = 0; k < K; k++) {
@@ -844,22 +960,16 @@ __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
             {
                 int64_t r;
                 double ap[K];
-                if (finish_cut_row<K, double>(a, a.carry, r, ap) && lane == 0) step_row(r, ap);
+                if (finish_cut_row<K, double>(a, wr, a.carry, r, ap) && lane == 0) step_row(r, ap);
             }
             {
                 double v[2 * K];
 #pragma unroll
                 for (int k = 0; k < K; k++) { v[k] = sr[k]; v[K + k] = sz[k]; }
-                block_partials<2 * K>(v, s_scratch, a.part, K, nb);
+                team_partials<2 * K>(team, v, s_scratch, K);
             }
-            if (!gb.sync()) return;
-            if (warp < 2) {
-                for (int k = 0; k < K; k++) {
-                    double t = reduce_part(a.part, (warp + 1) * K + k);
-                    if (lane == 0) s_red[(warp + 1) * K + k] = t;
-                }
-            }
-            __syncthreads();
+            if (!team.sync()) return;
+            team.total(K, 3 * K, s_red + K);
             // ---- C: convergence, beta, P = dinv R + beta P
             any_active = false;
             double beta[K];
@@ -899,7 +1009,7 @@ __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
                     for (int k = 0; k < K; k++) a.P[r * KP + k] = rr[u][k] * di[u] + beta[k] * p[u][k];
                 }
             }
-            if (!gb.sync()) return;
+            if (!team.sync()) return;
         }
         if (it > a.maxiter) it = a.maxiter;
     }
@@ -970,12 +1080,88 @@ int grid_blocks_for(int k)
     return cache[dev][k];
 }
 
+// Systems of at most this much work (nonzeros + 16 values a row of the dense
+// cross block + 32 a row) are solved by one cluster.
+#ifndef HDFE_PCG_CLUSTER_WORK
+#define HDFE_PCG_CLUSTER_WORK 260000
+#endif
+constexpr int64_t kClusterWork = HDFE_PCG_CLUSTER_WORK;
+
+inline bool small_system(const Params &p)
+{
+    return p.nnz + (p.ns > 0 ? kSmall * p.Lb : 0) + kRowCost * p.L <= kClusterWork;
+}
+
+// one cluster of kClusterCtas CTAs of `fn`; cudaErrorNotSupported when the
+// device does not hold one
+template <typename F>
+cudaError_t launch_cluster(F fn, Params p, int threads, cudaStream_t s)
+{
+    cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+    if (e != cudaSuccess) return e;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kClusterCtas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kClusterCtas);
+    cfg.blockDim = dim3(threads);
+    cfg.stream = s;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, fn, p);
+}
+
+template <typename F>
+bool holds_cluster(F fn, int threads)
+{
+    int n = 0;
+    if (cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = kClusterCtas;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kClusterCtas);
+    cfg.blockDim = dim3(threads);
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, fn, &cfg) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return n > 0;
+}
+
+// whether the current device holds a cluster of pcg_kernel's largest variant,
+// asked once per device
+bool clusters_fit()
+{
+    static std::atomic<int> known[64];      // 0 unknown, 1 yes, 2 no
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return false;
+    int v = known[dev].load();
+    if (v == 0) {
+        v = holds_cluster(pcg_kernel<4, 8, true, true>, threads_for(4)) &&
+                    holds_cluster(pcg_kernel<1, 8, true, true>, threads_for(1))
+                ? 1 : 2;
+        known[dev].store(v);
+    }
+    return v == 1;
+}
+
 template <int K, int LPR = 8>
 cudaError_t launch(Params p, int blocks, cudaStream_t s)
 {
     void *args[] = {&p};
     const void *fn = (const void *)pcg_kernel<K, LPR, false>;
     if constexpr (K <= HDFE_PCG_SMALL_MAX_K) {
+        if (blocks == kClusterCtas)
+            return p.ns > 0 ? launch_cluster(pcg_kernel<K, LPR, true, true>, p, threads_for(K), s)
+                            : launch_cluster(pcg_kernel<K, LPR, false, true>, p, threads_for(K), s);
         if (p.ns > 0) fn = (const void *)pcg_kernel<K, LPR, true>;
     }
     return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads_for(K)), args, 0, s);
@@ -1321,13 +1507,13 @@ __device__ __forceinline__ void pair_flush(int64_t r, int64_t st, int64_t en, in
 // out = S V over this warp's range of nonzeros, cut rows to the carry slots,
 // dot += V[r, col] (S V)[r, col] in lanes < K / 2
 template <int K, int T>
-__device__ void pair_spmm(const Params &a, const double *V, double *out, double *carry,
+__device__ void pair_spmm(const Params &a, const WarpRange &wr, const double *V, double *out, double *carry,
                           double2 &dot, bool want_dot)
 {
     constexpr int LPN = K / 2, H = 32 / LPN, U = pair_unroll(K, T);
     const int lane = threadIdx.x & 31, cp = lane % LPN, h = lane / LPN;
     const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const int64_t lo = a.wlo[gw], hi = a.wlo[gw + 1];
+    const int64_t lo = wr.lo, hi = wr.hi;
     if (lo >= hi) return;
     auto chunk = [&](int64_t e, int n, int32_t &c, double &w) {     // its indices and values
         c = 0;
@@ -1341,7 +1527,7 @@ __device__ void pair_spmm(const Params &a, const double *V, double *out, double 
     auto own = [&](int64_t r) {                                     // V[r] for p'Ap
         return want_dot ? reinterpret_cast<const double2 *>(V + r * K)[cp] : make_double2(0.0, 0.0);
     };
-    int64_t r = a.wfirst[gw];
+    int64_t r = wr.first;
     int64_t st = a.indptr[r];
     int64_t rw = r;     // row-end window: lane i holds indptr[rw + 1 + i]
     int64_t rend = rw + 1 + lane <= a.L ? a.indptr[rw + 1 + lane] : INT64_MAX;
@@ -1446,6 +1632,8 @@ __global__ void __launch_bounds__(T, 1) lane_kernel(Params a, LaneArgs x)
     // what the gathers need
     __shared__ double s_rel[K], s_bn[K], s_rz[K];
     __shared__ int s_active[K];
+    __shared__ WarpRange s_range[T / 32];
+    WarpRange &wr = s_range[threadIdx.x >> 5];
     GridBarrier gb{a.bar};
     const int lane = threadIdx.x & 31, cp = lane % LPN, c0 = 2 * cp;
     const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1473,10 +1661,7 @@ __global__ void __launch_bounds__(T, 1) lane_kernel(Params a, LaneArgs x)
 
     // ---- set-up: each warp's first row and the cut flags
     {
-        const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-        const int64_t lo = a.wlo[gw];
-        if (lane == 0 && lo < a.nnz) a.wfirst[gw] = upper_bound(a.indptr, L + 1, lo) - 1;
-        __syncwarp();
+        find_range(a, wr);
         for (int64_t r = gtid; r < L; r += gstride) {
             const int64_t rs = a.indptr[r], re = a.indptr[r + 1];
             a.cut[r] = (re > rs && warp_of(a, rs) != warp_of(a, re - 1) ? kRowCut : 0) |
@@ -1487,13 +1672,9 @@ __global__ void __launch_bounds__(T, 1) lane_kernel(Params a, LaneArgs x)
     // in turn (a year's row spans tens of warps, a dependent load each), then
     // over the groups; two columns a lane, the sum in every group
     auto finish_cut = [&](int64_t &row, double2 &ap) {
+        if (wr.cut < 0) return false;
         const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-        const int64_t lo = a.wlo[gw], hi = a.wlo[gw + 1];
-        if (lo >= hi) return false;
-        const int64_t r = a.wfirst[gw];
-        const int64_t rs = a.indptr[r], re = a.indptr[r + 1];
-        if (!(rs < lo && re <= hi)) return false;
-        const int64_t w0 = warp_of(a, rs);
+        const int64_t r = wr.cut, w0 = wr.w0;
         double2 s = make_double2(0.0, 0.0);
 #pragma unroll 4
         for (int64_t w = w0 + lane / LPN; w <= gw; w += 32 / LPN) {
@@ -1524,7 +1705,7 @@ __global__ void __launch_bounds__(T, 1) lane_kernel(Params a, LaneArgs x)
             P2[t] = v;
         }
         if (!gb.sync()) return;
-        pair_spmm<K, T>(a, a.P, a.AP, a.carry, dot, false);
+        pair_spmm<K, T>(a, wr, a.P, a.AP, a.carry, dot, false);
         if (!gb.sync()) return;
     }
     bool act0 = !zero0, act1 = !zero1;
@@ -1591,7 +1772,7 @@ __global__ void __launch_bounds__(T, 1) lane_kernel(Params a, LaneArgs x)
         for (it = 1; it <= a.maxiter; it++) {
             // ---- A: AP = S P, p'Ap
             dot = make_double2(0.0, 0.0);
-            pair_spmm<K, T>(a, a.P, a.AP, a.carry, dot, true);
+            pair_spmm<K, T>(a, wr, a.P, a.AP, a.carry, dot, true);
             {
                 double2 v[1] = {dot};
                 pair_partials<K, 1>(v, s_scratch, a.part, 0, nb);
@@ -1857,6 +2038,9 @@ int solve_registers(const int64_t *indptr, const int32_t *indices, const double 
     p.ns = small_count;
     p.cross = cross;
     p.small = small;
+    if (k <= HDFE_PCG_SMALL_MAX_K && blocks > pcg::kClusterCtas && pcg::small_system(p) &&
+        pcg::clusters_fit())
+        blocks = pcg::kClusterCtas;     // one cluster (the workspace is sized for the grid)
     const int64_t warps = (int64_t)blocks * (pcg::threads_for(k) / 32);
     p.nwarps = warps;
     p.dinv = dinv;
@@ -2045,6 +2229,8 @@ __global__ void __launch_bounds__(threads_for(K), 1) mixed_kernel(Params a, Mixe
     constexpr int VWF = FStride<K>::VW;
     __shared__ double s_red[4 * K];
     __shared__ double s_scratch[kMaxWarps * 3 * K];
+    __shared__ WarpRange s_range[kMaxWarps];
+    WarpRange &wr = s_range[threadIdx.x >> 5];
     GridBarrier gb{a.bar};
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int64_t gtid = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -2063,10 +2249,7 @@ __global__ void __launch_bounds__(threads_for(K), 1) mixed_kernel(Params a, Mixe
     }
     // each warp's first row and the cut flags, X = X0 (or 0), ||B||
     {
-        const int64_t gw = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp;
-        const int64_t lo = a.wlo[gw];
-        if (lane == 0 && lo < a.nnz) a.wfirst[gw] = upper_bound(a.indptr, L + 1, lo) - 1;
-        __syncwarp();
+        find_range(a, wr);
         double sb[K];
 #pragma unroll
         for (int k = 0; k < K; k++) sb[k] = 0.0;
@@ -2104,7 +2287,7 @@ __global__ void __launch_bounds__(threads_for(K), 1) mixed_kernel(Params a, Mixe
         if (have_x) {
 #pragma unroll
             for (int k = 0; k < K; k++) dot[k] = 0.0;
-            spmm_range<K, K, 1, double>(a, a.data, a.X, f.AX, a.carry, dot, false);
+            spmm_range<K, K, 1, double>(a, wr, a.data, a.X, f.AX, a.carry, dot, false);
             if (!gb.sync()) return;
         }
         double sr[K];
@@ -2129,7 +2312,7 @@ __global__ void __launch_bounds__(threads_for(K), 1) mixed_kernel(Params a, Mixe
         if (have_x) {
             int64_t r;
             double ax[K];
-            if (finish_cut_row<K, double>(a, a.carry, r, ax) && lane == 0) resid_row(r, ax);
+            if (finish_cut_row<K, double>(a, wr, a.carry, r, ax) && lane == 0) resid_row(r, ax);
         }
         block_partials<K>(sr, s_scratch, a.part, K, nb);
         if (!gb.sync()) return;
@@ -2190,7 +2373,7 @@ __global__ void __launch_bounds__(threads_for(K), 1) mixed_kernel(Params a, Mixe
             // A: AP = S P (FP32), p'Ap in FP64
 #pragma unroll
             for (int k = 0; k < K; k++) dot[k] = 0.0;
-            spmm_range<K, KF, VWF, float>(a, f.data32, f.P, f.AP, carry32, dot, true);
+            spmm_range<K, KF, VWF, float>(a, wr, f.data32, f.P, f.AP, carry32, dot, true);
             block_partials<K>(dot, s_scratch, a.part, 0, nb);
             if (!gb.sync()) return;
             if (warp == 0) {
@@ -2234,7 +2417,7 @@ __global__ void __launch_bounds__(threads_for(K), 1) mixed_kernel(Params a, Mixe
             {
                 int64_t r;
                 float ap[K];
-                if (finish_cut_row<K, float>(a, carry32, r, ap) && lane == 0) step_row(r, ap);
+                if (finish_cut_row<K, float>(a, wr, carry32, r, ap) && lane == 0) step_row(r, ap);
             }
             {
                 double v[2 * K];
