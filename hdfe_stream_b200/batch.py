@@ -137,13 +137,12 @@ def split_work(indptr, sys_of_new, n_systems, W, long_row=LONG_ROW, fixed_cost=R
         targets = c[-1] * np.arange(nw[i]) / nw[i]
         t = np.searchsorted(c, targets, side="left")
         t = np.minimum(np.maximum.accumulate(t), len(cost))
-        nrows = b - a
         system_warps[i] = w
-        for k in range(nw[i]):
-            warp_rows[w] = a + min(int(t[k]), nrows)
-            warp_chunks[w] = ca + max(int(t[k]) - nrows, 0)
-            warp_sys[w] = i
-            w += 1
+        at = slice(w, w + int(nw[i]))
+        warp_rows[at] = a + np.minimum(t, b - a)
+        warp_chunks[at] = ca + np.maximum(t - (b - a), 0)
+        warp_sys[at] = i
+        w += int(nw[i])
     system_warps[n_systems] = w
     while w < W:                  # any warps left over own no work
         warp_rows[w] = L

@@ -52,6 +52,8 @@ constexpr int kWarpSlots = 512;                 // max hash slots per warp (warp
 constexpr int kBlockSlots = 8192;               // max hash slots per CTA (block rows)
 constexpr int kWarpListCap = 128;               // groups per warp row
 constexpr int kBlockListCap = 2048;             // groups per block row
+constexpr int kMidSlots = 2048;                 // block rows of at most this table and list
+constexpr int kMidListCap = 512;                // run six CTAs an SM (see k_block_rows)
 constexpr int32_t kEmptyKey = -1;
 constexpr int32_t kKindEmpty = -1, kKindWarp = -2, kKindBlock = -3, kKindWide = -100;
 constexpr int kWideWarp = 16;                   // wide x wide on one warp's tiles up to this W
@@ -94,7 +96,8 @@ struct Args {
     int32_t *wide_list;         // wide index -> level
     int32_t *warp_rows, *block_rows;
     int64_t *tiles;             // scan partials
-    int64_t *ctr;               // [0] W, [1] warp rows, [2] block rows, [3] lgrp len,
+    int64_t *ctr;               // [0] W, [1], [6] warp rows (small, other), [2], [8] block
+                                // rows (mid, other), [3] lgrp len,
                                 // [7] bit d: dimension d has narrow levels, bit 8 + d:
                                 // wide levels,
                                 // [4] nnz, [5] temp len
@@ -186,7 +189,13 @@ __global__ void __launch_bounds__(kThreads) k_classify(Args a)
                 a.warp_rows[a.L - 1 - (int64_t)atomicAdd((unsigned long long *)(a.ctr + 6), 1ull)] =
                     (int32_t)r;
         }
-        if (k == kKindBlock) a.block_rows[atomicAdd((unsigned long long *)(a.ctr + 2), 1ull)] = (int32_t)r;
+        if (k == kKindBlock) {
+            if (cap <= kMidSlots * 3 / 4 && lc <= kMidListCap)      // mid rows from the front
+                a.block_rows[atomicAdd((unsigned long long *)(a.ctr + 2), 1ull)] = (int32_t)r;
+            else                                                     // the others from the back
+                a.block_rows[a.L - 1 - (int64_t)atomicAdd((unsigned long long *)(a.ctr + 8), 1ull)] =
+                    (int32_t)r;
+        }
         if (k == kKindWide) {
             const int64_t wi = (int64_t)atomicAdd((unsigned long long *)a.ctr, 1ull);
             a.wide_list[wi] = (int32_t)r;
@@ -204,18 +213,23 @@ __global__ void __launch_bounds__(kThreads) k_classify(Args a)
         atomicOr(reinterpret_cast<unsigned long long *>(a.ctr + 7), (unsigned long long)dims);
 }
 
-// the wide list in level order, so wide indices do not depend on atomics
-__global__ void k_sort_wide(Args a)
+// The wide list in level order, so wide indices do not depend on atomics: each
+// level's rank among them, from a copy in rnnz (written only after the lists).
+// One CTA; one thread's insertion sort took 0.4 ms for the 240 year levels of 24
+// systems solved together.
+__global__ void __launch_bounds__(1024) k_sort_wide(Args a)
 {
-    if (threadIdx.x != 0) return;
+    int32_t *copy = reinterpret_cast<int32_t *>(a.rnnz);
     const int64_t W = a.ctr[0];
-    for (int64_t i = 1; i < W; i++) {
-        int32_t x = a.wide_list[i];
-        int64_t j = i - 1;
-        while (j >= 0 && a.wide_list[j] > x) { a.wide_list[j + 1] = a.wide_list[j]; j--; }
-        a.wide_list[j + 1] = x;
+    for (int64_t i = threadIdx.x; i < W; i += 1024) copy[i] = a.wide_list[i];
+    __syncthreads();
+    for (int64_t i = threadIdx.x; i < W; i += 1024) {
+        const int32_t x = copy[i];
+        int64_t rank = 0;
+        for (int64_t j = 0; j < W; j++) rank += copy[j] < x;
+        a.wide_list[rank] = x;
+        a.kind[x] = (int32_t)rank;
     }
-    for (int64_t i = 0; i < W; i++) a.kind[a.wide_list[i]] = (int32_t)i;
 }
 
 // ------------------------------------------------- exclusive scan (int64)
@@ -232,21 +246,7 @@ __global__ void __launch_bounds__(kThreads) k_scan_tiles(const int64_t *x, int64
 
 __global__ void __launch_bounds__(1024) k_scan_top(int64_t *tiles, int64_t nt, int64_t *total)
 {
-    __shared__ int64_t s[1024];
-    const int64_t per = (nt + blockDim.x - 1) / blockDim.x;
-    const int64_t b0 = threadIdx.x * per, b1 = min(b0 + per, nt);
-    int64_t acc = 0;
-    for (int64_t b = b0; b < b1; b++) acc += tiles[b];
-    s[threadIdx.x] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t run = 0;
-        for (unsigned t = 0; t < blockDim.x; t++) { int64_t v = s[t]; s[t] = run; run += v; }
-        *total = run;
-    }
-    __syncthreads();
-    int64_t run = s[threadIdx.x];
-    for (int64_t b = b0; b < b1; b++) { int64_t v = tiles[b]; tiles[b] = run; run += v; }
+    cta_exclusive_scan<1024>(tiles, nt, total);
 }
 
 // out[i] = exclusive prefix of x (out may alias x); out[n] = total
@@ -585,11 +585,16 @@ __device__ void narrow_row(const Args &a, int64_t r, const RowSmem &sm, int max_
     if (lane == 0) sm.loff[nl] = carry;
     __syncwarp();
     const int32_t items = carry;
+    // The row's own column takes a third to a half of its items: it is summed
+    // over the warp (a fixed tree) and joins the table once, instead of one lane
+    // adding its peers one by one every round (5M-worker panel: 1.43 -> 1.37 ms).
+    double own_sum = 0.0;
     for (int32_t base = 0; base < items; base += 32) {
         const int32_t j = base + lane;
         const bool valid = j < items;
         int64_t i = 0;
         double v = 0.0;
+        bool own = false;
         if (valid) {
             int lo = 0, hi = nl;            // last group with loff <= j
             while (hi - lo > 1) {
@@ -599,19 +604,22 @@ __device__ void narrow_row(const Args &a, int64_t r, const RowSmem &sm, int max_
             i = sm.gs[lo] + (j - sm.loff[lo]);
             const double ni = a.n[i];
             v -= ni * sm.wv[lo];
-            if (a.codes[i * a.D + dr] == lr) v += ni;
+            own = a.codes[i * a.D + dr] == lr;
+            if (own) v += ni;
         }
+        own_sum += warp_sum(own ? v : 0.0);
         for (int d = 0; d < a.D; d++) {
-            const int32_t col = valid ? (int32_t)(a.offs[d] + a.codes[i * a.D + d]) : -1;
+            const bool take = valid && !(own && d == dr);
+            const int32_t col = take ? (int32_t)(a.offs[d] + a.codes[i * a.D + d]) : -1;
             const unsigned peers = __match_any_sync(0xffffffffu, col);
             const int leader = __ffs(peers) - 1;
             sm.stage[lane] = v;
             __syncwarp();
-            if (valid && lane == leader && split && col >= a.small_first) {
+            if (take && lane == leader && split && col >= a.small_first) {
                 double sum = 0.0;
                 for (unsigned p = peers; p; p &= p - 1) sum += sm.stage[__ffs(p) - 1];
                 sm.xs[col - a.small_first] += sum;      // a direct slot, not the hash
-            } else if (valid && lane == leader) {
+            } else if (take && lane == leader) {
                 double sum = 0.0;
                 for (unsigned p = peers; p; p &= p - 1) sum += sm.stage[__ffs(p) - 1];
                 // the leaders' columns are distinct, so a slot found holding col
@@ -630,6 +638,18 @@ __device__ void narrow_row(const Args &a, int64_t r, const RowSmem &sm, int max_
             __syncwarp();
         }
     }
+    if (lane == 0 && items > 0) {       // every listed group holds the row's level
+        uint32_t h = slot_of((int32_t)r, bits);
+        for (int probe = 0; probe < slots; probe++) {
+            if (sm.keys[h] == kEmptyKey) {
+                sm.keys[h] = (int32_t)r;
+                sm.vals[h] = own_sum;
+                break;
+            }
+            h = (h + 1) & (slots - 1);
+        }
+    }
+    __syncwarp();
     // compact the table to its first slots (entries never overtake unread slots)
     if (lane == 0) *sm.cnt = 0;
     __syncwarp();
@@ -707,25 +727,32 @@ __global__ void __launch_bounds__(kWarpsPerCta * 32) k_warp_rows(Args a)
         narrow_row(a, a.warp_rows[a.L - 1 - k], sm, 9);
 }
 
-// block rows: one warp per CTA with the large table in dynamic shared memory
+// Block rows: one warp per CTA with the table in dynamic shared memory.  MID:
+// the front of block_rows, whose tables of 2048 slots let six CTAs share an SM;
+// the others' of 8192 slots take one SM each (a firm of two dozen workers with
+// ten years is just past a warp row: 581 -> 115 us for a batch of 24 systems).
+template <bool MID>
 __global__ void __launch_bounds__(32) k_block_rows(Args a)
 {
+    constexpr int kSlots = MID ? kMidSlots : kBlockSlots;
+    constexpr int kCap = MID ? kMidListCap : kBlockListCap;
     extern __shared__ unsigned char s_raw[];
     double *vals = reinterpret_cast<double *>(s_raw);
-    double *wv = vals + kBlockSlots;
-    int64_t *gs = reinterpret_cast<int64_t *>(wv + kBlockListCap);
-    int32_t *keys = reinterpret_cast<int32_t *>(gs + kBlockListCap);
-    int32_t *list = keys + kBlockSlots;
-    int32_t *loff = list + kBlockListCap;
+    double *wv = vals + kSlots;
+    int64_t *gs = reinterpret_cast<int64_t *>(wv + kCap);
+    int32_t *keys = reinterpret_cast<int32_t *>(gs + kCap);
+    int32_t *list = keys + kSlots;
+    int32_t *loff = list + kCap;
     __shared__ double s_stage[32];
     __shared__ double s_xs[kCross];
     __shared__ int s_cnt;
     RowSmem sm{s_xs, keys, vals, list, loff, gs, wv, s_stage, &s_cnt};
-    const int64_t nrows = a.ctr[2];
+    const int64_t nrows = a.ctr[MID ? 2 : 8];
     for (int64_t k = blockIdx.x; k < nrows; k += gridDim.x)
-        narrow_row(a, a.block_rows[k], sm, 13);
+        narrow_row(a, a.block_rows[MID ? k : a.L - 1 - k], sm, MID ? 11 : 13);
 }
 
+constexpr size_t kMidSmem = (size_t)kMidSlots * 12 + (size_t)kMidListCap * (8 + 8 + 4 + 4) + 16;
 constexpr size_t kBlockSmem = (size_t)kBlockSlots * 12 + (size_t)kBlockListCap * (8 + 8 + 4 + 4) + 16;
 
 // narrow rows from the temp buffer to their place in the CSR
@@ -738,10 +765,12 @@ __global__ void __launch_bounds__(kThreads) k_copy_narrow(Args a)
     const int64_t t = (int64_t)blockIdx.x * kThreads + threadIdx.x;
     const int sl = (int)(t % kCopyLanes);
     const int64_t gs = t / kCopyLanes, ns = ((int64_t)gridDim.x * kThreads) / kCopyLanes;
-    const int64_t n1 = a.ctr[1], n6 = a.ctr[6], n2 = a.ctr[2];
-    for (int64_t k = gs; k < n1 + n6 + n2; k += ns) {
+    const int64_t n1 = a.ctr[1], n6 = a.ctr[6], n2 = a.ctr[2], n8 = a.ctr[8];
+    for (int64_t k = gs; k < n1 + n6 + n2 + n8; k += ns) {
+        const int64_t q = k - n1 - n6;
         const int64_t r = k < n1 ? a.warp_rows[k]
-                        : k < n1 + n6 ? a.warp_rows[a.L - 1 - (k - n1)] : a.block_rows[k - n1 - n6];
+                        : k < n1 + n6 ? a.warp_rows[a.L - 1 - (k - n1)]
+                        : q < n2 ? a.block_rows[q] : a.block_rows[a.L - 1 - (q - n2)];
         const int64_t src = a.toff[r], dst = a.indptr[r], cnt = a.rnnz[r];
         for (int64_t i = sl; i < cnt; i += kCopyLanes) {
             a.indices[dst + i] = a.tcol[src + i];
@@ -1084,7 +1113,7 @@ __global__ void k_write_info(Args a, hdfe_sbuild_info *info)
     info->L = a.L;
     info->n_wide = a.ctr[0];
     info->n_warp_rows = a.ctr[1] + a.ctr[6];
-    info->n_block_rows = a.ctr[2];
+    info->n_block_rows = a.ctr[2] + a.ctr[8];
     info->lgrp_len = a.ctr[3];
     info->nnz = a.ctr[4];
     info->temp_len = a.ctr[5];
@@ -1116,7 +1145,7 @@ inline Layout layout(int64_t L, int64_t M, int D)
     o.warp_rows = take(L * 4);
     o.block_rows = take(L * 4);
     o.tiles = take(((L + 1) / kScanTile + 2) * 8);
-    o.ctr = take(8 * 8);
+    o.ctr = take(16 * 8);
     o.status = take(8);
     o.total = p;
     return o;
@@ -1315,7 +1344,7 @@ static int analyze_impl(const int64_t *starts, int64_t n_groups, const uint32_t 
         HDFE_CUDA_TRY(cudaMemsetAsync(b + lay.work, 0, a.L * 8, c.s));
     }
     HDFE_CUDA_TRY(cudaMemsetAsync(b + lay.fillpos, 0, a.L * 4, c.s));
-    HDFE_CUDA_TRY(cudaMemsetAsync(b + lay.ctr, 0, 64, c.s));
+    HDFE_CUDA_TRY(cudaMemsetAsync(b + lay.ctr, 0, 128, c.s));
     HDFE_CUDA_TRY(cudaMemsetAsync(b + lay.status, 0, 8, c.s));
     const int cap = c.sms * 8;
     if (!lcount) {
@@ -1323,7 +1352,7 @@ static int analyze_impl(const int64_t *starts, int64_t n_groups, const uint32_t 
         launched++;
     }
     k_classify<<<grid_for(a.L, kThreads, cap), kThreads, 0, c.s>>>(a);
-    k_sort_wide<<<1, 32, 0, c.s>>>(a);
+    k_sort_wide<<<1, 1024, 0, c.s>>>(a);
     HDFE_CUDA_TRY(cudaGetLastError());
     if ((st = scan_exclusive(c, a.lptr, a.L, a.lptr, a.ctr + 3)) != HDFE_OK) return st;
     if ((st = scan_exclusive(c, a.toff, a.L, a.toff, a.ctr + 5)) != HDFE_OK) return st;
@@ -1422,10 +1451,12 @@ static int count_impl(const int64_t *starts, int64_t n_groups, const uint32_t *c
                    c.s>>>(a);
     k_warp_rows<<<(unsigned)(c.sms * (per_warp > 0 ? per_warp : 1)), kWarpsPerCta * 32, 0,
                   c.s>>>(a);
-    HDFE_CUDA_TRY(cudaFuncSetAttribute(k_block_rows, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    HDFE_CUDA_TRY(cudaFuncSetAttribute(k_block_rows<false>,
+                                       cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)kBlockSmem));
-    k_block_rows<<<(unsigned)(c.sms), 32, kBlockSmem, c.s>>>(a);
-    launched += 3;
+    k_block_rows<true><<<(unsigned)(c.sms * 6), 32, kMidSmem, c.s>>>(a);
+    k_block_rows<false><<<(unsigned)(c.sms), 32, kBlockSmem, c.s>>>(a);
+    launched += 4;
     if (n_wide > 0) {
         if (n_wide <= kWideWarp) {
             k_wide_block_warp<<<(unsigned)a.wide_ctas, kWideThreads, 0, c.s>>>(a);
