@@ -62,6 +62,8 @@ SIGNATURES = {
     "hdfe_code_components": (_c.c_int, [_vp, _i64, _i32, _i32, _i32, _i64, _i64, _vp, _vp, _vp,
                                         _i64, _vp]),
     "hdfe_levels_nested": (_c.c_int, [_vp, _i64, _vp, _i32, _i64, _vp, _vp, _vp]),
+    "hdfe_solve_setup_workspace_bytes": (_i64, [_i32]),
+    "hdfe_solve_setup": (_c.c_int, [_vp, _vp, _i64, _i32, _vp, _f64, _vp, _vp, _vp, _i64, _vp]),
     "hdfe_normalize_workspace_bytes": (_i64, [_i64, _i32]),
     "hdfe_normalize": (_c.c_int, [_vp, _i32, _i32, _vp, _vp, _vp, _vp, _i64, _vp]),
     "hdfe_row_groups_workspace_bytes": (_i64, [_i64]),

@@ -870,14 +870,20 @@ int run(const uint32_t *gcode, const uint32_t *codes, const double *V, int m, co
     for (int d = 0; d < D; d++) if (dm.small[d] < 0) dm.small[d] = 0;
     dm.n_small = slots;
 
-    HDFE_CUDA_TRY(cudaMemsetAsync(status, 0, 8, s));
-    HDFE_CUDA_TRY(cudaMemsetAsync(obs, 0, L * 8, s));
-    HDFE_CUDA_TRY(cudaMemsetAsync(cnt, 0, L * 8, s));
-    HDFE_CUDA_TRY(cudaMemsetAsync(diag, 0, L * 8, s));
-    if (m > 0) HDFE_CUDA_TRY(cudaMemsetAsync(rhs, 0, L * m * 8, s));
-    if (lcount) {
-        HDFE_CUDA_TRY(cudaMemsetAsync(lcount, 0, L * 4, s));
-        HDFE_CUDA_TRY(cudaMemsetAsync(work, 0, L * 8, s));
+    // group tiles: G <= N, sized on the worst case (the counts are on the device)
+    const int64_t gtiles = (N + kGroupTile - 1) / kGroupTile;
+    {
+        hdfe_zero_list z;
+        z.add(status, 8);
+        z.add(obs, L * 8);
+        z.add(cnt, L * 8);
+        z.add(diag, L * 8);
+        z.add(rhs, m > 0 ? L * m * 8 : 0);
+        z.add(lcount, lcount ? L * 4 : 0);
+        z.add(work, lcount ? L * 8 : 0);
+        z.add(gtile, (gtiles + 1) * 2 * 8);
+        const int st = hdfe_zero(z, s);
+        if (st != HDFE_OK) return st;
     }
     const int64_t rtiles = (N + kRowTile - 1) / kRowTile;
     RowArgs ra{gcode, codes, V, N, m, tile_cnt, tile_mom, status};
@@ -887,9 +893,6 @@ int run(const uint32_t *gcode, const uint32_t *codes, const double *V, int m, co
     HDFE_CUDA_TRY(cudaGetLastError());
     rows_index<D><<<(unsigned)rtiles, kThreads, 0, s>>>(ra, tile_cnt, grow, gcell, totals);
     HDFE_CUDA_TRY(cudaGetLastError());
-    // group tiles: G <= N, sized on the worst case (the counts are on the device)
-    const int64_t gtiles = (N + kGroupTile - 1) / kGroupTile;
-    HDFE_CUDA_TRY(cudaMemsetAsync(gtile, 0, (gtiles + 1) * 2 * 8, s));
     groups_count<<<(unsigned)gtiles, kThreads, 0, s>>>(gcell, totals, gtile);
     HDFE_CUDA_TRY(cudaGetLastError());
     scan_tiles<<<1, 1024, 0, s>>>(gtile, gtiles, 2, totals + 2, nullptr, 0, 0, nullptr, nullptr);

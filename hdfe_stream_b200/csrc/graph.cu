@@ -173,6 +173,7 @@ __global__ void __launch_bounds__(kCompThreads, 2) k_components(CompArgs a)
     const int64_t t0 = (int64_t)blockIdx.x * kCompThreads + threadIdx.x;
     const int64_t step = (int64_t)gridDim.x * kCompThreads;
     int32_t *parent = a.parent;
+    if (t0 == 0) *a.n_roots = 0;
     for (int64_t i = t0; i < a.nlev; i += step) parent[i] = (int32_t)i;
     if (!a.bar.sync()) return;
     for (int r = 0; r < kRounds; r++) {
@@ -333,6 +334,51 @@ __global__ void __launch_bounds__(kThreads) k_dim_apply(const double *part, int 
         for (int j = 0; j < m; j++) gamma[l * m + j] -= s_mean[j];
 }
 
+// ------------------------------------------------------------ solve set-up
+
+// What step 2 does before its PCG, in two launches instead of ten array
+// operations and a host read: dinv = 1 / diag (0 up to 1e-12, core/solve.py:
+// 142-146), and per right-hand side the sum of squares, a CTA's columns in
+// part[column * CTAs + CTA].
+constexpr int kSetupCtas = 148;
+
+__global__ void __launch_bounds__(kThreads) k_setup(const double *diag, const double *rhs,
+                                                    int64_t L, int m, double *dinv, double *part)
+{
+    __shared__ double s_red[kThreads / 32];
+    const int64_t t0 = (int64_t)blockIdx.x * kThreads + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * kThreads;
+    for (int64_t l = t0; l < L; l += step) {
+        const double d = diag[l];
+        dinv[l] = d > 1e-12 ? 1.0 / d : 0.0;
+    }
+    for (int j = 0; j < m; j++) {
+        double s = 0.0;
+        for (int64_t l = t0; l < L; l += step) {
+            const double v = rhs[l * m + j];
+            s += v * v;
+        }
+        s = block_sum(s, s_red);
+        if (threadIdx.x == 0) part[j * gridDim.x + blockIdx.x] = s;
+    }
+}
+
+// zero[j] = ||rhs_j|| <= tol sqrt(max(raw_ss_j, 0)) (core/solve.py:294-320), a
+// warp per column, the CTAs in a fixed order
+__global__ void __launch_bounds__(kThreads) k_zero_columns(const double *part, int ctas, int m,
+                                                           const double *raw_ss, double tol,
+                                                           uint8_t *zero)
+{
+    const int lane = threadIdx.x & 31;
+    for (int j = threadIdx.x >> 5; j < m; j += kThreads / 32) {
+        double s = 0.0;
+        for (int b = lane; b < ctas; b += 32) s += part[j * ctas + b];
+        s = warp_sum(s);
+        const double ss = raw_ss[j] < 0.0 ? 0.0 : raw_ss[j];
+        if (lane == 0) zero[j] = sqrt(s) <= tol * sqrt(ss) ? 1 : 0;
+    }
+}
+
 // From this many windows of 32 groups the rounds take one in four: below, a
 // window a warp is one wave and sampling saves nothing.
 constexpr int64_t kSampleFrom = 16384;
@@ -364,11 +410,11 @@ inline unsigned grid_for(int64_t n)
 template <bool ROWS>
 int launch_components(CompArgs &a, int64_t *n_components, void *workspace, cudaStream_t s)
 {
-    // the barrier's three words (its error word is the status) and the count
+    // the barrier's three words; its error word is the status, a bad code's too
     a.status = (unsigned *)workspace + 2;
-    a.n_roots = (unsigned long long *)((char *)workspace + 64);
+    a.n_roots = (unsigned long long *)n_components;
     a.bar = GridBarrier{(unsigned *)workspace};
-    HDFE_CUDA_TRY(cudaMemsetAsync(workspace, 0, 128, s));
+    HDFE_CUDA_TRY(cudaMemsetAsync(workspace, 0, 16, s));
     const int64_t windows = (a.G + 31) / 32;
     a.sample = windows >= kSampleFrom ? 4 : 1;
     const int64_t most = resident_ctas<ROWS>();
@@ -385,10 +431,8 @@ int launch_components(CompArgs &a, int64_t *n_components, void *workspace, cudaS
                                               dim3(kCompThreads), args, 0, s));
     HDFE_CUDA_TRY(cudaGetLastError());
     hdfe_add_launches(1);
-    // n_components[0] = roots, n_components[1] = status
-    HDFE_CUDA_TRY(cudaMemcpyAsync(n_components, a.n_roots, 8, cudaMemcpyDeviceToDevice, s));
-    HDFE_CUDA_TRY(cudaMemsetAsync(n_components + 1, 0, 8, s));
-    HDFE_CUDA_TRY(cudaMemcpyAsync(n_components + 1, a.status, 4, cudaMemcpyDeviceToDevice, s));
+    // n_components[1] = the status and the zero word after it
+    HDFE_CUDA_TRY(cudaMemcpyAsync(n_components + 1, a.status, 8, cudaMemcpyDeviceToDevice, s));
     return HDFE_OK;
 }
 
@@ -462,6 +506,32 @@ extern "C" int hdfe_levels_nested(const int64_t *clusters, int64_t n_rows, const
     graph::k_unseen<<<graph::grid_for(n_levels), graph::kThreads, 0, s>>>(first, n_levels, loose);
     HDFE_CUDA_TRY(cudaGetLastError());
     hdfe_add_launches(3);
+    return HDFE_OK;
+}
+
+extern "C" int64_t hdfe_solve_setup_workspace_bytes(int32_t m)
+{
+    if (m < 1) return -1;
+    return (int64_t)graph::kSetupCtas * m * 8;
+}
+
+extern "C" int hdfe_solve_setup(const double *diag, const double *rhs, int64_t L, int32_t m,
+                                const double *raw_ss, double tol, double *dinv, uint8_t *zero,
+                                void *workspace, int64_t workspace_bytes, void *stream)
+{
+    if (!diag || !rhs || L < 1 || m < 1 || !raw_ss || !dinv || !zero ||
+        !workspace)
+        return hdfe_set_arg_error("hdfe_solve_setup: bad argument");
+    if (workspace_bytes < hdfe_solve_setup_workspace_bytes(m))
+        return hdfe_set_error(HDFE_ERR_WORKSPACE, "hdfe_solve_setup: workspace too small");
+    cudaStream_t s = (cudaStream_t)stream;
+    double *part = (double *)workspace;
+    const unsigned g = graph::grid_for(L);
+    const int ctas = g < graph::kSetupCtas ? (int)g : graph::kSetupCtas;
+    graph::k_setup<<<ctas, graph::kThreads, 0, s>>>(diag, rhs, L, m, dinv, part);
+    graph::k_zero_columns<<<1, graph::kThreads, 0, s>>>(part, ctas, m, raw_ss, tol, zero);
+    HDFE_CUDA_TRY(cudaGetLastError());
+    hdfe_add_launches(2);
     return HDFE_OK;
 }
 

@@ -593,9 +593,10 @@ __device__ __forceinline__ void block_partials(double (&v)[N], double *scratch, 
 // (under 1 us) replaces the grid's (2.5-3 us with its skew) and whose partial sums are
 // stored straight into every CTA's shared memory before it.  An iteration of a
 // system of a few thousand levels is three barriers, two reductions and next to
-// no work: FIT20_WAS us on the whole GPU, FIT20_NOW us on a cluster (2,010 levels, 38k
-// nonzeros, 3 columns); from about CROSSOVER nonzeros on the 16 SMs take longer than
-// the barriers they save (see kClusterWork).
+// no work: 22 us on the whole GPU, 17 on a cluster (2,010 levels with the years
+// split off, 38k nonzeros, 3 columns); from about 90,000 nonzeros on (23.7 us
+// against 23.3 at 86k, 24.7 against 30 at 134k) the 16 SMs take longer than
+// the barriers they save.
 //   put(q, v): this CTA's partial of quantity q (one thread); total(q0, q1,
 // dst): after a sync, dst[q - q0] = the sum over the CTAs in a fixed order, in
 // every CTA.  A quantity's slots are written again only after two further

@@ -1339,13 +1339,15 @@ static int analyze_impl(const int64_t *starts, int64_t n_groups, const uint32_t 
     Layout lay = layout(a.L, n_cells, D);
     char *b = (char *)workspace;
     int launched = 0;
-    if (!lcount) {
-        HDFE_CUDA_TRY(cudaMemsetAsync(b + lay.lcount, 0, a.L * 4, c.s));
-        HDFE_CUDA_TRY(cudaMemsetAsync(b + lay.work, 0, a.L * 8, c.s));
+    {
+        hdfe_zero_list z;
+        z.add(b + lay.lcount, lcount ? 0 : a.L * 4);
+        z.add(b + lay.work, lcount ? 0 : a.L * 8);
+        z.add(b + lay.fillpos, a.L * 4);
+        z.add(b + lay.ctr, 128);
+        z.add(b + lay.status, 8);
+        if ((st = hdfe_zero(z, c.s)) != HDFE_OK) return st;
     }
-    HDFE_CUDA_TRY(cudaMemsetAsync(b + lay.fillpos, 0, a.L * 4, c.s));
-    HDFE_CUDA_TRY(cudaMemsetAsync(b + lay.ctr, 0, 128, c.s));
-    HDFE_CUDA_TRY(cudaMemsetAsync(b + lay.status, 0, 8, c.s));
     const int cap = c.sms * 8;
     if (!lcount) {
         k_level_stats<<<grid_for(a.G, kThreads, cap), kThreads, 0, c.s>>>(a);
@@ -1424,22 +1426,26 @@ static int count_impl(const int64_t *starts, int64_t n_groups, const uint32_t *c
     Args &a = c.a;
     a.indptr = indptr;
     int launched = 0;
-    if (split) {
-        HDFE_CUDA_TRY(cudaMemsetAsync(cross, 0, small_first * kCross * 8, c.s));
-        HDFE_CUDA_TRY(cudaMemsetAsync(small, 0, (int64_t)small_count * small_count * 8, c.s));
-    }
-    if (n_wide > 0) {
-        WideLayout wl = wide_layout(n_wide, a.L, a.M, a.D, a.wide_ctas);
-        if (!split)     // the dense wide rows (the split form writes cross instead)
-            HDFE_CUDA_TRY(cudaMemsetAsync(wide_workspace, 0, wl.dpres + n_wide * a.L, c.s));
-        HDFE_CUDA_TRY(cudaMemsetAsync((char *)wide_workspace + wl.wcross, 0,
-                                      n_wide * n_wide * 8, c.s));
+    {
+        hdfe_zero_list z;
+        if (split) {
+            z.add(cross, small_first * kCross * 8);
+            z.add(small, (int64_t)small_count * small_count * 8);
+        }
+        if (n_wide > 0) {
+            WideLayout wl = wide_layout(n_wide, a.L, a.M, a.D, a.wide_ctas);
+            // the dense wide rows (the split form writes cross instead); their
+            // flags are bytes, rounded up within their own 256-byte block
+            if (!split) z.add(wide_workspace, wl.dpres + (n_wide * a.L + 3) / 4 * 4);
+            z.add((char *)wide_workspace + wl.wcross, n_wide * n_wide * 8);
+        }
+        z.add(a.rnnz, (a.L + 1) * 8);
+        if ((st = hdfe_zero(z, c.s)) != HDFE_OK) return st;
         if (n_wide > kWideWarp) {       // the atomic wide block reads each cell's wide index
             k_cell_widx<<<grid_for(a.M * a.D, kThreads, c.sms * 8), kThreads, 0, c.s>>>(a);
             launched++;
         }
     }
-    HDFE_CUDA_TRY(cudaMemsetAsync(a.rnnz, 0, (a.L + 1) * 8, c.s));
     // one wave: as many CTAs as stay resident (the rows are grid-strided, so a
     // second partial wave would run its share of rows after the first)
     int per_small = 0, per_warp = 0;

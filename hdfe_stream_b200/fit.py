@@ -126,7 +126,7 @@ def pass1(rows: DeviceRows, keep_sums: bool = False, stream=None) -> DeviceCells
     rhs = torch.empty((L, m), **f64)
     lcount = torch.empty(L, dtype=torch.int32, device=dev)
     work = torch.empty(L, dtype=torch.int64, device=dev)
-    counts = torch.zeros(6, dtype=torch.int64, device=dev)
+    counts = torch.empty(6, dtype=torch.int64, device=dev)
     _lib.check(lib.hdfe_pass1(
         rows.gcode.data_ptr(), rows.codes.data_ptr(), D, rows.V.data_ptr(), m,
         None if rows.w is None else rows.w.data_ptr(), N, nlev.ctypes.data, means_buf.data_ptr(),
@@ -161,7 +161,7 @@ def build_s(cells: DeviceCells, stream=None) -> DeviceCSR:
     nlev = np.asarray(cells.n_levels, dtype=np.int64)
     sh = _lib.stream_handle(stream)
     ws = torch.empty(int(lib.hdfe_sbuild_workspace_bytes(L, M, D)), dtype=torch.uint8, device=dev)
-    info = torch.zeros(8, dtype=torch.int64, device=dev)
+    info = torch.empty(8, dtype=torch.int64, device=dev)
     lc = None if cells.lcount is None else cells.lcount.data_ptr()
     wk = None if cells.work is None else cells.work.data_ptr()
     args = (cells.starts.data_ptr(), G, cells.codes.data_ptr(), D, cells.n.data_ptr(),
@@ -207,7 +207,7 @@ def build_s_split(cells: DeviceCells, first: int, count: int, stream=None):
     nlev = np.asarray(cells.n_levels, dtype=np.int64)
     sh = _lib.stream_handle(stream)
     ws = torch.empty(int(lib.hdfe_sbuild_workspace_bytes(L, M, D)), dtype=torch.uint8, device=dev)
-    info = torch.zeros(8, dtype=torch.int64, device=dev)
+    info = torch.empty(8, dtype=torch.int64, device=dev)
     lc = None if cells.lcount is None else cells.lcount.data_ptr()
     wk = None if cells.work is None else cells.work.data_ptr()
     args = (cells.starts.data_ptr(), G, cells.codes.data_ptr(), D, cells.n.data_ptr(),
@@ -261,6 +261,24 @@ def jacobi(diag):
                        torch.zeros_like(diag))
 
 
+def solve_setup(cells: DeviceCells, stream=None):
+    """The Jacobi weights (`jacobi`) and the zero flags of the right-hand sides
+    (norm <= 1e-11 sqrt(total sum of squares), core/solve.py:294-320), both on
+    the device: `(dinv (L,), zero (m,) uint8)`."""
+    torch = _torch()
+    lib = _lib.lib()
+    diag, rhs, raw_ss = cells.diag.contiguous(), cells.rhs.contiguous(), cells.raw_ss.contiguous()
+    L, m = rhs.shape
+    dev = rhs.device
+    dinv = torch.empty(L, dtype=torch.float64, device=dev)
+    zero = torch.empty(m, dtype=torch.uint8, device=dev)
+    ws = torch.empty(int(lib.hdfe_solve_setup_workspace_bytes(m)), dtype=torch.uint8, device=dev)
+    _lib.check(lib.hdfe_solve_setup(
+        diag.data_ptr(), rhs.data_ptr(), L, m, raw_ss.data_ptr(), RHS_ZERO_TOL,
+        dinv.data_ptr(), zero.data_ptr(), ws.data_ptr(), ws.numel(), _lib.stream_handle(stream)))
+    return dinv, zero
+
+
 def components(cells: DeviceCells, col: int = 0, stream=None):
     """Component root of each level of dimension `col` (its smallest level),
     and the number of components (core/kernels_base.py:156-174)."""
@@ -269,7 +287,7 @@ def components(cells: DeviceCells, col: int = 0, stream=None):
     dev = cells.starts.device
     nl = int(cells.n_levels[col])
     root = torch.empty(nl, dtype=torch.int32, device=dev)
-    out = torch.zeros(2, dtype=torch.int64, device=dev)
+    out = torch.empty(2, dtype=torch.int64, device=dev)
     ws = torch.empty(int(lib.hdfe_components_workspace_bytes()), dtype=torch.uint8, device=dev)
     G = int(cells.starts.shape[0]) - 1
     _lib.check(lib.hdfe_components(cells.starts.data_ptr(), G, cells.codes.data_ptr(),
@@ -367,10 +385,12 @@ def solve(cells: DeviceCells, S: DeviceCSR, tol=1e-10, maxiter=5000, rhs_block=8
     torch = _torch()
     timer = timer or _NoTimer()
     m = int(cells.rhs.shape[1])
-    dinv = jacobi(cells.diag)
+    dinv, zero = solve_setup(cells)
     if solver == "stream_cg":
         from .gpu import StreamSolver
         solver = StreamSolver(cells, dinv, tol, maxiter)
+        zero = zero.cpu().numpy().astype(bool)      # its iteration is the host's
+        run = solver.solve_device
     elif solver == "explicit":
         small = small_levels(cells.n_levels) if small_block and precision == "fp64" else None
         if split is not None or S is None:
@@ -380,30 +400,34 @@ def solve(cells: DeviceCells, S: DeviceCSR, tol=1e-10, maxiter=5000, rhs_block=8
         solver = BlockSolver(S, dinv, tol, maxiter, precision=precision, small=small,
                              split=split if precision == "fp64" else None)
         solver.timer = timer
+        run = solver.solve_flagged
     else:
         raise ValueError("solver must be 'explicit' or 'stream_cg'")
-    scale = torch.sqrt(torch.clamp(cells.raw_ss, min=0.0))
-    zero_all = (torch.linalg.vector_norm(cells.rhs, dim=0) <= RHS_ZERO_TOL * scale).cpu().numpy()
     if comps is None:
         root, ncomp = components(cells, 0)
     else:
         root, ncomp, done = comps
         torch.cuda.current_stream(root.device).wait_event(done)
-    gamma = torch.empty_like(cells.rhs)
+    # one block's solution is Gamma itself
+    gamma = None if 0 < m <= rhs_block else torch.empty_like(cells.rhs)
     its, conv, rel = [], True, 0.0
     for j0 in range(0, m, rhs_block):
         j1 = min(m, j0 + rhs_block)
-        X, it, c, r = solver.solve_device(cells.rhs[:, j0:j1], zero_all[j0:j1],
-                                          None if x0 is None else x0[:, j0:j1])
-        gamma[:, j0:j1] = X
+        X, it, c, r = run(cells.rhs[:, j0:j1], zero[j0:j1],
+                          None if x0 is None else x0[:, j0:j1])
+        if gamma is None:
+            gamma = X
+        else:
+            gamma[:, j0:j1] = X
         its.append(it)
         conv &= c
         rel = max(rel, r)
-    if normalize_fe:
-        normalize(gamma, cells, root)
-    n_comp = ncomp.cpu().numpy()
+    n_comp = ncomp.cpu().numpy()        # (the solver has waited already)
     if int(n_comp[1]) != _lib.HDFE_OK:
         raise _lib.HDFEError(int(n_comp[1]), "components: union-find failed")
+    zero_all = zero if isinstance(zero, np.ndarray) else zero.cpu().numpy().astype(bool)
+    if normalize_fe:
+        normalize(gamma, cells, root)
     explicit = not hasattr(solver, "matvec")
     sp = getattr(solver, "split", None)
     if explicit and S is not None:

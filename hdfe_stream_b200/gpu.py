@@ -191,8 +191,11 @@ class BlockSolver:
         zp = None
         if zero is not None:
             import torch
-            self._zero[:k].copy_(torch.from_numpy(np.asarray(zero, bool).astype(np.uint8)))
-            zp = self._zero.data_ptr()
+            if torch.is_tensor(zero):
+                zp = zero.data_ptr()            # device flags (`solve_flagged`)
+            else:
+                self._zero[:k].copy_(torch.from_numpy(np.asarray(zero, bool).astype(np.uint8)))
+                zp = self._zero.data_ptr()
         x0p = None if X0 is None else X0.data_ptr()
         if self.split is not None and k <= _lib.PCG_SMALL_MAX_K:
             sp = self.split
@@ -233,17 +236,21 @@ class BlockSolver:
         return int(info.iterations), bool(info.converged), float(info.max_rel)
 
     def solve_device(self, B, zero=None, X0=None):
+        return self.solve_flagged(B, None if zero is None else np.asarray(zero, bool), X0)
+
+    def solve_flagged(self, B, zero, X0=None):
+        """`solve_device` with the zero flags as a host bool array, as a
+        contiguous uint8 tensor on the device, or None."""
         import torch
         B = B.to(self.dev, torch.float64).contiguous()
         L, k = B.shape
         X = torch.empty_like(B)
         its, conv, rel = 0, True, 0.0
-        zero = None if zero is None else np.asarray(zero, bool)
         width = _lib.PCG_MIXED_MAX_K if self.precision == "mixed" else _lib.PCG_MAX_K
         for j0 in range(0, k, width):
             j1 = min(k, j0 + width)
             Bj = B[:, j0:j1].contiguous()
-            Xj = torch.empty_like(Bj)
+            Xj = torch.empty_like(Bj) if k > width else X
             X0j = None if X0 is None else X0[:, j0:j1].to(self.dev, torch.float64).contiguous()
             zj = None if zero is None else zero[j0:j1]
             timer = getattr(self, "timer", None)
@@ -253,7 +260,8 @@ class BlockSolver:
             else:
                 self.launch(Bj, zj, X0j, Xj)
             it, c, r = self.read_info()
-            X[:, j0:j1] = Xj
+            if k > width:
+                X[:, j0:j1] = Xj
             its, conv, rel = max(its, it), conv and c, max(rel, r)
         if self.debug is not None:
             self.debug(f"  CG iter {its}: max rel. residual {rel:.2e}")

@@ -207,6 +207,14 @@ int hdfe_levels_nested(const int64_t *clusters, int64_t n_rows, const uint32_t *
                        int32_t stride, int64_t n_levels, int64_t *first, int32_t *loose,
                        void *stream);
 
+/* Step 2 before its solve (core/solve.py:142-146 `_jacobi`, :294-320): dinv (L) =
+ * 1 / diag, 0 where diag <= 1e-12; zero[j] (m bytes, device) = 1 when
+ * ||rhs_j|| <= tol sqrt(max(raw_ss_j, 0)), for rhs (L, m) row-major. */
+int64_t hdfe_solve_setup_workspace_bytes(int32_t m);
+int hdfe_solve_setup(const double *diag, const double *rhs, int64_t L, int32_t m,
+                     const double *raw_ss, double tol, double *dinv, uint8_t *zero,
+                     void *workspace, int64_t workspace_bytes, void *stream);
+
 int64_t hdfe_normalize_workspace_bytes(int64_t n_first, int32_t m);
 int hdfe_normalize(double *gamma, int32_t m, int32_t D, const int64_t *n_levels,
                    const double *obs, const int32_t *root, void *workspace,
