@@ -13,7 +13,7 @@
 //                             level under its threshold removed at once; the
 //                             host repeats until a round removes nothing
 //                             (`_nb_peel`'s rounds, same core)
-//   unions                    alive pairs joined, larger root under smaller
+//   k_join                    alive pairs joined, larger root under smaller
 //   labels                    roots numbered in vertex order (a scan of root
 //                             flags), -1 for removed levels; rows per label
 //
@@ -22,11 +22,13 @@
 // points of what is alive.  The reference finds them by Tarjan's depth-first
 // search (core/kernels_graph.py:23-86), which is sequential; here they come
 // from a breadth-first spanning tree and the Tarjan-Vishkin rules, which are
-// data-parallel:
+// data-parallel (k_cut_round, one cooperative launch a round; k_largest keeps
+// the largest component before and after it):
 //   BFS tree                  level-synchronous, from the smallest alive
-//                             vertex; depth and tree parent per vertex
+//                             vertex; depth and tree parent per vertex, the
+//                             vertices queued by depth
 //   subtree sizes, preorder   bottom-up sums per level, then each vertex's
-//                             children numbered in turn, top-down
+//                             number from its parent's, top-down
 //   low / high                min / max preorder number over every neighbour
 //                             of the subtree (bottom-up per level)
 //   tree-edge classes         union-find over tree edges (named by their
@@ -45,14 +47,13 @@
 #include <climits>
 #include <cuda_runtime.h>
 
-#include "common.cuh"
+#include "unionfind.cuh"
 
 namespace hdfe {
 namespace pairs {
 
 constexpr int kThreads = 256;
 constexpr int kTile = 4096;
-constexpr int kMaxSteps = 1 << 22;
 
 inline unsigned grid_for(int64_t n, int64_t cap = 148 * 32)
 {
@@ -172,61 +173,163 @@ __global__ void __launch_bounds__(kThreads) k_mark(int64_t n0, int64_t n, int64_
     }
 }
 
-__device__ __forceinline__ int32_t find_root(int32_t *parent, int32_t x)
-{
-    int32_t p = parent[x];
-    int steps = 0;
-    while (p != x && steps < kMaxSteps) {
-        const int32_t gp = parent[p];
-        if (gp != p) parent[x] = gp;
-        x = p;
-        p = gp;
-        steps++;
+// ---- cooperative kernels (k_join, k_largest, k_cut_round)
+//
+// One CTA of 1024 threads an SM; the phases of an algorithm are separated by
+// grid barriers (2.5-3 us) instead of launches and host reads (a launch over
+// every vertex per BFS level and phase, with a read per level: 60% of the
+// leave-one-out set's 3.7 ms on 8.5M rows).
+constexpr int kCoop = 1024;
+
+struct Graph {
+    const uint32_t *pa, *pb;    // the pairs, *P of them
+    const int64_t *count, *P;
+    int64_t n0, n;              // first-dimension vertices, all vertices
+    uint8_t *alive;
+    unsigned *status;
+    GridBarrier bar;
+
+    __device__ bool sync() const
+    {
+        if (bar.sync()) return true;
+        if (threadIdx.x == 0) atomicCAS(status, 0u, (unsigned)HDFE_ERR_SPIN_LIMIT);
+        return false;
     }
-    return x;
+};
+
+// The components of the vertices lo .. n over the edges that edges(join) gives:
+// rounds of hooking every edge's larger parent under the smaller and
+// flattening, which leave nearly every edge inside one tree, then unions of
+// what is left (unions alone contend for the giant component's root).  parent
+// must be the identity, visible to all; every root is its component's smallest
+// vertex, and the caller flattens after a further barrier.
+template <int ROUNDS, typename F>
+__device__ __forceinline__ bool join_edges(const Graph &g, int64_t lo, int32_t *parent, F edges)
+{
+    const int64_t t0 = (int64_t)blockIdx.x * kCoop + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * kCoop;
+    for (int r = 0; r < ROUNDS; r++) {
+        edges([&](int32_t x, int32_t y) {
+            const int32_t px = parent[x], py = parent[y];
+            if (px != py) hook(parent, px, py);
+        });
+        if (!g.sync()) return false;
+        for (int64_t v = lo + t0; v < g.n; v += step) parent[v] = root_of(parent, (int32_t)v);
+        if (!g.sync()) return false;
+    }
+    edges([&](int32_t x, int32_t y) {
+        if (parent[x] != parent[y]) unite(parent, x, y, g.status);
+    });
+    return true;
 }
 
-// The root of x without writing: for the flattening passes, where each thread
-// writes only its own vertex's entry (a compressing find could overwrite a
-// vertex another thread has just set to its root with a non-root ancestor).
-__device__ __forceinline__ int32_t root_of(const int32_t *parent, int32_t x)
+// f(x, y) for every pair whose levels are both alive
+template <typename F>
+__device__ __forceinline__ void alive_pairs(const Graph &g, int64_t np, F f)
 {
-    int steps = 0;
-    for (int32_t p = parent[x]; p != x && steps < kMaxSteps; p = parent[x], steps++) x = p;
-    return x;
+    const int64_t t0 = (int64_t)blockIdx.x * kCoop + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * kCoop;
+#pragma unroll 4
+    for (int64_t p = t0; p < np; p += step) {
+        const int32_t x = (int32_t)g.pa[p], y = (int32_t)(g.n0 + g.pb[p]);
+        if (g.alive[x] && g.alive[y]) f(x, y);
+    }
 }
 
-__global__ void __launch_bounds__(kThreads) k_init(int32_t *parent, int64_t n)
+// The components of the alive pairs: parent[v] = the component's smallest
+// second-dimension vertex, v itself for a vertex without alive pairs.  Each
+// first-dimension level picks one of its alive neighbours as its anchor (any:
+// a plain store) and its pairs join the anchor with the others, so that the
+// trees are over the second dimension alone: 100,000 firms instead of 1.1M
+// vertices, whose unions took 220 us of 310 (1.75M pairs) because a worker is
+// always the smaller end and the rounds' hooks found few of them.
+__device__ __forceinline__ bool components(const Graph &g, int32_t *parent)
 {
-    for (int64_t i = (int64_t)blockIdx.x * kThreads + threadIdx.x; i < n;
-         i += (int64_t)gridDim.x * kThreads)
-        parent[i] = (int32_t)i;
+    const int64_t t0 = (int64_t)blockIdx.x * kCoop + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * kCoop;
+    const int64_t np = *g.P;
+    for (int64_t v = t0; v < g.n; v += step) parent[v] = (int32_t)v;
+    if (!g.sync()) return false;
+    alive_pairs(g, np, [&](int32_t x, int32_t y) { parent[x] = y; });
+    if (!g.sync()) return false;
+    const bool ok = join_edges<3>(g, g.n0, parent, [&](auto join) {
+        alive_pairs(g, np, [&](int32_t x, int32_t y) {
+            const int32_t z = parent[x];
+            if (z != y) join(z, y);
+        });
+    });
+    if (!ok || !g.sync()) return false;
+    for (int64_t v = t0; v < g.n; v += step) {
+        const int32_t r = parent[v];
+        parent[v] = v < g.n0 ? (r == (int32_t)v ? r : root_of(parent, r))
+                             : root_of(parent, (int32_t)v);
+    }
+    return g.sync();
 }
 
-// alive pairs joined: the larger root under the smaller (bounded retries)
-__global__ void __launch_bounds__(kThreads) k_union(const uint32_t *pa, const uint32_t *pb,
-                                                    const int64_t *P, int64_t n0,
-                                                    const uint8_t *alive, int32_t *parent,
-                                                    unsigned *status)
+// least[r] = the smallest vertex of the component with root r (INT_MAX where no
+// first-dimension level has that root; those come first in vertex order), by a
+// warp's lanes of one root together: all warps meet at the giant's
+__device__ __forceinline__ void smallest(const Graph &g, const int32_t *parent, int32_t *least)
 {
-    const int64_t np = *P;
-    for (int64_t p = (int64_t)blockIdx.x * kThreads + threadIdx.x; p < np;
-         p += (int64_t)gridDim.x * kThreads) {
-        int32_t x = (int32_t)pa[p], y = (int32_t)(n0 + pb[p]);
-        if (!alive[x] || !alive[y]) continue;
-        for (int step = 0;; step++) {
-            if (step >= kMaxSteps) { atomicCAS(status, 0u, (unsigned)HDFE_ERR_SPIN_LIMIT); break; }
-            x = find_root(parent, x);
-            y = find_root(parent, y);
-            if (x == y) break;
-            const int32_t hi = x > y ? x : y, lo = x > y ? y : x;
-            const int32_t old = atomicCAS(parent + hi, hi, lo);
-            if (old == hi) break;
-            x = hi;
-            y = lo;
+    const int64_t t0 = (int64_t)blockIdx.x * kCoop + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * kCoop;
+    const int lane = threadIdx.x & 31;
+    for (int64_t base = t0 - lane; base < g.n0; base += step) {
+        const int64_t x = base + lane;
+        const int32_t r = x < g.n0 ? parent[x] : -1;
+        const unsigned peers = __match_any_sync(0xffffffffu, r);
+        if (r >= g.n0 && lane == __ffs(peers) - 1 && (int32_t)x < least[r])
+            atomicMin(least + r, (int32_t)x);
+    }
+}
+
+// the alive pairs' components with their smallest vertices as roots
+__global__ void __launch_bounds__(kCoop, 1) k_join(Graph g, int32_t *parent, int32_t *least)
+{
+    const int64_t t0 = (int64_t)blockIdx.x * kCoop + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * kCoop;
+    for (int64_t v = t0; v < g.n; v += step) least[v] = INT_MAX;
+    if (!components(g, parent)) return;
+    smallest(g, parent, least);
+    if (!g.sync()) return;
+    for (int64_t v = t0; v < g.n; v += step) {
+        const int32_t r = parent[v];
+        if (r >= g.n0 && least[r] != INT_MAX) parent[v] = least[r];
+    }
+}
+
+// Rows per root: a thread carries the count of its current root along its
+// pairs; at the end the lanes of a warp that hold the same one add theirs
+// together (nearly every pair is in the giant component, and an atomic a pair
+// on its address took 1.14 ms for 1.75M pairs).
+struct Carry {
+    unsigned long long *rows;
+    int32_t at = -1;
+    unsigned long long sum = 0;
+
+    __device__ void add(int32_t label, int64_t count)
+    {
+        if (label != at) {
+            if (sum) atomicAdd(rows + at, sum);
+            at = label;
+            sum = 0;
         }
+        sum += (unsigned long long)count;
     }
-}
+
+    __device__ void flush()         // by whole warps
+    {
+        const unsigned peers = __match_any_sync(0xffffffffu, at);
+        const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
+        unsigned long long total = 0;
+        for (int q = 0; q < 32; q++) {
+            const unsigned long long v = __shfl_sync(0xffffffffu, sum, q);
+            if ((peers >> q) & 1u) total += v;
+        }
+        if (lane == leader && at >= 0 && total) atomicAdd(rows + at, total);
+    }
+};
 
 // roots of every vertex, and the alive roots' flags per tile
 __global__ void __launch_bounds__(kThreads) k_roots(int32_t *parent, const uint8_t *alive,
@@ -292,40 +395,20 @@ __global__ void __launch_bounds__(kThreads) k_resolve(int32_t *labels, int64_t n
     }
 }
 
-// Rows per component: each pair's count where both levels are labeled.  Nearly
-// every pair of a panel is in the giant component, so one atomic a pair
-// serialises on one address (1.14 ms for the 1.75M pairs of a 1M-worker
-// panel).  A thread carries the count of its current label along its
-// grid-stride walk; at the end the lanes of a warp that hold the same label
-// add theirs together: one atomic a warp and label (about 10 us).
+// rows per component: each pair's count where both levels are labeled
 __global__ void __launch_bounds__(kThreads) k_pair_rows(const uint32_t *pa, const uint32_t *pb,
                                                         const int64_t *count, const int64_t *P,
                                                         int64_t n0, const int32_t *labels,
                                                         int64_t *rows)
 {
     const int64_t np = *P;
-    int32_t at = -1;                    // the label of the carried count
-    unsigned long long sum = 0;
+    Carry c{reinterpret_cast<unsigned long long *>(rows)};
     for (int64_t p = (int64_t)blockIdx.x * kThreads + threadIdx.x; p < np;
          p += (int64_t)gridDim.x * kThreads) {
         const int32_t la = labels[pa[p]], lb = labels[n0 + pb[p]];
-        if (la < 0 || lb < 0) continue;
-        if (la != at) {
-            if (sum) atomicAdd(reinterpret_cast<unsigned long long *>(rows) + at, sum);
-            at = la;
-            sum = 0;
-        }
-        sum += (unsigned long long)count[p];
+        if (la >= 0 && lb >= 0) c.add(la, count[p]);
     }
-    const unsigned peers = __match_any_sync(0xffffffffu, at);
-    const int lane = threadIdx.x & 31, leader = __ffs(peers) - 1;
-    unsigned long long total = 0;
-    for (int q = 0; q < 32; q++) {
-        const unsigned long long v = __shfl_sync(0xffffffffu, sum, q);
-        if ((peers >> q) & 1u) total += v;
-    }
-    if (lane == leader && at >= 0 && total)
-        atomicAdd(reinterpret_cast<unsigned long long *>(rows) + at, total);
+    c.flush();
 }
 
 // ------------------------------------------------ leave-one-out connected set
@@ -413,41 +496,71 @@ __global__ void __launch_bounds__(kThreads) k_adj_fill(const uint32_t *pa, const
     }
 }
 
-// the largest component by rows (the first of equals, i.e. the one whose
-// smallest vertex comes first): best = its label, -1 when there is none
-__global__ void __launch_bounds__(kThreads) k_best(const int64_t *crow, const int64_t *ncomp,
-                                                   int64_t *best)
+// Everything but the largest component by rows removed (the first of equals,
+// i.e. the one whose smallest vertex comes first); the number of components
+// into *ncomp.  Scratch: least and crow (n), smallest vertex and rows by root;
+// cbest, two words a CTA.
+__global__ void __launch_bounds__(kCoop, 1) k_largest(Graph g, int32_t *parent, int32_t *least,
+                                                      int64_t *crow, int64_t *cbest,
+                                                      int64_t *ncomp)
 {
-    __shared__ int64_t s_r[kThreads], s_i[kThreads];
-    const int64_t nc = *ncomp;
-    int64_t r = -1, i = -1;
-    for (int64_t c = threadIdx.x; c < nc; c += kThreads)
-        if (crow[c] > r) { r = crow[c]; i = c; }
-    s_r[threadIdx.x] = r;
-    s_i[threadIdx.x] = i;
-    __syncthreads();
-    for (int h = kThreads / 2; h > 0; h >>= 1) {
-        if (threadIdx.x < h) {
-            const int64_t r2 = s_r[threadIdx.x + h], i2 = s_i[threadIdx.x + h];
-            if (r2 > s_r[threadIdx.x] || (r2 == s_r[threadIdx.x] && i2 >= 0 &&
-                                          (s_i[threadIdx.x] < 0 || i2 < s_i[threadIdx.x]))) {
-                s_r[threadIdx.x] = r2;
-                s_i[threadIdx.x] = i2;
-            }
-        }
-        __syncthreads();
+    __shared__ int64_t s_r[kCoop / 32], s_i[kCoop / 32];
+    const int64_t t0 = (int64_t)blockIdx.x * kCoop + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * kCoop;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const int64_t np = *g.P;
+    for (int64_t v = t0; v < g.n; v += step) {
+        crow[v] = 0;
+        least[v] = INT_MAX;
     }
-    if (threadIdx.x == 0) *best = s_i[0];
-}
-
-__global__ void __launch_bounds__(kThreads) k_keep(uint8_t *alive, const int32_t *labels,
-                                                   int64_t n, const int64_t *best)
-{
-    const int64_t b = *best;
-    if (b < 0) return;
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads)
-        if (alive[v] && labels[v] != (int32_t)b) alive[v] = 0;
+    if (t0 == 0) *ncomp = 0;
+    if (!components(g, parent)) return;
+    unsigned long long roots = 0;
+    for (int64_t v = t0; v < g.n; v += step) roots += parent[v] == (int32_t)v && g.alive[v];
+    roots = warp_sum(roots);
+    if (lane == 0 && roots) atomicAdd(reinterpret_cast<unsigned long long *>(ncomp), roots);
+    smallest(g, parent, least);
+    Carry c{reinterpret_cast<unsigned long long *>(crow)};
+    for (int64_t p = t0; p < np; p += step) {
+        const int64_t y = g.n0 + g.pb[p];
+        if (g.alive[g.pa[p]] && g.alive[y]) c.add(parent[y], g.count[p]);
+    }
+    __syncwarp();
+    c.flush();
+    if (!g.sync()) return;
+    // the most rows, ties to the smallest vertex: per lane, warp, CTA, then
+    // every CTA over the CTAs' bests
+    int64_t br = -1, bi = -1;
+    auto take = [&](int64_t r, int64_t i) {
+        if (i >= 0 && (r > br || (r == br && (bi < 0 || i < bi)))) { br = r; bi = i; }
+    };
+    auto warp_take = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            const int64_t r = __shfl_xor_sync(0xffffffffu, br, o);
+            const int64_t i = __shfl_xor_sync(0xffffffffu, bi, o);
+            take(r, i);
+        }
+    };
+    for (int64_t v = t0; v < g.n; v += step)
+        if (g.alive[v] && parent[v] == (int32_t)v)
+            take(crow[v], least[v] != INT_MAX ? least[v] : v);
+    warp_take();
+    if (lane == 0) { s_r[warp] = br; s_i[warp] = bi; }
+    __syncthreads();
+    if (warp == 0) {
+        take(s_r[lane], s_i[lane]);
+        warp_take();
+        if (lane == 0) { cbest[2 * blockIdx.x] = br; cbest[2 * blockIdx.x + 1] = bi; }
+    }
+    if (!g.sync()) return;
+    br = bi = -1;
+    for (unsigned b = lane; b < gridDim.x; b += 32) take(cbest[2 * b], cbest[2 * b + 1]);
+    warp_take();
+    if (bi < 0) return;
+    const int32_t keep = parent[bi];
+    for (int64_t v = t0; v < g.n; v += step)
+        if (g.alive[v] && parent[v] != keep) g.alive[v] = 0;
 }
 
 // rows per first-dimension level over the alive pairs (`_nb_level_rows`)
@@ -486,225 +599,252 @@ __global__ void __launch_bounds__(kThreads) k_single(uint8_t *alive, const int64
         }
 }
 
-// smallest alive vertex (the BFS root); depth and tree parent cleared
-__global__ void __launch_bounds__(kThreads) k_bfs_init(const uint8_t *alive, int64_t n,
-                                                       int32_t *depth, int32_t *tpar,
-                                                       int32_t *cut, int *root)
+struct CutArgs {
+    Graph g;
+    const int64_t *indptr;
+    const int32_t *indices;
+    int32_t *depth, *tpar, *size, *pre, *low, *high, *aux, *cut;
+    int32_t *order;         // (n) reached vertices by depth
+    int32_t *lvl;           // (n + 1) where each depth begins in order
+    // zeroed before the launch: three queue counters, the root's key
+    unsigned *queue;
+    int *root_key;          // n - the smallest alive vertex
+    unsigned long long *removed;
+    int64_t *levels;
+};
+
+// f(u, v) for every neighbour u of the vertices v in list[0 .. count), the
+// edges of up to 32 vertices dealt to the lanes one by one (a hub's neighbours
+// to one thread would be a serial chain); all lanes reach every f together,
+// with u < 0 where a lane has no edge.  Few vertices are dealt to more warps.
+template <typename F>
+__device__ __forceinline__ void walk_edges(const CutArgs &a, const int32_t *list, int64_t count,
+                                           F f)
 {
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads) {
-        depth[v] = -1;
-        tpar[v] = -1;
-        cut[v] = 0;
-        if (alive[v]) atomicMin(root, (int)v);
+    const int lane = threadIdx.x & 31;
+    const int64_t wid = ((int64_t)blockIdx.x * kCoop + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * kCoop) >> 5;
+    int64_t per = (count + nw - 1) / nw;
+    per = per > 32 ? 32 : (per < 1 ? 1 : per);
+    for (int64_t base = wid * per; base < count; base += nw * per) {
+        const bool have = lane < per && base + lane < count;
+        const int32_t v = have ? list[base + lane] : 0;
+        const int64_t beg = have ? a.indptr[v] : 0;
+        const int64_t deg = have ? a.indptr[v + 1] - beg : 0;
+        int64_t inc = deg;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int64_t y = __shfl_up_sync(0xffffffffu, inc, o);
+            if (lane >= o) inc += y;
+        }
+        const int64_t total = __shfl_sync(0xffffffffu, inc, 31);
+        const int64_t shift = beg - (inc - deg);        // edge e of the 32 is at e + shift
+        for (int64_t e0 = 0; e0 < total; e0 += 32) {
+            const int64_t e = e0 + lane;
+            int own = 0;                // the first lane whose edges end after e
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                const int64_t y = __shfl_sync(0xffffffffu, inc, own + o - 1);
+                if (y <= e) own += o;
+            }
+            const int64_t sh = __shfl_sync(0xffffffffu, shift, own);
+            const int32_t w = __shfl_sync(0xffffffffu, v, own);
+            f(e < total ? a.indices[e + sh] : -1, w);
+        }
     }
 }
 
-__global__ void k_reset_root(int *root, int *first_child)
+// One round of the articulation points (the rules above): every alive worker
+// that is a cut vertex of the alive graph, which is connected, is removed.
+// The levels of the breadth-first tree are stretches of `order`, so the passes
+// up and down the tree touch each vertex once.  A vertex's preorder number is
+// its parent's plus what the sizes' pass up the tree returned when it added the
+// vertex's size to its parent's (one plus the siblings added before).
+__global__ void __launch_bounds__(kCoop, 1) k_cut_round(CutArgs a)
 {
-    if (threadIdx.x == 0 && blockIdx.x == 0) {
-        *root = INT_MAX;
-        *first_child = INT_MAX;
+    constexpr int kBuf = 128, kFull = kBuf - 32;
+    __shared__ int32_t s_buf[kCoop / 32][kBuf];
+    const Graph &g = a.g;
+    const int64_t t0 = (int64_t)blockIdx.x * kCoop + threadIdx.x;
+    const int64_t step = (int64_t)gridDim.x * kCoop;
+    const int lane = threadIdx.x & 31;
+    const int64_t np = *g.P;
+    int key = 0;
+    for (int64_t v = t0; v < g.n; v += step) {
+        const bool up = g.alive[v];
+        a.depth[v] = up ? -1 : -2;
+        a.tpar[v] = -1;
+        a.size[v] = 1;
+        a.aux[v] = (int32_t)v;
+        a.cut[v] = 0;
+        if (up && key == 0) key = (int)(g.n - v);
     }
-}
-
-__global__ void k_bfs_root(const int *root, int64_t n, int32_t *depth, int32_t *pre)
-{
-    const int r = *root;
-    if (threadIdx.x == 0 && blockIdx.x == 0 && r >= 0 && r < n) {
-        depth[r] = 0;
-        pre[r] = 0;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) key = max(key, __shfl_xor_sync(0xffffffffu, key, o));
+    if (lane == 0 && key) atomicMax(a.root_key, key);
+    if (!g.sync()) return;
+    key = *(volatile int *)a.root_key;
+    if (key == 0) return;                       // nothing is alive
+    const int32_t root = (int32_t)(g.n - key);
+    if (t0 == 0) {
+        a.order[0] = root;
+        a.depth[root] = 0;
+        a.pre[root] = 0;
     }
-}
-
-// one BFS level: the vertices at depth `level` claim their unreached neighbours
-__global__ void __launch_bounds__(kThreads) k_bfs_level(int level, int64_t n,
-                                                        const int64_t *indptr,
-                                                        const int32_t *indices,
-                                                        const uint8_t *alive, int32_t *depth,
-                                                        int32_t *tpar, unsigned *changed)
-{
-    bool any = false;
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads) {
-        if (depth[v] != level) continue;
-        for (int64_t k = indptr[v]; k < indptr[v + 1]; k++) {
-            const int32_t u = indices[k];
-            if (!alive[u] || depth[u] != -1) continue;
-            if (atomicCAS(depth + u, -1, level + 1) == -1) {
-                tpar[u] = (int32_t)v;
-                any = true;
+    __syncwarp();                               // the root's warp is thread 0's
+    // the tree, level by level; claimed vertices leave a warp's buffer 96 or
+    // more at a time
+    int32_t *buf = s_buf[threadIdx.x >> 5];
+    int64_t start = 0, count = 1;
+    int level = 0;
+    for (;; level++) {
+        unsigned *tail = a.queue + (level + 1) % 3;
+        int32_t *next = a.order + start + count;
+        if (t0 == 0) {
+            a.lvl[level] = (int32_t)start;
+            a.queue[(level + 2) % 3] = 0;       // last read before the previous barrier
+        }
+        int held = 0;
+        auto flush = [&]() {
+            unsigned at = 0;
+            if (lane == 0) at = atomicAdd(tail, (unsigned)held);
+            at = __shfl_sync(0xffffffffu, at, 0);
+            __syncwarp();
+            for (int i = lane; i < held; i += 32) next[at + i] = buf[i];
+            __syncwarp();
+            held = 0;
+        };
+        walk_edges(a, a.order + start, count, [&](int32_t u, int32_t v) {
+            const bool mine = u >= 0 && a.depth[u] == -1 &&
+                              atomicCAS(a.depth + u, -1, level + 1) == -1;
+            const unsigned m = __ballot_sync(0xffffffffu, mine);
+            if (mine) {
+                a.tpar[u] = v;
+                buf[held + __popc(m & ((1u << lane) - 1))] = u;
+            }
+            held += __popc(m);
+            if (held >= kFull) flush();
+        });
+        if (held) flush();
+        if (!g.sync()) return;
+        start += count;
+        count = *(volatile unsigned *)tail;
+        if (count == 0) break;
+    }
+    if (t0 == 0) a.lvl[level + 1] = (int32_t)start;
+    if (!g.sync()) return;
+    // subtree sizes up, preorder numbers down
+    for (int l = level; l >= 1; l--) {
+        const int64_t e = a.lvl[l + 1];
+        for (int64_t i = a.lvl[l] + t0; i < e; i += step) {
+            const int32_t v = a.order[i];
+            a.pre[v] = atomicAdd(a.size + a.tpar[v], a.size[v]);
+        }
+        if (!g.sync()) return;
+    }
+    for (int l = 1; l <= level; l++) {
+        const int64_t e = a.lvl[l + 1];
+        for (int64_t i = a.lvl[l] + t0; i < e; i += step) {
+            const int32_t v = a.order[i];
+            a.pre[v] += a.pre[a.tpar[v]];
+        }
+        if (!g.sync()) return;
+    }
+    // least and greatest number over each vertex and its neighbours: a thread a
+    // vertex, a warp for one of 32 neighbours or more
+    for (int64_t base = t0 - lane; base < g.n; base += step) {
+        const int64_t v = base + lane;
+        const bool have = v < g.n && a.depth[v] >= 0;
+        const int64_t beg = have ? a.indptr[v] : 0, end = have ? a.indptr[v + 1] : 0;
+        int32_t lo = have ? a.pre[v] : 0, hi = lo;
+        if (end - beg < 32) {
+#pragma unroll 4
+            for (int64_t k = beg; k < end; k++) {
+                const int32_t w = a.indices[k];
+                if (a.depth[w] < 0) continue;
+                const int32_t p = a.pre[w];
+                lo = min(lo, p);
+                hi = max(hi, p);
             }
         }
-    }
-    if (__any_sync(0xffffffffu, any) && (threadIdx.x & 31) == 0) *changed = 1;
-}
-
-__global__ void __launch_bounds__(kThreads) k_size_init(const int32_t *depth, int64_t n,
-                                                        int32_t *size)
-{
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads)
-        size[v] = depth[v] >= 0 ? 1 : 0;
-}
-
-__global__ void __launch_bounds__(kThreads) k_push_size(int level, const int32_t *depth,
-                                                        const int32_t *tpar, int64_t n,
-                                                        int32_t *size)
-{
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads)
-        if (depth[v] == level) atomicAdd(size + tpar[v], size[v]);
-}
-
-// each vertex at depth `level` numbers its children in preorder
-__global__ void __launch_bounds__(kThreads) k_assign_pre(int level, int64_t n,
-                                                         const int64_t *indptr,
-                                                         const int32_t *indices,
-                                                         const int32_t *depth,
-                                                         const int32_t *tpar,
-                                                         const int32_t *size, int32_t *pre)
-{
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads) {
-        if (depth[v] != level) continue;
-        int32_t next = pre[v] + 1;
-        for (int64_t k = indptr[v]; k < indptr[v + 1]; k++) {
-            const int32_t c = indices[k];
-            if (tpar[c] == (int32_t)v && depth[c] == level + 1) {
-                pre[c] = next;
-                next += size[c];
+        for (unsigned big = __ballot_sync(0xffffffffu, end - beg >= 32); big; big &= big - 1) {
+            const int q = __ffs(big) - 1;
+            const int64_t b = __shfl_sync(0xffffffffu, beg, q), e = __shfl_sync(0xffffffffu, end, q);
+            int32_t l = INT_MAX, h = -1;
+#pragma unroll 4
+            for (int64_t k = b + lane; k < e; k += 32) {
+                const int32_t w = a.indices[k];
+                if (a.depth[w] < 0) continue;
+                const int32_t p = a.pre[w];
+                l = min(l, p);
+                h = max(h, p);
+            }
+#pragma unroll
+            for (int o = 16; o > 0; o >>= 1) {
+                l = min(l, __shfl_xor_sync(0xffffffffu, l, o));
+                h = max(h, __shfl_xor_sync(0xffffffffu, h, o));
+            }
+            if (lane == q) {
+                lo = min(lo, l);
+                hi = max(hi, h);
             }
         }
-    }
-}
-
-// low / high of each reached vertex over itself and its reached neighbours
-__global__ void __launch_bounds__(kThreads) k_local(int64_t n, const int64_t *indptr,
-                                                    const int32_t *indices,
-                                                    const int32_t *depth, const int32_t *pre,
-                                                    int32_t *low, int32_t *high)
-{
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads) {
-        if (depth[v] < 0) continue;
-        int32_t lo = pre[v], hi = pre[v];
-        for (int64_t k = indptr[v]; k < indptr[v + 1]; k++) {
-            const int32_t w = indices[k];
-            if (depth[w] < 0) continue;
-            lo = min(lo, pre[w]);
-            hi = max(hi, pre[w]);
-        }
-        low[v] = lo;
-        high[v] = hi;
-    }
-}
-
-__global__ void __launch_bounds__(kThreads) k_push_low(int level, const int32_t *depth,
-                                                       const int32_t *tpar, int64_t n,
-                                                       int32_t *low, int32_t *high)
-{
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads)
-        if (depth[v] == level) {
-            atomicMin(low + tpar[v], low[v]);
-            atomicMax(high + tpar[v], high[v]);
-        }
-}
-
-__device__ __forceinline__ void unite(int32_t *parent, int32_t x, int32_t y, unsigned *status)
-{
-    for (int step = 0;; step++) {
-        if (step >= kMaxSteps) { atomicCAS(status, 0u, (unsigned)HDFE_ERR_SPIN_LIMIT); return; }
-        x = find_root(parent, x);
-        y = find_root(parent, y);
-        if (x == y) return;
-        const int32_t hi = x > y ? x : y, lo = x > y ? y : x;
-        if (atomicCAS(parent + hi, hi, lo) == hi) return;
-        x = hi;
-        y = lo;
-    }
-}
-
-// tree-edge classes, rule 1: a non-tree edge joins its two ends' tree edges
-// (each edge taken once, from its smaller end)
-__global__ void __launch_bounds__(kThreads) k_tv_cross(int64_t n, const int64_t *indptr,
-                                                       const int32_t *indices,
-                                                       const int32_t *depth,
-                                                       const int32_t *tpar, int32_t *aux,
-                                                       unsigned *status)
-{
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads) {
-        if (depth[v] < 0) continue;
-        for (int64_t k = indptr[v]; k < indptr[v + 1]; k++) {
-            const int32_t w = indices[k];
-            if (w < (int32_t)v || depth[w] < 0 || tpar[v] == w || tpar[w] == (int32_t)v)
-                continue;
-            unite(aux, (int32_t)v, w, status);
+        if (have) {
+            a.low[v] = lo;
+            a.high[v] = hi;
         }
     }
-}
-
-// rule 2: (u, v) joins (parent(u), u) when v's subtree reaches outside u's
-__global__ void __launch_bounds__(kThreads) k_tv_tree(int64_t n, const int32_t *depth,
-                                                      const int32_t *tpar, const int32_t *pre,
-                                                      const int32_t *size, const int32_t *low,
-                                                      const int32_t *high, int32_t *aux,
-                                                      unsigned *status)
-{
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads) {
-        if (depth[v] < 2) continue;                   // u = tpar[v] is not the root
-        const int32_t u = tpar[v];
-        if (low[v] < pre[u] || high[v] >= pre[u] + size[u]) unite(aux, u, (int32_t)v, status);
-    }
-}
-
-// cut vertices: u (not the root) when a child's edge is not in u's class; the
-// root's first child (smallest vertex) found for the second step
-__global__ void __launch_bounds__(kThreads) k_tv_cut(int64_t n, const int32_t *depth,
-                                                     const int32_t *tpar, int32_t *aux,
-                                                     int32_t *cut, int *first_child)
-{
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads) {
-        if (depth[v] < 1) continue;
-        const int32_t u = tpar[v];
-        if (depth[v] == 1) atomicMin(first_child, (int)v);
-        else if (find_root(aux, (int32_t)v) != find_root(aux, u)) cut[u] = 1;
-    }
-}
-
-// the root: cut when two of its children's edges are in different classes
-__global__ void __launch_bounds__(kThreads) k_tv_root(int64_t n, const int32_t *depth,
-                                                      const int *root, const int *first_child,
-                                                      int32_t *aux, int32_t *cut)
-{
-    const int c0 = *first_child;
-    if (c0 == INT_MAX) return;
-    const int32_t r0 = find_root(aux, c0);
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n;
-         v += (int64_t)gridDim.x * kThreads)
-        if (depth[v] == 1 && find_root(aux, (int32_t)v) != r0) cut[*root] = 1;
-}
-
-// workers that are cut vertices removed; their number added to *removed
-__global__ void __launch_bounds__(kThreads) k_remove_cut(uint8_t *alive, const int32_t *cut,
-                                                         int64_t n0, int64_t *removed)
-{
-    for (int64_t v = (int64_t)blockIdx.x * kThreads + threadIdx.x; v < n0;
-         v += (int64_t)gridDim.x * kThreads)
-        if (alive[v] && cut[v]) {
-            alive[v] = 0;
-            atomicAdd(reinterpret_cast<unsigned long long *>(removed), 1ull);
+    if (!g.sync()) return;
+    for (int l = level; l >= 3; l--) {          // the rules read them from depth 2 on
+        const int64_t e = a.lvl[l + 1];
+        for (int64_t i = a.lvl[l] + t0; i < e; i += step) {
+            const int32_t v = a.order[i], u = a.tpar[v];
+            const int32_t lo = a.low[v], hi = a.high[v];
+            if (lo < a.low[u]) atomicMin(a.low + u, lo);
+            if (hi > a.high[u]) atomicMax(a.high + u, hi);
         }
+        if (!g.sync()) return;
+    }
+    // tree-edge classes: rule 1 over the non-tree pairs, rule 2 over the tree
+    // edges (u, v) with u not the root
+    const bool ok = join_edges<2>(g, 0, a.aux, [&](auto join) {
+#pragma unroll 4
+        for (int64_t p = t0; p < np; p += step) {
+            const int32_t x = (int32_t)g.pa[p], y = (int32_t)(g.n0 + g.pb[p]);
+            if (a.depth[x] >= 0 && a.depth[y] >= 0 && a.tpar[x] != y && a.tpar[y] != x)
+                join(x, y);
+        }
+        for (int64_t v = t0; v < g.n; v += step) {
+            if (a.depth[v] < 2) continue;
+            const int32_t u = a.tpar[v], pu = a.pre[u];
+            if (a.low[v] < pu || a.high[v] >= pu + a.size[u]) join(u, (int32_t)v);
+        }
+    });
+    if (!ok || !g.sync()) return;
+    for (int64_t v = t0; v < g.n; v += step) a.aux[v] = root_of(a.aux, (int32_t)v);
+    if (!g.sync()) return;
+    // cut vertices: u with a child's edge outside u's own edge's class, the root
+    // with children's edges in two classes
+    const int32_t first = level > 0 ? a.aux[a.order[1]] : 0;
+    unsigned long long gone = 0;
+    for (int64_t v = t0; v < g.n; v += step) {
+        if (a.depth[v] < 1) continue;
+        const int32_t u = a.tpar[v];
+        if (a.aux[v] != (u == root ? first : a.aux[u]) && u < g.n0 &&
+            atomicExch(a.cut + u, 1) == 0) {
+            g.alive[u] = 0;
+            gone++;
+        }
+    }
+    gone = warp_sum(gone);
+    if (lane == 0 && gone) atomicAdd(a.removed, gone);
+    if (t0 == 0) *a.levels = level;
 }
 
 struct Layout {
     int64_t tiles, first, pa, pb, count, deg, parent, scalars, total;
     // leave-one-out only
-    int64_t indptr, indices, depth, tpar, size, pre, low, high, aux, cut, lab, crow, lrows;
+    int64_t indptr, indices, depth, tpar, size, pre, low, high, aux, cut, order, crow, cbest, lrows;
 };
 
 inline Layout layout(int64_t N, int64_t n, bool loo = false)
@@ -732,8 +872,9 @@ inline Layout layout(int64_t N, int64_t n, bool loo = false)
         o.high = take(n * 4);
         o.aux = take(n * 4);
         o.cut = take(n * 4);
-        o.lab = take(n * 4);
-        o.crow = take(n * 8);
+        o.order = take(n * 4);
+        o.crow = take((n + 1) * 8);
+        o.cbest = take(1024 * 16);
         o.lrows = take(n * 8);
     }
     o.total = p;
@@ -756,11 +897,13 @@ struct Ctx {
     int64_t *tiles, *first, *count, *deg;
     uint32_t *pa, *pb;
     int32_t *parent;
-    // scalars (8 bytes each): P, ncomp, status, changed, best, root, first child, removed,
-    // rows kept, components before, single observations
-    int64_t *P, *ncomp, *best, *removed, *kept, *before, *single;
-    unsigned *status, *changed;
-    int *root, *first_child;
+    pairs::Graph g;
+    // scalars (8 bytes each): P, ncomp, status, changed, rows kept, components before,
+    // single observations; from 8 a round's own (queue counters and root key, workers
+    // removed, the tree's depth); at 16 the grid barrier
+    int64_t *P, *ncomp, *removed, *levels, *kept, *before, *single;
+    unsigned *status, *changed, *queue;
+    int *root_key;
     int launches = 0;
 
     Ctx(const uint32_t *a_, const uint32_t *b_, int64_t N_, int64_t n0_, int64_t n1_, bool loo,
@@ -781,13 +924,21 @@ struct Ctx {
         ncomp = sc + 1;
         status = (unsigned *)(sc + 2);
         changed = (unsigned *)(sc + 3);
-        best = sc + 4;
-        root = (int *)(sc + 5);
-        first_child = (int *)(sc + 6);
-        removed = sc + 7;
-        kept = sc + 8;
-        before = sc + 9;
-        single = sc + 10;
+        kept = sc + 4;
+        before = sc + 5;
+        single = sc + 6;
+        queue = (unsigned *)(sc + 8);
+        root_key = (int *)(queue + 3);
+        removed = sc + 10;
+        levels = sc + 11;
+        g.pa = pa;
+        g.pb = pb;
+        g.count = count;
+        g.P = P;
+        g.n0 = n0;
+        g.n = n;
+        g.status = status;
+        g.bar = GridBarrier{(unsigned *)(sc + 16)};
     }
 
     // the distinct pairs and the (k0, k1)-core; returns the peel rounds
@@ -820,22 +971,41 @@ struct Ctx {
         return HDFE_OK;
     }
 
+    // a cooperative launch of one CTA an SM, fewer where the graph is small
+    int coop(const void *kernel, void **args)
+    {
+        using namespace pairs;
+        int dev = 0, sms = 0;
+        HDFE_CUDA_TRY(cudaGetDevice(&dev));
+        HDFE_CUDA_TRY(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+        int64_t need = ((N > n ? N : n) + 4 * kCoop - 1) / (4 * kCoop);
+        need = need < 1 ? 1 : (need > sms ? sms : need);
+        HDFE_CUDA_TRY(cudaLaunchCooperativeKernel(kernel, dim3((unsigned)need), dim3(kCoop), args,
+                                                  0, s));
+        launches++;
+        return HDFE_OK;
+    }
+
     // components of the alive pairs numbered by their roots into labels, rows
     // per label into rows (n), their number into *ncomp
-    void components(const uint8_t *alive, int32_t *labels, int64_t *rows)
+    int components(uint8_t *alive, int32_t *labels, int64_t *rows)
     {
         using namespace pairs;
         const int64_t vt = (n + kTile - 1) / kTile;
-        k_init<<<grid_for(n), kThreads, 0, s>>>(parent, n);
-        k_union<<<grid_for(N), kThreads, 0, s>>>(pa, pb, P, n0, alive, parent, status);
+        g.alive = alive;
+        int32_t *least = (int32_t *)deg;        // (the degrees are done with)
+        void *args[] = {&g, &parent, &least};
+        const int st = coop((const void *)k_join, args);
+        if (st != HDFE_OK) return st;
         k_roots<<<(unsigned)vt, kThreads, 0, s>>>(parent, alive, n, tiles);
         k_scan<<<1, 1024, 0, s>>>(tiles, vt, ncomp);
         k_number<<<(unsigned)vt, kThreads, 0, s>>>(parent, alive, n, tiles, labels);
         k_label<<<grid_for(n), kThreads, 0, s>>>(parent, alive, n, labels);
         k_resolve<<<grid_for(n), kThreads, 0, s>>>(labels, n);
-        cudaMemsetAsync(rows, 0, n * 8, s);
+        HDFE_CUDA_TRY(cudaMemsetAsync(rows, 0, n * 8, s));
         k_pair_rows<<<grid_for(N, 148 * 4), kThreads, 0, s>>>(pa, pb, count, P, n0, labels, rows);
-        launches += 8;
+        launches += 6;
+        return HDFE_OK;
     }
 };
 
@@ -862,7 +1032,7 @@ extern "C" int hdfe_pair_components(const uint32_t *a, const uint32_t *b, int64_
     int64_t rounds = 0;
     int st = c.pairs_and_core(alive, k0, k1, &rounds);
     if (st != HDFE_OK) return st;
-    c.components(alive, labels, rows);
+    if ((st = c.components(alive, labels, rows)) != HDFE_OK) return st;
     HDFE_CUDA_TRY(cudaGetLastError());
     hdfe_add_launches(c.launches);
     // counts: pairs, components, status, peel rounds
@@ -903,7 +1073,7 @@ extern "C" int hdfe_leave_one_out(const uint32_t *a, const uint32_t *b, int64_t 
     int32_t *size = (int32_t *)(ws + L.size), *pre = (int32_t *)(ws + L.pre);
     int32_t *low = (int32_t *)(ws + L.low), *high = (int32_t *)(ws + L.high);
     int32_t *aux = (int32_t *)(ws + L.aux), *cut = (int32_t *)(ws + L.cut);
-    int32_t *lab = (int32_t *)(ws + L.lab);
+    int32_t *order = (int32_t *)(ws + L.order);
     int64_t *crow = (int64_t *)(ws + L.crow), *lrows = (int64_t *)(ws + L.lrows);
     int64_t peel_rounds = 0;
     int st = c.pairs_and_core(alive, k0, k1, &peel_rounds);
@@ -921,11 +1091,12 @@ extern "C" int hdfe_leave_one_out(const uint32_t *a, const uint32_t *b, int64_t 
                                                 indices);
     c.launches += 5;
 
-    auto keep_largest = [&]() {
-        c.components(alive, lab, crow);
-        k_best<<<1, kThreads, 0, s>>>(crow, c.ncomp, c.best);
-        k_keep<<<grid_for(n), kThreads, 0, s>>>(alive, lab, n, c.best);
-        c.launches += 2;
+    c.g.alive = alive;
+    int64_t *cbest = (int64_t *)(ws + L.cbest);
+    auto keep_largest = [&]() -> int {
+        int32_t *least = (int32_t *)c.deg;      // (the adjacency's degrees are done with)
+        void *args[] = {&c.g, &c.parent, &least, &crow, &cbest, &c.ncomp};
+        return c.coop((const void *)k_largest, args);
     };
     auto read = [&](const void *dev, size_t bytes, void *host) -> int {
         HDFE_CUDA_TRY(cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, s));
@@ -934,7 +1105,7 @@ extern "C" int hdfe_leave_one_out(const uint32_t *a, const uint32_t *b, int64_t 
     };
 
     // 1. the largest component
-    keep_largest();
+    if ((st = keep_largest()) != HDFE_OK) return st;
     HDFE_CUDA_TRY(cudaMemcpyAsync(c.before, c.ncomp, 8, cudaMemcpyDeviceToDevice, s));
     // 2. workers seen once (their leverage is 1), then the largest piece left
     HDFE_CUDA_TRY(cudaMemsetAsync(lrows, 0, n0 * 8, s));
@@ -942,51 +1113,24 @@ extern "C" int hdfe_leave_one_out(const uint32_t *a, const uint32_t *b, int64_t 
                                                   nullptr);
     k_single<<<grid_for(n0), kThreads, 0, s>>>(alive, lrows, n0, c.single);
     c.launches += 2;
-    keep_largest();
+    if ((st = keep_largest()) != HDFE_OK) return st;
     // 3-4. workers that are articulation points, until there are none
     int64_t cut_total = 0, rounds = 0, max_levels = 0;
+    // (the levels' stretches lie in the rows by root, done with by then)
+    CutArgs ca{c.g,  indptr, indices, depth,   tpar,    size,       pre,       low,
+               high, aux,    cut,     order, (int32_t *)crow, c.queue, c.root_key,
+               reinterpret_cast<unsigned long long *>(c.removed), c.levels};
     for (;;) {
-        k_reset_root<<<1, 32, 0, s>>>(c.root, c.first_child);
-        k_bfs_init<<<grid_for(n), kThreads, 0, s>>>(alive, n, depth, tpar, cut, c.root);
-        k_bfs_root<<<1, 32, 0, s>>>(c.root, n, depth, pre);
-        c.launches += 3;
-        int levels = 0;
-        for (;; levels++) {
-            HDFE_CUDA_TRY(cudaMemsetAsync(c.changed, 0, 4, s));
-            k_bfs_level<<<grid_for(n), kThreads, 0, s>>>(levels, n, indptr, indices, alive,
-                                                         depth, tpar, c.changed);
-            c.launches++;
-            unsigned h = 0;
-            if ((st = read(c.changed, 4, &h)) != HDFE_OK) return st;
-            if (!h || levels > n) break;
-        }
-        // `levels` is now the largest depth
-        if (levels > max_levels) max_levels = levels;
-        k_size_init<<<grid_for(n), kThreads, 0, s>>>(depth, n, size);
-        for (int l = levels; l >= 1; l--)
-            k_push_size<<<grid_for(n), kThreads, 0, s>>>(l, depth, tpar, n, size);
-        for (int l = 0; l < levels; l++)
-            k_assign_pre<<<grid_for(n), kThreads, 0, s>>>(l, n, indptr, indices, depth, tpar,
-                                                          size, pre);
-        k_local<<<grid_for(n), kThreads, 0, s>>>(n, indptr, indices, depth, pre, low, high);
-        for (int l = levels; l >= 1; l--)
-            k_push_low<<<grid_for(n), kThreads, 0, s>>>(l, depth, tpar, n, low, high);
-        k_init<<<grid_for(n), kThreads, 0, s>>>(aux, n);
-        k_tv_cross<<<grid_for(n), kThreads, 0, s>>>(n, indptr, indices, depth, tpar, aux,
-                                                    c.status);
-        k_tv_tree<<<grid_for(n), kThreads, 0, s>>>(n, depth, tpar, pre, size, low, high, aux,
-                                                   c.status);
-        k_tv_cut<<<grid_for(n), kThreads, 0, s>>>(n, depth, tpar, aux, cut, c.first_child);
-        k_tv_root<<<grid_for(n), kThreads, 0, s>>>(n, depth, c.root, c.first_child, aux, cut);
-        HDFE_CUDA_TRY(cudaMemsetAsync(c.removed, 0, 8, s));
-        k_remove_cut<<<grid_for(n0), kThreads, 0, s>>>(alive, cut, n0, c.removed);
-        c.launches += 9 + 3 * levels;
-        int64_t n_cut = 0;
-        if ((st = read(c.removed, 8, &n_cut)) != HDFE_OK) return st;
-        if (!n_cut || rounds > n) break;
-        cut_total += n_cut;
+        HDFE_CUDA_TRY(cudaMemsetAsync(c.queue, 0, 32, s));
+        void *args[] = {&ca};
+        if ((st = c.coop((const void *)k_cut_round, args)) != HDFE_OK) return st;
+        int64_t h[2];                       // workers removed, the tree's depth
+        if ((st = read(c.removed, 16, h)) != HDFE_OK) return st;
+        if (h[1] > max_levels) max_levels = h[1];
+        if (!h[0] || rounds > n) break;
+        cut_total += h[0];
         rounds++;
-        keep_largest();
+        if ((st = keep_largest()) != HDFE_OK) return st;
     }
     // rows kept
     HDFE_CUDA_TRY(cudaMemsetAsync(c.kept, 0, 8, s));
@@ -998,14 +1142,14 @@ extern "C" int hdfe_leave_one_out(const uint32_t *a, const uint32_t *b, int64_t 
     // counts: pairs, components before, single observations, workers cut, rounds, rows
     // kept, status, BFS depth (largest over rounds)
     int64_t h[8];
-    int64_t dev_sc[11];
+    int64_t dev_sc[7];
     if ((st = read(c.P, sizeof(dev_sc), dev_sc)) != HDFE_OK) return st;
     h[0] = dev_sc[0];
-    h[1] = dev_sc[9];
-    h[2] = dev_sc[10];
+    h[1] = dev_sc[5];
+    h[2] = dev_sc[6];
     h[3] = cut_total;
     h[4] = rounds;
-    h[5] = dev_sc[8];
+    h[5] = dev_sc[4];
     h[6] = (int64_t)(unsigned)(dev_sc[2] & 0xffffffff);
     h[7] = max_levels;
     HDFE_CUDA_TRY(cudaMemcpyAsync(counts, h, sizeof(h), cudaMemcpyHostToDevice, s));
