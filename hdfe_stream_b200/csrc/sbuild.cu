@@ -106,6 +106,8 @@ struct Args {
     double *dval;               // (W, L)
     uint8_t *dpres;             // (W, L)
     int32_t *cell_widx;         // (M, D) wide index of each cell's level, or -1
+    uint8_t *wide_far;          // per 32 groups: their wide levels are 32 or more apart;
+                                // null: all of them
     double *wpart;              // (CTAs, W*W) per-CTA wide x wide sums
     uint8_t *wpres;             // (CTAs, W*W)
     double *wcross;             // (W*W) n of cells with two wide levels
@@ -797,7 +799,7 @@ __global__ void __launch_bounds__(kThreads) k_cell_widx(Args a)
     }
 }
 
-// The wide x wide block for W <= 16.  Per group g the block adds
+// The wide x wide block (W <= 16, see below for more).  Per group g the block adds
 //     C_g(a, b) - (u_a / N_g) u_b
 // (the reference's per-cell sum  sum_{i has b} (n_i [i has a] - n_i u_a / N_g)
 // regrouped), with u_a = sum of n over g's cells with wide level a and
@@ -813,6 +815,12 @@ __global__ void __launch_bounds__(kThreads) k_cell_widx(Args a)
 // their wide levels, into its own array by atomic adds (exact for counts;
 // in atomic order for weighted n).  Warps and CTAs are summed in a fixed
 // order, so the rest of the block is deterministic.
+//   SLIDE, for W > 16 (up to 32 years, or a batch of panels with its years once
+// per panel): a warp takes consecutive chunks and holds the tiles of 32 wide
+// levels at a time, adding them to the dense rows by atomics when a chunk's
+// levels leave them; chunks that meet levels further apart are left to
+// k_wide_block_atomic.  All groups by atomics met at the same 100 addresses a
+// panel: 504 us for 24 panels of 10 years, 104 now.
 // D += A B for one 8 x 8 x 4 FP64 tile, the whole warp: A row-major (this lane
 // holds row lane / 4, column lane % 4), B column-major (row lane % 4, column
 // lane / 4), D (row lane / 4, columns 2 (lane % 4) and 2 (lane % 4) + 1)
@@ -827,37 +835,89 @@ constexpr int kWideThreads = 128;
 constexpr int kWideWarps = kWideThreads / 32;
 constexpr int kWideRounds = 4;          // rounds of 32 cells whose loads are in flight together
 
+template <bool SLIDE>
 __global__ void __launch_bounds__(kWideThreads) k_wide_block_warp(Args a)
 {
-    __shared__ double s_u[kWideWarps][32][kWideWarp + 1];
-    __shared__ double s_w[kWideWarps][32][kWideWarp + 1];
+    constexpr int KW = SLIDE ? 32 : kWideWarp;      // levels of the tiles
+    constexpr int NT = KW / 8;
+    __shared__ double s_u[kWideWarps][32][KW + 1];
+    __shared__ double s_inv[kWideWarps][32];
+    __shared__ unsigned s_bits[SLIDE ? kWideWarps : 1][32];     // levels of each group
     __shared__ int64_t s_gs[kWideWarps][33];
     __shared__ double s_stage[kWideWarps][32];
-    __shared__ double s_acc[kWideWarps][kWideWarp * kWideWarp];
-    __shared__ unsigned s_pat[kWideWarps][kWideWarp];
+    __shared__ double s_acc[kWideWarps][SLIDE ? 1 : KW * KW];
+    __shared__ unsigned s_pat[kWideWarps][SLIDE ? 1 : KW];
     const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
-    const int W = (int)a.W;
+    const int W = SLIDE ? KW : (int)a.W;
     const int E = W * W;
-    double (*u)[kWideWarp + 1] = s_u[wl];
-    double (*wv)[kWideWarp + 1] = s_w[wl];
+    int base = -1;              // SLIDE: the tiles' first wide level
+    double (*u)[KW + 1] = s_u[wl];
     int64_t *gs = s_gs[wl];
-    // sum over groups of (u_a / N_g) u_b as 8 x 8 tiles (ta, tb) of the 16 x 16
+    // sum over groups of (u_a / N_g) u_b as 8 x 8 tiles (ta, tb) of the KW x KW
     // block: this lane holds entries (8 ta + lane / 4, 8 tb + 2 (lane % 4) + i)
-    double acc[2][2][2] = {};
+    double acc[NT][NT][2] = {};
     const int r8 = lane >> 2, c4 = lane & 3;
     double dsum = 0.0;          // lane a < W: sum of u_a
     const int wdims = (int)(a.ctr[7] >> 8) & 0xff;     // dimensions with wide levels
     unsigned pat = 0;           // lane a < W: levels sharing a group with a
     const int64_t chunks = (a.G + 31) / 32;
-    const int64_t wstep = (int64_t)gridDim.x * kWideWarps;
-    for (int64_t ch = (int64_t)blockIdx.x * kWideWarps + wl; ch < chunks; ch += wstep) {
+    const int64_t warps = (int64_t)gridDim.x * kWideWarps;
+    const int64_t wid = (int64_t)blockIdx.x * kWideWarps + wl;
+    const int64_t share = SLIDE ? (chunks + warps - 1) / warps : 0;
+    const int64_t ch0 = SLIDE ? wid * share : wid;
+    const int64_t ch1 = SLIDE ? min(ch0 + share, chunks) : chunks;
+    // the tiles' entries added to the dense rows, and begun anew
+    [[maybe_unused]] auto flush = [&]() {
+#pragma unroll
+        for (int ta = 0; ta < NT; ta++)
+#pragma unroll
+            for (int tb = 0; tb < NT; tb++)
+#pragma unroll
+                for (int i = 0; i < 2; i++) {
+                    const int ra = 8 * ta + r8, rb = 8 * tb + 2 * c4 + i;
+                    if ((__shfl_sync(0xffffffffu, pat, ra) >> rb) & 1u) {
+                        const int64_t at = (int64_t)(base + ra) * a.L + a.wide_list[base + rb];
+                        atomicAdd(a.dval + at, -acc[ta][tb][i]);
+                        a.dpres[at] = 1;
+                    }
+                    acc[ta][tb][i] = 0.0;
+                }
+        if ((pat >> lane) & 1u)
+            atomicAdd(a.dval + (int64_t)(base + lane) * a.L + a.wide_list[base + lane], dsum);
+        dsum = 0.0;
+        pat = 0;
+    };
+    for (int64_t ch = ch0; ch < ch1; ch += SLIDE ? 1 : warps) {
         const int64_t g0 = ch * 32;
         const int ng = (int)min((int64_t)32, a.G - g0);
         gs[lane] = a.starts[g0 + min(lane, ng)];
         if (lane == 0) gs[32] = a.starts[g0 + ng];
-        for (int q = lane; q < 32 * (kWideWarp + 1); q += 32) (&u[0][0])[q] = 0.0;
+        for (int q = lane; q < 32 * (KW + 1); q += 32) (&u[0][0])[q] = 0.0;
         __syncwarp();
         const int64_t c0 = gs[0], c1 = gs[ng];
+        if constexpr (SLIDE) {
+            s_bits[wl][lane] = 0;
+            int least = INT_MAX, most = -1;
+#pragma unroll 4
+            for (int64_t q = c0 * a.D + lane; q < c1 * a.D; q += 32) {
+                const int32_t x = a.cell_widx[q];
+                if (x >= 0) least = min(least, x);
+                most = max(most, x);
+            }
+            least = __reduce_min_sync(0xffffffffu, least);
+            most = __reduce_max_sync(0xffffffffu, most);
+            // (a total of zero or no number must not reach other levels' tiles)
+            const double N = lane < ng ? a.group_n[g0 + lane] : 1.0;
+            const bool odd = __any_sync(0xffffffffu, !(N > 0.0 && N < INFINITY));
+            const bool far = most >= 0 && (most - least >= KW || odd);
+            if (lane == 0) a.wide_far[ch] = far;
+            if (most < 0 || far) continue;
+            if (base < 0 || least < base || most >= base + KW) {
+                if (base >= 0) flush();
+                // room on both sides, should the next chunk meet a year more
+                base = max(0, least - (KW - 1 - (most - least)) / 2);
+            }
+        }
         // the chunk's cells, kWideRounds rounds of 32 at a time: every round's
         // loads (n, the codes and their levels' wide indices) issued before the first is used
         for (int64_t b0 = c0; b0 < c1; b0 += 32 * kWideRounds) {
@@ -883,9 +943,14 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_block_warp(Args a)
 #pragma unroll
                 for (int d = 0; d < HDFE_MAX_DIMS; d++)
                     if (d < a.D && ((wdims >> d) & 1)) {
-                        const uint32_t c = a.codes[i * a.D + d];
-                        const int32_t k = (int64_t)c < a.nlev[d] ? a.kind[a.offs[d] + c] : -1;
-                        kr[t][d] = k >= 0 ? k : -1;
+                        if constexpr (SLIDE) {
+                            const int32_t k = a.cell_widx[i * a.D + d];
+                            kr[t][d] = k >= 0 ? k - base : -1;
+                        } else {
+                            const uint32_t c = a.codes[i * a.D + d];
+                            const int32_t k = (int64_t)c < a.nlev[d] ? a.kind[a.offs[d] + c] : -1;
+                            kr[t][d] = k >= 0 ? k : -1;
+                        }
                     }
             }
           }
@@ -910,13 +975,20 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_block_warp(Args a)
                     double sum = 0.0;
                     for (unsigned p = peers; p; p &= p - 1) sum += s_stage[wl][__ffs(p) - 1];
                     u[gq][k] += sum;
+                    if constexpr (SLIDE) atomicOr(&s_bits[wl][gq], 1u << k);
                 }
                 if (k >= 0) {
                     // a cell with several wide levels: C(a, k) and C(k, a) for
                     // each wide level a of its earlier dimensions
                     for (int q = 0; q < nk; q++) {
-                        atomicAdd(a.wcross + (int64_t)ks[q] * W + k, ni);
-                        atomicAdd(a.wcross + (int64_t)k * W + ks[q], ni);
+                        if constexpr (SLIDE) {
+                            const int32_t x = base + ks[q], y = base + k;
+                            atomicAdd(a.dval + (int64_t)x * a.L + a.wide_list[y], ni);
+                            atomicAdd(a.dval + (int64_t)y * a.L + a.wide_list[x], ni);
+                        } else {
+                            atomicAdd(a.wcross + (int64_t)ks[q] * W + k, ni);
+                            atomicAdd(a.wcross + (int64_t)k * W + ks[q], ni);
+                        }
                     }
                     ks[nk++] = k;
                 }
@@ -925,16 +997,15 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_block_warp(Args a)
           }
         }
         __syncwarp();
-        // each group's u / N_g and level mask; rows past the chunk's groups
-        // and columns past W are zeros (the tiles below read them)
+        // each group's 1 / N_g and level mask; rows past the chunk's groups and
+        // columns past W are zeros (the tiles below read them)
         unsigned mask = 0;
-        {
-            const double inv = lane < ng ? 1.0 / a.group_n[g0 + lane] : 0.0;
-            for (int k = 0; k < kWideWarp; k++) {
-                const double x = (lane < ng && k < W) ? u[lane][k] : 0.0;
-                wv[lane][k] = x * inv;
-                if (x > 0.0) mask |= 1u << k;
-            }
+        s_inv[wl][lane] = lane < ng ? 1.0 / a.group_n[g0 + lane] : 0.0;
+        if constexpr (SLIDE) {
+            mask = s_bits[wl][lane];
+        } else {
+            for (int k = 0; k < KW; k++)
+                if (lane < ng && k < W && u[lane][k] > 0.0) mask |= 1u << k;
         }
         __syncwarp();
         for (int q = 0; q < ng; q++) {
@@ -950,39 +1021,45 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_block_warp(Args a)
         for (int ks = 0; ks < 8; ks++) {
             if (ks * 4 >= ng) break;                    // warp-uniform
             const int q = ks * 4 + c4;
-            const double a0 = wv[q][r8], a1 = wv[q][8 + r8];
-            const double b0 = u[q][r8], b1 = u[q][8 + r8];
-            dmma_m8n8k4(acc[0][0], a0, b0);
-            dmma_m8n8k4(acc[0][1], a0, b1);
-            dmma_m8n8k4(acc[1][0], a1, b0);
-            dmma_m8n8k4(acc[1][1], a1, b1);
+            const double inv = s_inv[wl][q];
+            double b[NT];
+#pragma unroll
+            for (int t = 0; t < NT; t++) b[t] = u[q][8 * t + r8];
+#pragma unroll
+            for (int ta = 0; ta < NT; ta++)
+#pragma unroll
+                for (int tb = 0; tb < NT; tb++) dmma_m8n8k4(acc[ta][tb], b[ta] * inv, b[tb]);
         }
         __syncwarp();
     }
-    // the warp's entries, then the CTA's warps summed in order
+    if constexpr (SLIDE) {
+        if (base >= 0) flush();
+    } else {
+        // the warp's entries, then the CTA's warps summed in order
 #pragma unroll
-    for (int ta = 0; ta < 2; ta++)
+        for (int ta = 0; ta < NT; ta++)
 #pragma unroll
-        for (int tb = 0; tb < 2; tb++)
+            for (int tb = 0; tb < NT; tb++)
 #pragma unroll
-            for (int i = 0; i < 2; i++) {
-                const int ra = 8 * ta + r8, rb = 8 * tb + 2 * c4 + i;
-                if (ra < W && rb < W) s_acc[wl][ra * W + rb] = -acc[ta][tb][i];
+                for (int i = 0; i < 2; i++) {
+                    const int ra = 8 * ta + r8, rb = 8 * tb + 2 * c4 + i;
+                    if (ra < W && rb < W) s_acc[wl][ra * W + rb] = -acc[ta][tb][i];
+                }
+        if (lane < W) s_pat[wl][lane] = pat;
+        __syncwarp();
+        if (lane < W) s_acc[wl][lane * W + lane] += dsum;
+        __syncthreads();
+        for (int en = threadIdx.x; en < E; en += kWideThreads) {
+            double sum = 0.0;
+            uint8_t p = 0;
+            const int ra = en / W, rb = en % W;
+            for (int w = 0; w < kWideWarps; w++) {
+                sum += s_acc[w][en];
+                p |= (uint8_t)((s_pat[w][ra] >> rb) & 1u);
             }
-    if (lane < W) s_pat[wl][lane] = pat;
-    __syncwarp();
-    if (lane < W) s_acc[wl][lane * W + lane] += dsum;
-    __syncthreads();
-    for (int en = threadIdx.x; en < E; en += kWideThreads) {
-        double sum = 0.0;
-        uint8_t p = 0;
-        const int ra = en / W, rb = en % W;
-        for (int w = 0; w < kWideWarps; w++) {
-            sum += s_acc[w][en];
-            p |= (uint8_t)((s_pat[w][ra] >> rb) & 1u);
+            a.wpart[(int64_t)blockIdx.x * E + en] = sum;
+            a.wpres[(int64_t)blockIdx.x * E + en] = p;
         }
-        a.wpart[(int64_t)blockIdx.x * E + en] = sum;
-        a.wpres[(int64_t)blockIdx.x * E + en] = p;
     }
 }
 
@@ -1013,11 +1090,13 @@ __global__ void __launch_bounds__(kThreads) k_wide_block_reduce(Args a)
     }
 }
 
-// the wide x wide block for W > 16: atomics into the dense buffer
+// the chunks k_wide_block_warp<true> left: a thread a group, atomics into the
+// dense buffer
 __global__ void __launch_bounds__(kThreads) k_wide_block_atomic(Args a)
 {
     for (int64_t g = (int64_t)blockIdx.x * kThreads + threadIdx.x; g < a.G;
          g += (int64_t)gridDim.x * kThreads) {
+        if (a.wide_far && !a.wide_far[g / 32]) continue;
         const int64_t s = a.starts[g], e = a.starts[g + 1];
         const double Ng = a.group_n[g];
         for (int da = 0; da < a.D; da++) {
@@ -1152,7 +1231,7 @@ inline Layout layout(int64_t L, int64_t M, int D)
 }
 
 struct WideLayout {
-    int64_t dval, dpres, widx, wpart, wpres, wcross, segcnt, total;
+    int64_t dval, dpres, widx, far, wpart, wpres, wcross, segcnt, total;
 };
 
 inline int64_t wide_ctas_for(int sms) { return (int64_t)sms * 4; }
@@ -1166,6 +1245,7 @@ inline WideLayout wide_layout(int64_t W, int64_t L, int64_t M, int D, int64_t ct
     o.dval = take(W * L * 8);
     o.dpres = take(W * L);
     o.widx = take(M * (int64_t)D * 4);
+    o.far = take(M / 32 + 1);       // (for G <= M)
     o.wpart = take(ctas * W * W * 8);
     o.wpres = take(ctas * W * W);
     o.wcross = take(W * W * 8);
@@ -1247,6 +1327,7 @@ int set_wide(Ctx &c, int64_t W, void *wide_ws, int64_t wide_bytes_given)
     a.dval = (double *)(b + wl.dval);
     a.dpres = (uint8_t *)(b + wl.dpres);
     a.cell_widx = (int32_t *)(b + wl.widx);
+    a.wide_far = (uint8_t *)(b + wl.far);
     a.wpart = (double *)(b + wl.wpart);
     a.wpres = (uint8_t *)(b + wl.wpres);
     a.wcross = (double *)(b + wl.wcross);
@@ -1441,7 +1522,7 @@ static int count_impl(const int64_t *starts, int64_t n_groups, const uint32_t *c
         }
         z.add(a.rnnz, (a.L + 1) * 8);
         if ((st = hdfe_zero(z, c.s)) != HDFE_OK) return st;
-        if (n_wide > kWideWarp) {       // the atomic wide block reads each cell's wide index
+        if (n_wide > kWideWarp) {       // the wide block reads each cell's wide index
             k_cell_widx<<<grid_for(a.M * a.D, kThreads, c.sms * 8), kThreads, 0, c.s>>>(a);
             launched++;
         }
@@ -1465,12 +1546,16 @@ static int count_impl(const int64_t *starts, int64_t n_groups, const uint32_t *c
     launched += 4;
     if (n_wide > 0) {
         if (n_wide <= kWideWarp) {
-            k_wide_block_warp<<<(unsigned)a.wide_ctas, kWideThreads, 0, c.s>>>(a);
+            k_wide_block_warp<false><<<(unsigned)a.wide_ctas, kWideThreads, 0, c.s>>>(a);
             k_wide_block_reduce<<<grid_for(n_wide * n_wide * 32, kThreads, 64), kThreads, 0, c.s>>>(a);
             launched += 2;
         } else {
+            if (a.G <= a.M)
+                k_wide_block_warp<true><<<(unsigned)a.wide_ctas, kWideThreads, 0, c.s>>>(a);
+            else                        // empty groups: more flags than the workspace holds
+                a.wide_far = nullptr;
             k_wide_block_atomic<<<(unsigned)(c.sms * 8), kThreads, 0, c.s>>>(a);
-            launched++;
+            launched += 2;
         }
         if (!split) {
             k_wide_count<<<grid_for(n_wide * a.nseg, 1, c.sms * 8), kThreads, 0, c.s>>>(a);
