@@ -155,9 +155,10 @@ __device__ __forceinline__ int64_t warp_of(const Params &a, int64_t e)
 // of short rows take fewer nonzeros than warps inside long rows.
 // The lane kernel's nonzeros are heavy (K-wide gathers), so its rows cost
 // their nonzeros alone.
-#ifndef HDFE_PCG_UNROLL
-#define HDFE_PCG_UNROLL 6               // nonzeros per lane in flight (k = 3, 4)
-#endif
+// Nonzeros of a row per lane in flight: a row longer than LPR times this takes
+// a second round trip.  With 4 lanes a row the launch picks 6 or 8 (kLongerRows);
+// with 8, what the registers of K columns hold.
+__host__ __device__ constexpr int unroll_for(int K) { return K <= 2 ? 4 : (K <= 4 ? 6 : 2); }
 
 #ifndef HDFE_PCG_ROW_COST
 #define HDFE_PCG_ROW_COST 32
@@ -311,11 +312,10 @@ __device__ __forceinline__ void gather(const T *V, int64_t c, T (&g)[K])
 // acc += sum over e = e0, e0 + STEP, ... < re of vals[e] * V[indices[e]]:
 // U nonzeros per lane per round, their index/value loads and then their
 // gathers all issued before the multiply-adds, so U round trips overlap.
-template <int K, int VS, int VW, int STEP, typename T>
+template <int K, int VS, int VW, int STEP, typename T, int U>
 __device__ __forceinline__ void row_products(const Params &a, const T *vals, const T *V,
                                              int64_t e0, int64_t re, T (&acc)[K])
 {
-    constexpr int U = K <= 2 ? 4 : (K <= 4 ? HDFE_PCG_UNROLL : 2);
     for (; e0 < re; e0 += STEP * U) {
         int64_t c[U];
         T d[U];
@@ -416,7 +416,8 @@ __device__ __forceinline__ void finish_row(int64_t row, const T (&acc)[K], int64
 // products, which are summed over the subgroups of each step and added, in
 // step order, to this warp's slots s_colw (kSmall x K, zeroed here).  Only
 // the warp holding a row's first nonzero does this for the row.
-template <int K, int VS, int VW, typename T, int LPR = 8, bool DENSE = false>
+template <int K, int VS, int VW, typename T, int LPR = 8, bool DENSE = false,
+          int U = unroll_for(K)>
 __device__ void spmm_range(const Params &a, const WarpRange &wr, const T *__restrict__ vals, const T *__restrict__ V,
                            T *__restrict__ out, T *carry, double (&dot)[K], bool want_dot,
                            const double *s_ps = nullptr, double *s_colw = nullptr)
@@ -462,7 +463,7 @@ __device__ void spmm_range(const Params &a, const WarpRange &wr, const T *__rest
                 T acc[K];
 #pragma unroll
                 for (int k = 0; k < K; k++) acc[k] = T(0);
-                row_products<K, VS, VW, 32, T>(a, vals, V, rs + lane, re, acc);
+                row_products<K, VS, VW, 32, T, U>(a, vals, V, rs + lane, re, acc);
                 if constexpr (DENSE) {
                     if (dense) {
 #pragma unroll
@@ -511,7 +512,7 @@ __device__ void spmm_range(const Params &a, const WarpRange &wr, const T *__rest
                 T acc[K];
 #pragma unroll
                 for (int k = 0; k < K; k++) acc[k] = T(0);
-                if (mine) row_products<K, VS, VW, LPR, T>(a, vals, V, rs + sl, re, acc);
+                if (mine) row_products<K, VS, VW, LPR, T, U>(a, vals, V, rs + sl, re, acc);
                 if constexpr (DENSE) {
 #pragma unroll
                     for (int q = 0; q < JPL; q++)
@@ -750,7 +751,7 @@ __device__ __forceinline__ void dense_small_rows(const Params &a, const TEAM &te
 
 // SPLIT: S in the split form (a.ns > 0); the kernels for the whole CSR carry
 // none of its code (and none of its registers)
-template <int K, int LPR = 8, bool SPLIT = false, bool CLUSTER = false>
+template <int K, int LPR = 8, bool SPLIT = false, bool CLUSTER = false, int U = unroll_for(K)>
 __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
 {
     constexpr int KP = Stride<K>::P;
@@ -805,11 +806,11 @@ __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
     if (a.X0 != nullptr) {
         if ((SPLIT && a.ns > 0)) {
             load_small<K, K>(a, a.X0, s_small, s_ps, s_sp);
-            spmm_range<K, K, 1, double, LPR, true>(a, wr, a.data, a.X0, a.AP, a.carry, dot, false,
+            spmm_range<K, K, 1, double, LPR, true, U>(a, wr, a.data, a.X0, a.AP, a.carry, dot, false,
                                                    s_ps, s_col + warp * kSmall * K);
             dense_partials<K>(a, team, s_ps, s_sp, s_col, s_cta, kQc, dot, false);
         } else {
-            spmm_range<K, K, 1, double, LPR>(a, wr, a.data, a.X0, a.AP, a.carry, dot, false);
+            spmm_range<K, K, 1, double, LPR, false, U>(a, wr, a.data, a.X0, a.AP, a.carry, dot, false);
         }
         if (!team.sync()) return;
         if ((SPLIT && a.ns > 0)) dense_small_rows<K>(a, team, s_sp, kQc, s_aps);
@@ -888,11 +889,11 @@ __global__ void __launch_bounds__(threads_for(K), 1) pcg_kernel(Params a)
             constexpr int VWP = (KP == 4) ? 4 : ((KP % 2 == 0) ? 2 : 1);
             if ((SPLIT && a.ns > 0)) {
                 load_small<K, KP>(a, a.P, s_small, s_ps, s_sp);
-                spmm_range<K, KP, VWP, double, LPR, true>(a, wr, a.data, a.P, a.AP, a.carry, dot,
+                spmm_range<K, KP, VWP, double, LPR, true, U>(a, wr, a.data, a.P, a.AP, a.carry, dot,
                                                           true, s_ps, s_col + warp * kSmall * K);
                 dense_partials<K>(a, team, s_ps, s_sp, s_col, s_cta, kQc, dot, true);
             } else {
-                spmm_range<K, KP, VWP, double, LPR>(a, wr, a.data, a.P, a.AP, a.carry, dot, true);
+                spmm_range<K, KP, VWP, double, LPR, false, U>(a, wr, a.data, a.P, a.AP, a.carry, dot, true);
             }
             team_partials<K>(team, dot, s_scratch, 0);
             if (!team.sync()) return;
@@ -1154,16 +1155,16 @@ bool clusters_fit()
     return v == 1;
 }
 
-template <int K, int LPR = 8>
+template <int K, int LPR = 8, int U = unroll_for(K)>
 cudaError_t launch(Params p, int blocks, cudaStream_t s)
 {
     void *args[] = {&p};
-    const void *fn = (const void *)pcg_kernel<K, LPR, false>;
+    const void *fn = (const void *)pcg_kernel<K, LPR, false, false, U>;
     if constexpr (K <= HDFE_PCG_SMALL_MAX_K) {
         if (blocks == kClusterCtas)
-            return p.ns > 0 ? launch_cluster(pcg_kernel<K, LPR, true, true>, p, threads_for(K), s)
-                            : launch_cluster(pcg_kernel<K, LPR, false, true>, p, threads_for(K), s);
-        if (p.ns > 0) fn = (const void *)pcg_kernel<K, LPR, true>;
+            return p.ns > 0 ? launch_cluster(pcg_kernel<K, LPR, true, true, U>, p, threads_for(K), s)
+                            : launch_cluster(pcg_kernel<K, LPR, false, true, U>, p, threads_for(K), s);
+        if (p.ns > 0) fn = (const void *)pcg_kernel<K, LPR, true, false, U>;
     }
     return cudaLaunchCooperativeKernel(fn, dim3(blocks), dim3(threads_for(K)), args, 0, s);
 }
@@ -1178,6 +1179,21 @@ cudaError_t launch(Params p, int blocks, cudaStream_t s)
 #endif
 constexpr int64_t kShortRowNnz = HDFE_PCG_SHORT_ROW_NNZ;
 constexpr int kShortLpr = HDFE_PCG_SHORT_LPR;
+// Short rows averaging more than this take 8 nonzeros a lane instead of 6: up
+// to 32 a row in one round trip.  21 a row, 3 columns: 30.5 us an iteration
+// against 34.7 (40,000 levels), 23.2 against 28.2 (10,000), 56.5 against 60.0
+// (150,000); 18.0: 29.8 both; 15.5: 30.9 against 30.2; 16.4 on 500,000 levels:
+// 131 against 128.
+constexpr int64_t kLongerRows = 18;
+
+// launch with the lanes and nonzeros a lane that S's rows ask for
+template <int K>
+cudaError_t launch_rows(const Params &p, int blocks, int64_t rows, cudaStream_t s)
+{
+    if (p.nnz > kShortRowNnz * rows) return launch<K>(p, blocks, s);
+    return p.nnz > kLongerRows * rows ? launch<K, kShortLpr, 8>(p, blocks, s)
+                                      : launch<K, kShortLpr, 6>(p, blocks, s);
+}
 
 // ------------------------------------------------ one column per lane
 //
@@ -2065,12 +2081,11 @@ int solve_registers(const int64_t *indptr, const int32_t *indices, const double 
     pcg::k_partition<<<(unsigned)((p.nwarps + 256) / 256), 256, 0, s>>>(indptr, L, nnz, p.nwarps,
                                                                       pcg::kRowCost, (int64_t *)p.wlo);
     cudaError_t e = cudaErrorInvalidValue;
-    const bool short_rows = nnz <= pcg::kShortRowNnz * L;
     switch (k) {
-    case 1: e = short_rows ? pcg::launch<1, pcg::kShortLpr>(p, blocks, s) : pcg::launch<1>(p, blocks, s); break;
-    case 2: e = short_rows ? pcg::launch<2, pcg::kShortLpr>(p, blocks, s) : pcg::launch<2>(p, blocks, s); break;
-    case 3: e = short_rows ? pcg::launch<3, pcg::kShortLpr>(p, blocks, s) : pcg::launch<3>(p, blocks, s); break;
-    case 4: e = short_rows ? pcg::launch<4, pcg::kShortLpr>(p, blocks, s) : pcg::launch<4>(p, blocks, s); break;
+    case 1: e = pcg::launch_rows<1>(p, blocks, L, s); break;
+    case 2: e = pcg::launch_rows<2>(p, blocks, L, s); break;
+    case 3: e = pcg::launch_rows<3>(p, blocks, L, s); break;
+    case 4: e = pcg::launch_rows<4>(p, blocks, L, s); break;
     case 5: e = pcg::launch<5>(p, blocks, s); break;
     case 6: e = pcg::launch<6>(p, blocks, s); break;
     case 7: e = pcg::launch<7>(p, blocks, s); break;
