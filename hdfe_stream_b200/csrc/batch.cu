@@ -89,6 +89,14 @@ struct Args {
     int64_t nwarps;
 };
 
+// What warp j of a CTA, j < its systems, knows about its system first + j: which
+// warps of the CTA are its, its CTAs bf .. bl, and its place in the slots of CTA
+// bf + lane (looked up once: each total would wait two round trips for it).
+struct Mine {
+    unsigned warps;
+    int bf, bl, place;
+};
+
 // Totals over each warp's system of N per-warp values v (already summed over
 // the warp, the same in every lane), through slots [q0, q0 + N) of cpart;
 // S the slots per entry.  One grid barrier.  Returns false when the kernel
@@ -96,7 +104,7 @@ struct Args {
 template <int N, int S>
 __device__ __forceinline__ bool system_totals(const Args &a, const GridBarrier &gb, double (&v)[N],
                                               int q0, double *s_w, double *s_sys, int first,
-                                              int nsys, int local)
+                                              int nsys, int local, const Mine &my)
 {
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     if (lane == 0) {
@@ -108,23 +116,25 @@ __device__ __forceinline__ bool system_totals(const Args &a, const GridBarrier &
         for (int q = lane; q < N; q += 32) {
             double t = 0.0;
             for (int w = 0; w < kWarps; w++)
-                if (a.wsys[blockIdx.x * kWarps + w] == first + warp) t += s_w[w * N + q];
+                if ((my.warps >> w) & 1u) t += s_w[w * N + q];
             a.cpart[((int64_t)blockIdx.x * kWarps + warp) * S + q0 + q] = t;
         }
     }
     if (!gb.sync()) return false;
     if (warp < nsys) {
-        const int sys = first + warp;
-        const int bf = a.swarp[sys] / kWarps, bl = (a.swarp[sys + 1] - 1) / kWarps;
+        double t[N];
+#pragma unroll
+        for (int q = 0; q < N; q++) t[q] = 0.0;
+        for (int b = my.bf + lane; b <= my.bl; b += 32) {
+            const int j = b < my.bf + 32 ? my.place : first + warp - a.wsys[b * kWarps];
+            const double *slot = a.cpart + ((int64_t)b * kWarps + j) * S + q0;
+#pragma unroll
+            for (int q = 0; q < N; q++) t[q] += slot[q];
+        }
 #pragma unroll
         for (int q = 0; q < N; q++) {
-            double t = 0.0;
-            for (int b = bf + lane; b <= bl; b += 32) {
-                const int j = sys - a.wsys[b * kWarps];
-                t += a.cpart[((int64_t)b * kWarps + j) * S + q0 + q];
-            }
-            t = warp_sum(t);
-            if (lane == 0) s_sys[warp * N + q] = t;
+            t[q] = warp_sum(t[q]);
+            if (lane == 0) s_sys[warp * N + q] = t[q];
         }
     }
     __syncthreads();
@@ -134,9 +144,49 @@ __device__ __forceinline__ bool system_totals(const Args &a, const GridBarrier &
     return true;
 }
 
+// acc += sum over j = j0, j0 + STEP, ... < e of data[j] * P[indices[j]]: U
+// nonzeros a lane in flight (their indices and values, then their gathers, all
+// issued before the multiply-adds; one at a time, a row of 19 nonzeros on 8 lanes
+// was three dependent pairs of round trips).
+template <int K, int PS, int STEP, int U>
+__device__ __forceinline__ void products(const Args &a, const GridBarrier &gb, int64_t j0,
+                                         int64_t e, double (&acc)[K])
+{
+    for (; j0 < e; j0 += STEP * U) {
+        int32_t c[U];
+        double v[U], g[U][K];
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            const int64_t j = j0 + STEP * u;
+            c[u] = -1;
+            v[u] = 0.0;
+            if (j < e) {
+                c[u] = a.indices[j];
+                v[u] = a.data[j];
+                if (c[u] < 0 || c[u] >= a.L) { gb.fail(HDFE_ERR_BAD_CODE); c[u] = -1; }
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++) {
+            if (c[u] >= 0) {
+                gather_p<K, PS>(a.P, c[u], g[u]);
+            } else {
+                v[u] = 0.0;
+#pragma unroll
+                for (int k = 0; k < K; k++) g[u][k] = 0.0;
+            }
+        }
+#pragma unroll
+        for (int u = 0; u < U; u++)
+#pragma unroll
+            for (int k = 0; k < K; k++) acc[k] += v[u] * g[u][k];
+    }
+}
+
 template <int K, int LPR>
 __global__ void __launch_bounds__(kThreads) k_batch_pcg(Args a)
 {
+    constexpr int U = K <= 4 ? 6 : (K <= 6 ? 2 : 1);
     __shared__ double s_w[kWarps * 2 * K], s_sys[kWarps * 2 * K];
     GridBarrier gb{a.bar};
     const int lane = threadIdx.x & 31;
@@ -147,6 +197,18 @@ __global__ void __launch_bounds__(kThreads) k_batch_pcg(Args a)
     const int first = a.wsys[blockIdx.x * kWarps];
     const int nsys = a.wsys[blockIdx.x * kWarps + kWarps - 1] - first + 1;
     const int local = sys - first;
+    Mine my{0u, 0, -1, 0};
+    {
+        const int warp = threadIdx.x >> 5;
+        my.warps = __ballot_sync(0xffffffffu, lane < kWarps && a.wsys[blockIdx.x * kWarps +
+                                                                      (lane < kWarps ? lane : 0)] ==
+                                                                   first + warp);
+        if (warp < nsys) {
+            my.bf = a.swarp[first + warp] / kWarps;
+            my.bl = (a.swarp[first + warp + 1] - 1) / kWarps;
+            if (my.bf + lane <= my.bl) my.place = first + warp - a.wsys[(my.bf + lane) * kWarps];
+        }
+    }
     constexpr int S5 = 5 * K;       // slots: set-up 2K, phase A K, phase B 2K
     constexpr int PS = p_stride(K);
 
@@ -178,7 +240,7 @@ __global__ void __launch_bounds__(kThreads) k_batch_pcg(Args a)
 #pragma unroll
         for (int k = 0; k < K; k++) { v[k] = warp_sum(sb[k]); v[K + k] = warp_sum(sz[k]); }
         if (blockIdx.x == 0 && threadIdx.x == 0) { a.flag[0] = 0; a.flag[1] = 0; }
-        if (!system_totals<2 * K, S5>(a, gb, v, 0, s_w, s_sys, first, nsys, local)) return;
+        if (!system_totals<2 * K, S5>(a, gb, v, 0, s_w, s_sys, first, nsys, local, my)) return;
 #pragma unroll
         for (int k = 0; k < K; k++) { sb[k] = v[k]; sz[k] = v[K + k]; }
     }
@@ -201,33 +263,34 @@ __global__ void __launch_bounds__(kThreads) k_batch_pcg(Args a)
         {
             constexpr int RPW = 32 / LPR;           // rows per warp step
             const int sub = lane / LPR, sl = lane % LPR;
-            for (int64_t base = r0; base < r1; base += RPW) {
-                const int64_t r = base + sub;
-                double acc[K];
+            for (int64_t b0 = r0; b0 < r1; b0 += 32) {
+                // the bounds of 32 rows, a row a lane (none for a long row)
+                const int64_t q = b0 + lane;
+                const bool own = q < r1 && a.row_chunk[q] < 0;
+                const int64_t st = own ? a.indptr[q] : 0;
+                const int64_t en = own ? a.indptr[q + 1] : -1;
+                const int n = (int)min((int64_t)32, r1 - b0);
+                for (int i = 0; i < n; i += RPW) {
+                    const int64_t r = b0 + i + sub;
+                    const int64_t s = __shfl_sync(0xffffffffu, st, i + sub);
+                    const int64_t e = __shfl_sync(0xffffffffu, en, i + sub);
+                    const bool mine = i + sub < n && e >= s;
+                    double acc[K], p[K];
 #pragma unroll
-                for (int k = 0; k < K; k++) acc[k] = 0.0;
-                if (r < r1 && a.row_chunk[r] < 0) {
-                    const int64_t e = a.indptr[r + 1];
-                    for (int64_t j = a.indptr[r] + sl; j < e; j += LPR) {
-                        const int32_t c = a.indices[j];
-                        const double v = a.data[j];
-                        if (c < 0 || c >= a.L) { gb.fail(HDFE_ERR_BAD_CODE); continue; }
-                        double g[K];
-                        gather_p<K, PS>(a.P, c, g);
+                    for (int k = 0; k < K; k++) acc[k] = p[k] = 0.0;
+                    if (mine && sl == 0) gather_p<K, PS>(a.P, r, p);
+                    if (mine) products<K, PS, LPR, U>(a, gb, s + sl, e, acc);
 #pragma unroll
-                        for (int k = 0; k < K; k++) acc[k] += v * g[k];
-                    }
-                }
+                    for (int k = 0; k < K; k++)
 #pragma unroll
-                for (int k = 0; k < K; k++)
+                        for (int o = LPR / 2; o > 0; o >>= 1)
+                            acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
+                    if (mine && sl == 0) {
 #pragma unroll
-                    for (int o = LPR / 2; o > 0; o >>= 1)
-                        acc[k] += __shfl_xor_sync(0xffffffffu, acc[k], o);
-                if (sl == 0 && r < r1 && a.row_chunk[r] < 0) {
-#pragma unroll
-                    for (int k = 0; k < K; k++) {
-                        a.AP[r * K + k] = acc[k];
-                        dot[k] += acc[k] * a.P[r * PS + k];
+                        for (int k = 0; k < K; k++) {
+                            a.AP[r * K + k] = acc[k];
+                            dot[k] += acc[k] * p[k];
+                        }
                     }
                 }
             }
@@ -239,15 +302,7 @@ __global__ void __launch_bounds__(kThreads) k_batch_pcg(Args a)
                 double acc[K];
 #pragma unroll
                 for (int k = 0; k < K; k++) acc[k] = 0.0;
-                for (int64_t j = a.chunk_lo[c] + lane; j < e; j += 32) {
-                    const int32_t col = a.indices[j];
-                    const double v = a.data[j];
-                    if (col < 0 || col >= a.L) { gb.fail(HDFE_ERR_BAD_CODE); continue; }
-                    double g[K];
-                    gather_p<K, PS>(a.P, col, g);
-#pragma unroll
-                    for (int k = 0; k < K; k++) acc[k] += v * g[k];
-                }
+                products<K, PS, 32, U>(a, gb, a.chunk_lo[c] + lane, e, acc);
 #pragma unroll
                 for (int k = 0; k < K; k++) {
                     const double t = warp_sum(acc[k]);
@@ -260,7 +315,7 @@ __global__ void __launch_bounds__(kThreads) k_batch_pcg(Args a)
         }
 #pragma unroll
         for (int k = 0; k < K; k++) dot[k] = warp_sum(dot[k]);
-        if (!system_totals<K, S5>(a, gb, dot, 2 * K, s_w, s_sys, first, nsys, local)) return;
+        if (!system_totals<K, S5>(a, gb, dot, 2 * K, s_w, s_sys, first, nsys, local, my)) return;
         // the parity-(it + 1) flag was read by everyone before that barrier
         if (blockIdx.x == 0 && threadIdx.x == 0) a.flag[(it + 1) & 1] = 0;
         double alpha[K];
@@ -301,7 +356,7 @@ __global__ void __launch_bounds__(kThreads) k_batch_pcg(Args a)
         double v[2 * K];
 #pragma unroll
         for (int k = 0; k < K; k++) { v[k] = warp_sum(sr[k]); v[K + k] = warp_sum(s2[k]); }
-        if (!system_totals<2 * K, S5>(a, gb, v, 3 * K, s_w, s_sys, first, nsys, local)) return;
+        if (!system_totals<2 * K, S5>(a, gb, v, 3 * K, s_w, s_sys, first, nsys, local, my)) return;
         // ---- C: convergence, beta, P = dinv R + beta P
         bool sys_active = false;
         double beta[K];
