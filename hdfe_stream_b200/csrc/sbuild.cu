@@ -587,16 +587,11 @@ __device__ void narrow_row(const Args &a, int64_t r, const RowSmem &sm, int max_
     if (lane == 0) sm.loff[nl] = carry;
     __syncwarp();
     const int32_t items = carry;
-    // The row's own column takes a third to a half of its items: it is summed
-    // over the warp (a fixed tree) and joins the table once, instead of one lane
-    // adding its peers one by one every round (5M-worker panel: 1.43 -> 1.37 ms).
-    double own_sum = 0.0;
     for (int32_t base = 0; base < items; base += 32) {
         const int32_t j = base + lane;
         const bool valid = j < items;
         int64_t i = 0;
         double v = 0.0;
-        bool own = false;
         if (valid) {
             int lo = 0, hi = nl;            // last group with loff <= j
             while (hi - lo > 1) {
@@ -606,22 +601,19 @@ __device__ void narrow_row(const Args &a, int64_t r, const RowSmem &sm, int max_
             i = sm.gs[lo] + (j - sm.loff[lo]);
             const double ni = a.n[i];
             v -= ni * sm.wv[lo];
-            own = a.codes[i * a.D + dr] == lr;
-            if (own) v += ni;
+            if (a.codes[i * a.D + dr] == lr) v += ni;
         }
-        own_sum += warp_sum(own ? v : 0.0);
         for (int d = 0; d < a.D; d++) {
-            const bool take = valid && !(own && d == dr);
-            const int32_t col = take ? (int32_t)(a.offs[d] + a.codes[i * a.D + d]) : -1;
+            const int32_t col = valid ? (int32_t)(a.offs[d] + a.codes[i * a.D + d]) : -1;
             const unsigned peers = __match_any_sync(0xffffffffu, col);
             const int leader = __ffs(peers) - 1;
             sm.stage[lane] = v;
             __syncwarp();
-            if (take && lane == leader && split && col >= a.small_first) {
+            if (valid && lane == leader && split && col >= a.small_first) {
                 double sum = 0.0;
                 for (unsigned p = peers; p; p &= p - 1) sum += sm.stage[__ffs(p) - 1];
                 sm.xs[col - a.small_first] += sum;      // a direct slot, not the hash
-            } else if (take && lane == leader) {
+            } else if (valid && lane == leader) {
                 double sum = 0.0;
                 for (unsigned p = peers; p; p &= p - 1) sum += sm.stage[__ffs(p) - 1];
                 // the leaders' columns are distinct, so a slot found holding col
@@ -638,17 +630,6 @@ __device__ void narrow_row(const Args &a, int64_t r, const RowSmem &sm, int max_
                 }
             }
             __syncwarp();
-        }
-    }
-    if (lane == 0 && items > 0) {       // every listed group holds the row's level
-        uint32_t h = slot_of((int32_t)r, bits);
-        for (int probe = 0; probe < slots; probe++) {
-            if (sm.keys[h] == kEmptyKey) {
-                sm.keys[h] = (int32_t)r;
-                sm.vals[h] = own_sum;
-                break;
-            }
-            h = (h + 1) & (slots - 1);
         }
     }
     __syncwarp();
