@@ -1490,7 +1490,7 @@ __device__ __forceinline__ void column_partials(double (&v)[N], double *scratch,
 // memory by cp.async, 8 bytes a lane, cost 28 instructions a nonzero and left
 // one window of 32 in flight.)  An iteration took 229 us at 32 columns on the
 // 1M-worker KSS panel (3.1M nonzeros), 41 on the 100k-worker one and 114 at 8
-// columns on the 400k-worker panel with years; now 151, 37 and 61.
+// columns on the 400k-worker panel with years; now 147, 35 and 61.
 //   A warp walks its range of nonzeros in chunks of up to 32 of one row.  Cut
 // rows leave their partial sums in the carry slots as everywhere here.
 __host__ __device__ constexpr int pair_unroll(int K, int T)
