@@ -941,40 +941,55 @@ inline int take_small(Args &a)
     return (int)(slots * a.B * 8);
 }
 
-template <typename K>
-int launch_window(K kernel, Args &a, int smem, cudaStream_t s)
+template <int BP, int C>
+int launch_spread(Args &a, cudaStream_t s)
 {
-    if (smem > 48 * 1024)
-        HDFE_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                           smem));
-    const unsigned grid = window_grid(a.G, a.Bp, &a.chunk);
-    kernel<<<grid, kThreads, smem, s>>>(a);
+    constexpr int subs = kThreads / BP, most = C < 0 ? kMaxCov : C;
+    static hdfe_shared_limit limit;
+    const int st = limit.raise((const void *)k_spread_win<BP, C>,
+                               subs * Win<BP>::bytes(most, HDFE_MAX_DIMS, true, false, false));
+    if (st != HDFE_OK) return st;
+    const unsigned grid = window_grid(a.G, BP, &a.chunk);
+    k_spread_win<BP, C><<<grid, kThreads,
+                          subs * Win<BP>::bytes(a.c, a.D, a.w != nullptr, false, false), s>>>(a);
     return HDFE_OK;
 }
 
 template <int BP>
 int launch_spread(Args &a, cudaStream_t s)
 {
-    const int smem = kThreads / BP * Win<BP>::bytes(a.c, a.D, a.w != nullptr, false, false);
     switch (a.c) {
-    case 0: return launch_window(k_spread_win<BP, 0>, a, smem, s);
-    case 1: return launch_window(k_spread_win<BP, 1>, a, smem, s);
-    case 2: return launch_window(k_spread_win<BP, 2>, a, smem, s);
-    case 3: return launch_window(k_spread_win<BP, 3>, a, smem, s);
-    default: return launch_window(k_spread_win<BP, -1>, a, smem, s);
+    case 0: return launch_spread<BP, 0>(a, s);
+    case 1: return launch_spread<BP, 1>(a, s);
+    case 2: return launch_spread<BP, 2>(a, s);
+    case 3: return launch_spread<BP, 3>(a, s);
+    default: return launch_spread<BP, -1>(a, s);
     }
+}
+
+template <int BP, int C, bool COLLECT>
+int launch_project(Args &a, cudaStream_t s)
+{
+    constexpr int subs = kThreads / BP, most = C < 0 ? kMaxCov : C;
+    static hdfe_shared_limit limit;
+    const int st = limit.raise((const void *)k_project_win<BP, C, COLLECT>,
+                               subs * Win<BP>::bytes(most, HDFE_MAX_DIMS, true, true, COLLECT));
+    if (st != HDFE_OK) return st;
+    const unsigned grid = window_grid(a.G, BP, &a.chunk);
+    k_project_win<BP, C, COLLECT>
+        <<<grid, kThreads, subs * Win<BP>::bytes(a.c, a.D, a.w != nullptr, true, COLLECT), s>>>(a);
+    return HDFE_OK;
 }
 
 template <int BP, bool COLLECT>
 int launch_project(Args &a, cudaStream_t s)
 {
-    const int smem = kThreads / BP * Win<BP>::bytes(a.c, a.D, a.w != nullptr, true, COLLECT);
     switch (a.c) {
-    case 0: return launch_window(k_project_win<BP, 0, COLLECT>, a, smem, s);
-    case 1: return launch_window(k_project_win<BP, 1, COLLECT>, a, smem, s);
-    case 2: return launch_window(k_project_win<BP, 2, COLLECT>, a, smem, s);
-    case 3: return launch_window(k_project_win<BP, 3, COLLECT>, a, smem, s);
-    default: return launch_window(k_project_win<BP, -1, COLLECT>, a, smem, s);
+    case 0: return launch_project<BP, 0, COLLECT>(a, s);
+    case 1: return launch_project<BP, 1, COLLECT>(a, s);
+    case 2: return launch_project<BP, 2, COLLECT>(a, s);
+    case 3: return launch_project<BP, 3, COLLECT>(a, s);
+    default: return launch_project<BP, -1, COLLECT>(a, s);
     }
 }
 

@@ -3,6 +3,7 @@
 // reductions whose order is fixed, so sums do not depend on scheduling.
 #pragma once
 
+#include <atomic>
 #include <cstdint>
 #include <cuda_runtime.h>
 
@@ -152,6 +153,10 @@ __device__ __forceinline__ void cta_exclusive_scan(int64_t *v, int64_t n, int64_
 
 }  // namespace hdfe
 
+int hdfe_set_cuda_error(cudaError_t e);
+int hdfe_set_error(int code, const char *msg);
+int hdfe_set_arg_error(const char *msg);
+
 #define HDFE_CUDA_TRY(expr)                                            \
     do {                                                               \
         cudaError_t _e = (expr);                                       \
@@ -173,8 +178,26 @@ struct hdfe_zero_list {
 };
 int hdfe_zero(const hdfe_zero_list &list, cudaStream_t s);
 
-int hdfe_set_cuda_error(cudaError_t e);
-int hdfe_set_error(int code, const char *msg);
-int hdfe_set_arg_error(const char *msg);
+// A kernel's dynamic shared memory limit, raised once per device to the most
+// that any of its launches asks for.  The limit belongs to the kernel, not to
+// the launch: set to each launch's own size, another host thread could lower it
+// between this thread's set and its launch; and compared with 48 KB it would
+// leave out the kernel's static shared memory, which counts against them too.
+// One object per kernel (a static of the template that launches it).
+struct hdfe_shared_limit {
+    std::atomic<bool> done[64];
+    int raise(const void *kernel, size_t most)
+    {
+        int dev = 0;
+        HDFE_CUDA_TRY(cudaGetDevice(&dev));
+        const bool known = dev >= 0 && dev < 64;
+        if (known && done[dev].load()) return HDFE_OK;
+        HDFE_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                           (int)most));
+        if (known) done[dev].store(true);
+        return HDFE_OK;
+    }
+};
+
 // counts kernels launched by the library (hdfe_kernel_launches)
 void hdfe_add_launches(int n);
