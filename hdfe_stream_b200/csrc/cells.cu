@@ -929,7 +929,11 @@ int run(const uint32_t *gcode, const uint32_t *codes, const double *V, int m, co
                                        : m == 1 ? groups_work<D, 1> : m == 2 ? groups_work<D, 2>
                                        : m == 3 ? groups_work<D, 3> : m == 4 ? groups_work<D, 4>
                                        : groups_work<D, 0>;
-    HDFE_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    static hdfe_shared_limit limits[6];     // by the kernel: m = 0 .. 4, more
+    const int st = limits[m < 5 ? m : 5].raise(
+        (const void *)kern, (size_t)kSmemLevelBudget +
+                                (size_t)kWarpsPerCta * 32 * ((kSlotFixed + kMaxVars) | 1) * 8);
+    if (st != HDFE_OK) return st;
     HDFE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kThreads, smem));
     int64_t blocks = (int64_t)sms * (per_sm > 0 ? per_sm : 1);
     if (blocks > gtiles * kMaxParts) blocks = gtiles > 0 ? gtiles * kMaxParts : 1;

@@ -170,9 +170,12 @@ int launch_draws(Args &a, cudaStream_t s)
     constexpr int SUBS = kPassThreads / BP;
     const int smem = (Pass::kTile ? 0 : (int)((a.n_small * a.B * 8 + 15) / 16 * 16)) +
                      SUBS * Win<BP>::bytes(a.c, a.D, W, Pass::kTile);
-    if (smem > 48 * 1024)
-        HDFE_CUDA_TRY(cudaFuncSetAttribute(Pass::kernel(),
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    static hdfe_shared_limit limit;
+    const int st = limit.raise((const void *)Pass::kernel(),
+                               (Pass::kTile ? 0 : kSmallBytes) +
+                                   SUBS * Win<BP>::bytes(C < 0 ? kMaxCov : C, HDFE_MAX_DIMS, true,
+                                                         Pass::kTile));
+    if (st != HDFE_OK) return st;
     const int64_t ctas = 148 * 5;
     a.chunk = window_chunk(a.G, ctas * SUBS);
     int64_t b = (a.G + a.chunk * SUBS - 1) / (a.chunk * SUBS);

@@ -461,8 +461,6 @@ constexpr int project_smem()
 template <int BP>
 constexpr int center_chunk_smem() { return (kPassThreads / BP) * Chunk<BP>::kBytes; }
 
-constexpr int kSmallBytes = 40 * 1024;    // small dimensions' level x draw sums per CTA
-
 // the dynamic shared memory limits of the explicit-vector passes, raised once
 // per device
 bool set_smem_limits()

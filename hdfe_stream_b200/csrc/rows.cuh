@@ -41,6 +41,7 @@ struct Args {
 };
 
 constexpr int kPassThreads = 128;
+constexpr int kSmallBytes = 40 * 1024;    // small dimensions' level x draw sums per CTA
 
 // a sub-warp of BP lanes: lane j holds draw j of the block (on: j < B)
 template <int BP>

@@ -1422,8 +1422,9 @@ static int analyze_impl(const int64_t *starts, int64_t n_groups, const uint32_t 
     if ((st = scan_exclusive(c, a.toff, a.L, a.toff, a.ctr + 5)) != HDFE_OK) return st;
     {
         const size_t smem = list_smem(a.D);
-        HDFE_CUDA_TRY(cudaFuncSetAttribute(k_fill_lists,
-                                           cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        static hdfe_shared_limit limit;
+        if ((st = limit.raise((const void *)k_fill_lists, list_smem(HDFE_MAX_DIMS))) != HDFE_OK)
+            return st;
         int per = 0;
         HDFE_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, k_fill_lists,
                                                                   kListWarps * 32, smem));
