@@ -599,6 +599,13 @@ __global__ void __launch_bounds__(kThreads) k_single(uint8_t *alive, const int64
         }
 }
 
+// Vertices of this many neighbours or more are dealt to the whole grid, one
+// after the other, instead of to one warp: a warp takes some 1.5 us per 32
+// edges, so a vertex of tens of millions would hold the grid at a barrier for
+// longer than the barrier's limit.  A hub costs a barrier a level; below the
+// bound a warp's 32 vertices take 0.1 s at most.
+constexpr int64_t kHub = 1 << 16;
+
 struct CutArgs {
     Graph g;
     const int64_t *indptr;
@@ -606,9 +613,12 @@ struct CutArgs {
     int32_t *depth, *tpar, *size, *pre, *low, *high, *aux, *cut;
     int32_t *order;         // (n) reached vertices by depth
     int32_t *lvl;           // (n + 1) where each depth begins in order
-    // zeroed before the launch: three queue counters, the root's key
+    int32_t *hubs;          // (n + 1) reached vertices of kHub neighbours or more
+    // zeroed before the launch: three queue counters, the root's key, three hub
+    // counters
     unsigned *queue;
     int *root_key;          // n - the smallest alive vertex
+    unsigned *hub_queue;
     unsigned long long *removed;
     int64_t *levels;
 };
@@ -617,9 +627,10 @@ struct CutArgs {
 // edges of up to 32 vertices dealt to the lanes one by one (a hub's neighbours
 // to one thread would be a serial chain); all lanes reach every f together,
 // with u < 0 where a lane has no edge.  Few vertices are dealt to more warps.
+// Hubs are left out: put into hubs, counted by *n_hubs (walk_hubs).
 template <typename F>
 __device__ __forceinline__ void walk_edges(const CutArgs &a, const int32_t *list, int64_t count,
-                                           F f)
+                                           int32_t *hubs, unsigned *n_hubs, F f)
 {
     const int lane = threadIdx.x & 31;
     const int64_t wid = ((int64_t)blockIdx.x * kCoop + threadIdx.x) >> 5;
@@ -630,7 +641,11 @@ __device__ __forceinline__ void walk_edges(const CutArgs &a, const int32_t *list
         const bool have = lane < per && base + lane < count;
         const int32_t v = have ? list[base + lane] : 0;
         const int64_t beg = have ? a.indptr[v] : 0;
-        const int64_t deg = have ? a.indptr[v + 1] - beg : 0;
+        int64_t deg = have ? a.indptr[v + 1] - beg : 0;
+        if (deg >= kHub) {
+            hubs[atomicAdd(n_hubs, 1u)] = v;
+            deg = 0;
+        }
         int64_t inc = deg;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -651,6 +666,24 @@ __device__ __forceinline__ void walk_edges(const CutArgs &a, const int32_t *list
             const int32_t w = __shfl_sync(0xffffffffu, v, own);
             f(e < total ? a.indices[e + sh] : -1, w);
         }
+    }
+}
+
+// f(u, v) for every neighbour u of the hubs v in list[0 .. count), each hub's
+// edges dealt to the grid's warps 32 at a time; the lanes of a warp together, u
+// < 0 where a lane has no edge.
+template <typename F>
+__device__ __forceinline__ void walk_hubs(const CutArgs &a, const int32_t *list, unsigned count,
+                                          F f)
+{
+    const int lane = threadIdx.x & 31;
+    const int64_t wid = ((int64_t)blockIdx.x * kCoop + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * kCoop) >> 5;
+    for (unsigned i = 0; i < count; i++) {
+        const int32_t v = list[i];
+        const int64_t end = a.indptr[v + 1];
+        for (int64_t e = a.indptr[v] + wid * 32; e < end; e += nw * 32)
+            f(e + lane < end ? a.indices[e + lane] : -1, v);
     }
 }
 
@@ -696,13 +729,15 @@ __global__ void __launch_bounds__(kCoop, 1) k_cut_round(CutArgs a)
     // more at a time
     int32_t *buf = s_buf[threadIdx.x >> 5];
     int64_t start = 0, count = 1;
+    unsigned n_hubs = 0;                        // on the levels so far
     int level = 0;
     for (;; level++) {
-        unsigned *tail = a.queue + (level + 1) % 3;
+        unsigned *tail = a.queue + (level + 1) % 3, *more = a.hub_queue + (level + 1) % 3;
         int32_t *next = a.order + start + count;
         if (t0 == 0) {
             a.lvl[level] = (int32_t)start;
             a.queue[(level + 2) % 3] = 0;       // last read before the previous barrier
+            a.hub_queue[(level + 2) % 3] = 0;
         }
         int held = 0;
         auto flush = [&]() {
@@ -714,7 +749,7 @@ __global__ void __launch_bounds__(kCoop, 1) k_cut_round(CutArgs a)
             __syncwarp();
             held = 0;
         };
-        walk_edges(a, a.order + start, count, [&](int32_t u, int32_t v) {
+        auto claim = [&](int32_t u, int32_t v) {
             const bool mine = u >= 0 && a.depth[u] == -1 &&
                               atomicCAS(a.depth + u, -1, level + 1) == -1;
             const unsigned m = __ballot_sync(0xffffffffu, mine);
@@ -724,9 +759,17 @@ __global__ void __launch_bounds__(kCoop, 1) k_cut_round(CutArgs a)
             }
             held += __popc(m);
             if (held >= kFull) flush();
-        });
+        };
+        walk_edges(a, a.order + start, count, a.hubs + n_hubs, more, claim);
         if (held) flush();
         if (!g.sync()) return;
+        const unsigned found = *(volatile unsigned *)more;
+        if (found) {                            // the same in every CTA
+            walk_hubs(a, a.hubs + n_hubs, found, claim);
+            if (held) flush();
+            n_hubs += found;
+            if (!g.sync()) return;
+        }
         start += count;
         count = *(volatile unsigned *)tail;
         if (count == 0) break;
@@ -751,7 +794,7 @@ __global__ void __launch_bounds__(kCoop, 1) k_cut_round(CutArgs a)
         if (!g.sync()) return;
     }
     // least and greatest number over each vertex and its neighbours: a thread a
-    // vertex, a warp for one of 32 neighbours or more
+    // vertex, a warp for one of 32 neighbours or more, the grid for hubs
     for (int64_t base = t0 - lane; base < g.n; base += step) {
         const int64_t v = base + lane;
         const bool have = v < g.n && a.depth[v] >= 0;
@@ -767,7 +810,8 @@ __global__ void __launch_bounds__(kCoop, 1) k_cut_round(CutArgs a)
                 hi = max(hi, p);
             }
         }
-        for (unsigned big = __ballot_sync(0xffffffffu, end - beg >= 32); big; big &= big - 1) {
+        for (unsigned big = __ballot_sync(0xffffffffu, end - beg >= 32 && end - beg < kHub); big;
+             big &= big - 1) {
             const int q = __ffs(big) - 1;
             const int64_t b = __shfl_sync(0xffffffffu, beg, q), e = __shfl_sync(0xffffffffu, end, q);
             int32_t l = INT_MAX, h = -1;
@@ -795,6 +839,17 @@ __global__ void __launch_bounds__(kCoop, 1) k_cut_round(CutArgs a)
         }
     }
     if (!g.sync()) return;
+    if (n_hubs) {
+        walk_hubs(a, a.hubs, n_hubs, [&](int32_t w, int32_t v) {
+            const bool in = w >= 0 && a.depth[w] >= 0;
+            const int32_t p = in ? a.pre[w] : 0;
+            const int32_t l = __reduce_min_sync(0xffffffffu, in ? p : INT_MAX);
+            const int32_t h = __reduce_max_sync(0xffffffffu, in ? p : -1);
+            if (lane == 0 && l < a.low[v]) atomicMin(a.low + v, l);
+            if (lane == 0 && h > a.high[v]) atomicMax(a.high + v, h);
+        });
+        if (!g.sync()) return;
+    }
     for (int l = level; l >= 3; l--) {          // the rules read them from depth 2 on
         const int64_t e = a.lvl[l + 1];
         for (int64_t i = a.lvl[l] + t0; i < e; i += step) {
@@ -900,9 +955,9 @@ struct Ctx {
     pairs::Graph g;
     // scalars (8 bytes each): P, ncomp, status, changed, rows kept, components before,
     // single observations; from 8 a round's own (queue counters and root key, workers
-    // removed, the tree's depth); at 16 the grid barrier
+    // removed, the tree's depth, hub counters); at 16 the grid barrier
     int64_t *P, *ncomp, *removed, *levels, *kept, *before, *single;
-    unsigned *status, *changed, *queue;
+    unsigned *status, *changed, *queue, *hub_queue;
     int *root_key;
     int launches = 0;
 
@@ -931,6 +986,7 @@ struct Ctx {
         root_key = (int *)(queue + 3);
         removed = sc + 10;
         levels = sc + 11;
+        hub_queue = (unsigned *)(sc + 12);
         g.pa = pa;
         g.pb = pb;
         g.count = count;
@@ -1116,12 +1172,14 @@ extern "C" int hdfe_leave_one_out(const uint32_t *a, const uint32_t *b, int64_t 
     if ((st = keep_largest()) != HDFE_OK) return st;
     // 3-4. workers that are articulation points, until there are none
     int64_t cut_total = 0, rounds = 0, max_levels = 0;
-    // (the levels' stretches lie in the rows by root, done with by then)
+    // (the levels' stretches and the hubs, n + 1 each, lie in the rows by root,
+    // done with by then)
     CutArgs ca{c.g,  indptr, indices, depth,   tpar,    size,       pre,       low,
-               high, aux,    cut,     order, (int32_t *)crow, c.queue, c.root_key,
-               reinterpret_cast<unsigned long long *>(c.removed), c.levels};
+               high, aux,    cut,     order, (int32_t *)crow, (int32_t *)crow + n + 1, c.queue,
+               c.root_key, c.hub_queue, reinterpret_cast<unsigned long long *>(c.removed),
+               c.levels};
     for (;;) {
-        HDFE_CUDA_TRY(cudaMemsetAsync(c.queue, 0, 32, s));
+        HDFE_CUDA_TRY(cudaMemsetAsync(c.queue, 0, 48, s));      // through hub_queue
         void *args[] = {&ca};
         if ((st = c.coop((const void *)k_cut_round, args)) != HDFE_OK) return st;
         int64_t h[2];                       // workers removed, the tree's depth
