@@ -186,16 +186,18 @@ class BlockSolver:
 
     def launch(self, B, zero, X0, X, stream=None):
         """Enqueue one solve of at most 8 columns on `stream` (no sync)."""
-        k = B.shape[1]
-        ws = self._workspace(k)
         zp = None
         if zero is not None:
             import torch
-            if torch.is_tensor(zero):
-                zp = zero.data_ptr()            # device flags (`solve_flagged`)
-            else:
-                self._zero[:k].copy_(torch.from_numpy(np.asarray(zero, bool).astype(np.uint8)))
-                zp = self._zero.data_ptr()
+            self._zero[:B.shape[1]].copy_(
+                torch.from_numpy(np.asarray(zero, bool).astype(np.uint8)))
+            zp = self._zero.data_ptr()
+        self._launch(B, zp, X0, X, stream)
+
+    def _launch(self, B, zp, X0, X, stream=None):
+        """`launch` with the flags already on the device: zp, their address."""
+        k = B.shape[1]
+        ws = self._workspace(k)
         x0p = None if X0 is None else X0.data_ptr()
         if self.split is not None and k <= _lib.PCG_SMALL_MAX_K:
             sp = self.split
@@ -244,6 +246,11 @@ class BlockSolver:
         import torch
         B = B.to(self.dev, torch.float64).contiguous()
         L, k = B.shape
+        on_device = torch.is_tensor(zero)
+        if on_device and (zero.device != B.device or zero.dtype != torch.uint8 or
+                          zero.shape != (k,) or not zero.is_contiguous()):
+            raise ValueError("solve_flagged: a flag tensor is one contiguous uint8 per column, on "
+                             "the solver's device")
         X = torch.empty_like(B)
         its, conv, rel = 0, True, 0.0
         width = _lib.PCG_MIXED_MAX_K if self.precision == "mixed" else _lib.PCG_MAX_K
@@ -253,12 +260,16 @@ class BlockSolver:
             Xj = torch.empty_like(Bj) if k > width else X
             X0j = None if X0 is None else X0[:, j0:j1].to(self.dev, torch.float64).contiguous()
             zj = None if zero is None else zero[j0:j1]
+            if on_device:
+                go = lambda: self._launch(Bj, zj.data_ptr(), X0j, Xj)
+            else:
+                go = lambda: self.launch(Bj, zj, X0j, Xj)
             timer = getattr(self, "timer", None)
             if timer is not None:
                 with timer("pcg_kernel"):
-                    self.launch(Bj, zj, X0j, Xj)
+                    go()
             else:
-                self.launch(Bj, zj, X0j, Xj)
+                go()
             it, c, r = self.read_info()
             if k > width:
                 X[:, j0:j1] = Xj
