@@ -210,6 +210,17 @@ def ptr(t) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+def is_plain(t) -> bool:
+    """Whether t is a dense tensor of values and nothing else -- no gradient to
+    record, no forward derivative, no vmap level, no negation to be applied --,
+    so that a kernel may take its address in place of torch operations."""
+    import torch
+    return type(t) is torch.Tensor and t.layout == torch.strided and \
+        not (t.requires_grad and torch.is_grad_enabled()) and \
+        not torch._C._functorch.is_functorch_wrapped_tensor(t) and \
+        torch.autograd.forward_ad.unpack_dual(t).tangent is None and not t.is_neg()
+
+
 def stream_handle(stream=None) -> int:
     import torch
     s = torch.cuda.current_stream() if stream is None else stream

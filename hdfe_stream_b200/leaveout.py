@@ -337,14 +337,34 @@ class InverseOperator:
     def drop_null(self, levels, streamed):
         """inverse.py:445-460 `_drop_null_component` (`hdfe_drop_null`):
         (levels, streamed) less their part in the null space, for any number
-        of columns."""
+        of columns.  What the kernel does not take -- inputs that record
+        gradients or stand for others (vmap, a forward derivative), vectors,
+        columns to be broadcast -- goes through the dense basis, which also
+        refuses what does not fit the operator."""
         torch = _torch()
+        if not self._plain(levels, streamed):
+            return self._drop_null_dense(levels, streamed)
         parts = [self._drop_null(levels[:, j:j + MAX_BLOCK], streamed[:, j:j + MAX_BLOCK])
                  for j in range(0, int(levels.shape[1]), MAX_BLOCK)]
         return torch.cat([p[0] for p in parts], 1), torch.cat([p[1] for p in parts], 1)
 
+    def _plain(self, levels, streamed):
+        """Whether the blocks are (L, B) and (G, B) FP64 values on the
+        operator's device."""
+        torch = _torch()
+        return all(_lib.is_plain(t) and t.dtype == torch.float64 and t.device == self.dev
+                   and t.dim() == 2 and t.shape[0] == n
+                   for t, n in ((levels, self.L), (streamed, self.G))) and \
+            levels.shape[1] == streamed.shape[1] > 0
+
+    def _drop_null_dense(self, levels, streamed):
+        qs, ql = self.null_space()
+        overlap = qs.T @ streamed + ql.T @ levels
+        return (levels - ql @ overlap).contiguous(), (streamed - qs @ overlap).contiguous()
+
     def _drop_null(self, levels, streamed):
-        """`drop_null`, and the sums of squares (B) of what is left."""
+        """`drop_null` of blocks that are `_plain`, and the sums of squares
+        (B) of what is left."""
         torch = _torch()
         lib = _lib.lib()
         comp_g, comp_l, K, inv_size, Q = self._null_blocks()
@@ -382,7 +402,12 @@ class InverseOperator:
             raise ValueError(f"apply_inverse: 1 <= B <= {MAX_BLOCK}")
         f64 = dict(dtype=torch.float64, device=self.dev)
         Z, schur_inv = self.border()
-        levels, streamed, norm2 = self._drop_null(levels.to(**f64), streamed.to(**f64))
+        levels, streamed = levels.to(**f64), streamed.to(**f64)
+        if self._plain(levels, streamed):
+            levels, streamed, norm2 = self._drop_null(levels, streamed)
+        else:
+            levels, streamed = self._drop_null_dense(levels, streamed)
+            norm2 = (levels * levels).sum(dim=0) + (streamed * streamed).sum(dim=0)
         scale = torch.sqrt(norm2)
         acc = torch.zeros((self.L, B), **f64)
         acc_x = torch.zeros((max(self.c, 1), B), **f64)
