@@ -243,7 +243,7 @@ def _rows_by_one_key(coded, sizes, D, V, w, N):
     one sort, the codes out of the sorted keys, one gather.  None for every
     other form of the input (several keys, ties that the variables break, no
     rows, columns of different lengths or devices, inputs that record
-    gradients): those take the general path."""
+    gradients or carry a forward derivative): those take the general path."""
     torch = _torch()
     lib = _lib.lib()
     bits = [_bits(n) for n in sizes]
@@ -251,10 +251,11 @@ def _rows_by_one_key(coded, sizes, D, V, w, N):
     if N == 0 or D == 0 or sum(bits) > 64 or max(bits) > 31 or len(bits) > 8:
         return None
     if any(c.numel() != N or c.device != dev for c, _ in coded) or V.dim() != 2 or \
-            V.shape[0] != N or V.device != dev or V.requires_grad or V.is_complex():
+            V.shape[0] != N or V.device != dev or V.requires_grad or V.is_complex() or \
+            not _lib.is_plain(V):
         return None
     if w is not None and (w.dim() != 1 or w.numel() != N or w.device != dev or w.requires_grad
-                          or w.is_complex()):
+                          or w.is_complex() or not _lib.is_plain(w)):
         return None
     m = int(V.shape[1])
     cols = (ctypes.c_void_p * len(bits))(*[c.data_ptr() for c, _ in coded])
