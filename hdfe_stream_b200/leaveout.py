@@ -292,10 +292,12 @@ class InverseOperator:
             root, out = components(self.cells, 0)
             root = root.to(torch.int64)
             number = torch.cumsum(root == torch.arange(nl0, device=self.dev), 0) - 1
-            comp_l = number[root]
+            comp_l = number[root].to(torch.int32)
             # inverse.py:430-437 `_group_components`: each group's first row
             first = self.rows.codes.view(-1, D)[self.starts[:-1], 0]
             comp_g = comp_l[first.to(torch.int64)]
+            # (everything is complete when the sizes have been read: the blocks
+            # are kept, and a later call may come on another stream)
             K = int(out[0].item())
             size = torch.cat([torch.bincount(comp_g, minlength=K),
                               torch.bincount(comp_l, minlength=K)]).cpu().numpy().astype(float)
@@ -313,8 +315,7 @@ class InverseOperator:
                     q -= Q[:, :d - 1] @ (Q[:, :d - 1].T @ (size * q))
                 Q[:, d - 1] = q / np.sqrt(size @ (q * q))
             up = lambda x: torch.as_tensor(np.ascontiguousarray(x), device=self.dev)
-            self._null = (comp_g.to(torch.int32), comp_l.to(torch.int32), K, up(1.0 / whole),
-                          up(Q))
+            self._null = (comp_g, comp_l, K, up(1.0 / whole), up(Q))
         return self._null
 
     def null_space(self):
