@@ -555,7 +555,10 @@ __global__ void __launch_bounds__(kThreads) k_spread_win(Args a)
         int q0 = 0;
         for (int f = 0; f < ng; f++) {
             const int q1 = next_bit(gheads, q0, n);
-            group(f, q0, q1, heads, streamed_of(a, ln, wn, g, f) * wn.gx[f * (c + 2) + c + 1]);
+            // (nothing of a group without weight: its value may be no number)
+            const double *gx = wn.gx + f * (c + 2);
+            group(f, q0, q1, heads,
+                  gx[c] > 0.0 ? streamed_of(a, ln, wn, g, f) * gx[c + 1] : 0.0);
             q0 = q1;
         }
     };
@@ -684,7 +687,7 @@ __global__ void __launch_bounds__(kThreads) k_project_win(Args a)
                 if (k >= c) break;
                 tot -= gx[k] * Cj[k];
             }
-            const double mean = tot * gx[c + 1];
+            const double mean = gx[c] > 0.0 ? tot * gx[c + 1] : 0.0;
             if (a.groups && ln.on) a.groups[(g + f) * a.B + ln.j] = mean;
             if (a.rows || COLLECT) {
                 const double gs = emit(heads, i0, q0, q1, r, mean);
