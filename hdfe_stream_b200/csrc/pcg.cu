@@ -1901,6 +1901,7 @@ __global__ void __launch_bounds__(T, 1) lane_kernel(Params a, LaneArgs x)
             if (c0 + 1 < kc) a.X[r * kc + c0 + 1] = v.y;
         }
     }
+    __syncthreads();        // the last s_rel and s_active, by the first K / 2 threads
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         double mx = 0.0;
         bool conv = true;
