@@ -498,7 +498,9 @@ extern "C" int hdfe_factorize_range(const void *ids, int32_t id_bytes, int64_t n
     if (!ids || (id_bytes != 4 && id_bytes != 8) || n < 1 || n > INT32_MAX || range < 1 ||
         !codes || !levels || !n_levels || !workspace)
         return hdfe_set_arg_error("hdfe_factorize_range: bad argument");
-    if (workspace_bytes < hdfe_factorize_range_workspace_bytes(range))
+    const int64_t need = hdfe_factorize_range_workspace_bytes(range);
+    if (need < 0) return hdfe_set_arg_error("hdfe_factorize_range: range must be below 2^40");
+    if (workspace_bytes < need)
         return hdfe_set_error(HDFE_ERR_WORKSPACE, "hdfe_factorize_range: workspace too small");
     cudaStream_t s = (cudaStream_t)stream;
     using namespace sorting;

@@ -712,8 +712,8 @@ int hdfe_factorize(const uint64_t *ids, int64_t n, int32_t key_bits, int32_t *co
                    uint64_t *levels, int64_t *n_levels, void *workspace, int64_t workspace_bytes,
                    void *stream);
 
-/* The same for signed ids (id_bytes 4 or 8) within [lo, lo + range): a bitmap
- * of the range instead of a sort; levels (min(n, range)) int64.  An id outside
+/* The same for signed ids (id_bytes 4 or 8) within [lo, lo + range), range below
+ * 2^40: a bitmap of the range instead of a sort; levels (min(n, range)) int64.  An id outside
  * the range gets no code and is recorded in the workspace's first word.
  *
  * hdfe_pack_codes: keys[i] = the columns' codes packed most significant first,
