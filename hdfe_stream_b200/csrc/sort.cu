@@ -435,12 +435,15 @@ extern "C" int hdfe_sort_pairs(const uint64_t *keys, const int32_t *vals, int64_
     if (n == 0) return HDFE_OK;
     cudaStream_t s = (cudaStream_t)stream;
     sorting::Work w = sorting::layout(workspace, n);
-    // outputs over the inputs: one pass (or none) would write what it still reads
-    auto meet = [](const void *a, const void *b, int64_t bytes) {
+    // an output over an input: one pass (or none) would write what it still reads
+    auto meet = [](const void *a, int64_t a_bytes, const void *b, int64_t b_bytes) {
         const char *x = (const char *)a, *y = (const char *)b;
-        return a && x < y + bytes && y < x + bytes;
+        return a && x < y + b_bytes && y < x + a_bytes;
     };
-    if (key_bits <= 8 && (meet(keys, keys_out, n * 8) || meet(vals, vals_out, n * 4))) {
+    auto over = [&](const void *out, int64_t out_bytes) {
+        return meet(keys, n * 8, out, out_bytes) || meet(vals, n * 4, out, out_bytes);
+    };
+    if (key_bits <= 8 && (over(keys_out, n * 8) || over(vals_out, n * 4))) {
         HDFE_CUDA_TRY(cudaMemcpyAsync(w.keys[1], keys, n * 8, cudaMemcpyDeviceToDevice, s));
         keys = w.keys[1];
         if (vals) {
