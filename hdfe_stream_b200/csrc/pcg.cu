@@ -87,6 +87,7 @@ struct Params {
     int64_t L, nnz;
     int64_t Lb;                 // first small level (L when there is no dense block)
     int ns;                     // small levels, 0 .. kSmall
+    int cluster;                // pcg_kernel: one cluster, not a cooperative grid
     const double *cross;        // (Lb, kSmall) S[r, Lb + j]
     const double *small;        // (ns, ns) S[Lb + i, Lb + j]
     const int64_t *wlo;     // (warps + 1) first nonzero of each warp's range
@@ -1161,7 +1162,7 @@ cudaError_t launch(Params p, int blocks, cudaStream_t s)
     void *args[] = {&p};
     const void *fn = (const void *)pcg_kernel<K, LPR, false, false, U>;
     if constexpr (K <= HDFE_PCG_SMALL_MAX_K) {
-        if (blocks == kClusterCtas)
+        if (p.cluster)
             return p.ns > 0 ? launch_cluster(pcg_kernel<K, LPR, true, true, U>, p, threads_for(K), s)
                             : launch_cluster(pcg_kernel<K, LPR, false, true, U>, p, threads_for(K), s);
         if (p.ns > 0) fn = (const void *)pcg_kernel<K, LPR, true, false, U>;
@@ -2059,8 +2060,10 @@ int solve_registers(const int64_t *indptr, const int32_t *indices, const double 
     p.cross = cross;
     p.small = small;
     if (k <= HDFE_PCG_SMALL_MAX_K && blocks > pcg::kClusterCtas && pcg::small_system(p) &&
-        pcg::clusters_fit())
+        pcg::clusters_fit()) {
         blocks = pcg::kClusterCtas;     // one cluster (the workspace is sized for the grid)
+        p.cluster = 1;
+    }
     const int64_t warps = (int64_t)blocks * (pcg::threads_for(k) / 32);
     p.nwarps = warps;
     p.dinv = dinv;
