@@ -267,9 +267,17 @@ def solve_setup(cells: DeviceCells, stream=None):
     the device: `(dinv (L,), zero (m,) uint8)`."""
     torch = _torch()
     lib = _lib.lib()
-    diag, rhs, raw_ss = cells.diag.contiguous(), cells.rhs.contiguous(), cells.raw_ss.contiguous()
+    diag, rhs, raw_ss = cells.diag, cells.rhs, cells.raw_ss
     L, m = rhs.shape
     dev = rhs.device
+    if not all(_lib.is_plain(t) and t.dtype == torch.float64 and t.device == dev and t.is_cuda
+               and tuple(t.shape) == shape
+               for t, shape in ((diag, (L,)), (rhs, (L, m)), (raw_ss, (m,)))):
+        # other types, sizes or devices than pass 1's: torch's rules
+        scale = torch.sqrt(torch.clamp(raw_ss, min=0.0))
+        zero = torch.linalg.vector_norm(rhs, dim=0) <= RHS_ZERO_TOL * scale
+        return jacobi(diag), zero.to(torch.uint8).contiguous()
+    diag, rhs, raw_ss = diag.contiguous(), rhs.contiguous(), raw_ss.contiguous()
     dinv = torch.empty(L, dtype=torch.float64, device=dev)
     zero = torch.empty(m, dtype=torch.uint8, device=dev)
     ws = torch.empty(int(lib.hdfe_solve_setup_workspace_bytes(m)), dtype=torch.uint8, device=dev)
@@ -400,6 +408,7 @@ def solve(cells: DeviceCells, S: DeviceCSR, tol=1e-10, maxiter=5000, rhs_block=8
         solver = BlockSolver(S, dinv, tol, maxiter, precision=precision, small=small,
                              split=split if precision == "fp64" else None)
         solver.timer = timer
+        zero = zero.to(solver.dev)
         run = solver.solve_flagged
     else:
         raise ValueError("solver must be 'explicit' or 'stream_cg'")
