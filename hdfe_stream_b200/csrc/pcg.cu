@@ -1971,9 +1971,7 @@ int solve_lanes(const int64_t *indptr, const int32_t *indices, const double *dat
     const LaneLayout lay = lane_layout(L, k, blocks);
     if (workspace_bytes < lay.total)
         return hdfe_set_error(HDFE_ERR_WORKSPACE, "hdfe_pcg_solve: workspace too small");
-    // rows of two columns a lane are read 16 bytes at a time; the layout's last
-    // piece is 64 bytes of 256, so a workspace on any 8 bytes can be shifted
-    char *ws = (char *)(((uintptr_t)workspace + 15) & ~(uintptr_t)15);
+    char *ws = (char *)workspace;
     Params p{};
     p.indptr = indptr;
     p.indices = indices;
