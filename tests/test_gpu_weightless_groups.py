@@ -65,5 +65,7 @@ def test_wide_as_narrow(size, bad, B):
         for a, b in zip(wide, narrow):
             fine = b.isfinite()
             assert torch.equal(a.isfinite(), fine)
+            if not bool(fine.any()):        # (the covariate block meets every level)
+                continue
             assert float((a[fine] - b[fine]).abs().max()) <= 1e-12 * max(
                 float(b[fine].abs().max()), 1.0)
