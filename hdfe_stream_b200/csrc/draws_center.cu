@@ -58,9 +58,24 @@ __global__ void __launch_bounds__(kPassThreads) k_center_draws(Args a)
             }
         }
     };
+    // a group without weight adds nothing, whatever its covariates: they are
+    // staged as zeros
+    auto drop_weightless = [&](unsigned gheads, int ng, int n) {
+        if constexpr (W && C != 0) {
+            for (int g = ln.j; g < ng; g += BP) {
+                double *gx = wn.gx + g * (c + 1);
+                if (gx[c] > 0.0) continue;
+                const int q0 = nth_bit(gheads, g), q1 = next_bit(gheads, q0, n);
+                for (int k = 0; k < c; k++) gx[k] = 0.0;
+                for (int t = q0 * c; t < q1 * c; t++) wn.x[t] = 0.0;
+            }
+            __syncwarp(ln.mask);
+        }
+    };
     auto window = [&](int64_t, int64_t i0, int n, unsigned gheads, int ng) {
         const unsigned heads = load_window<BP, C, W>(a, ln, wn, i0, n, &sq) | gheads;
         group_sums<BP, C, W>(a, ln, wn, gheads, ng, n);
+        drop_weightless(gheads, ng, n);
         const uint32_t word = window_signs(a, i0, n, dterm);
         cov_rows(word, n);
         int q0 = 0;
@@ -99,6 +114,10 @@ __global__ void __launch_bounds__(kPassThreads) k_center_draws(Args a)
         for (int64_t i0 = s; i0 < e; i0 += kWin) {
             const int n = (int)min((int64_t)kWin, e - i0);
             const unsigned heads = load_window<BP, C, W>(a, ln, wn, i0, n, &sq);
+            if (W && !(sw > 0.0)) {         // as drop_weightless
+                __syncwarp(ln.mask);
+                continue;
+            }
             group_sums<BP, C, W>(a, ln, wn, 1u, 1, n);
             const uint32_t word = window_signs(a, i0, n, dterm);
             cov_rows(word, n);
