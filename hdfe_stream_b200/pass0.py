@@ -210,7 +210,8 @@ def pass0(streamed, fixed_effects, V, w=None, sort_only=()):
     effects.  Returns (rows, levels): levels per column, streamed first."""
     torch = _torch()
     N = streamed.numel()
-    ids = [streamed] + list(fixed_effects) + list(sort_only)
+    fixed_effects = list(fixed_effects)         # (any iterable, read once)
+    ids = [streamed] + fixed_effects + list(sort_only)
     coded = _factorize_all(ids)
     sizes = [len(l) for _, l in coded]
     D = len(fixed_effects)
