@@ -37,6 +37,8 @@
 // instead of the hash (the same additions in the same order) and writes them
 // as its row of `cross`; the wide x wide block goes to `small`; no wide row
 // is written to the CSR, which holds the big block only.
+#include <cfloat>
+
 #include <cuda_runtime.h>
 
 #include "common.cuh"
@@ -887,9 +889,10 @@ __global__ void __launch_bounds__(kWideThreads) k_wide_block_warp(Args a)
             }
             least = __reduce_min_sync(0xffffffffu, least);
             most = __reduce_max_sync(0xffffffffu, most);
-            // (a total of zero or no number must not reach other levels' tiles)
-            const double N = lane < ng ? a.group_n[g0 + lane] : 1.0;
-            const bool odd = __any_sync(0xffffffffu, !(N > 0.0 && N < INFINITY));
+            // (a total whose reciprocal is no positive normal number must not
+            // reach other levels' tiles)
+            const double inv = lane < ng ? 1.0 / a.group_n[g0 + lane] : 1.0;
+            const bool odd = __any_sync(0xffffffffu, !(inv >= DBL_MIN && inv < INFINITY));
             const bool far = most >= 0 && (most - least >= KW || odd);
             if (lane == 0) a.wide_far[ch] = far;
             if (most < 0 || far) continue;
