@@ -3,8 +3,8 @@
     python -m hdfe_stream_b200.build          # or __graft_entry__.build()
 
 Each csrc/*.cu compiles to an object under _build/ (in parallel), linked into
-hdfe_stream_b200/libhdfe_b200.so; a file is recompiled only when it or a
-header is newer than its object.
+hdfe_stream_b200/libhdfe_b200.so; a file is recompiled only when it, a header
+or this file is newer than its object.
 """
 
 from __future__ import annotations
@@ -22,8 +22,10 @@ INCLUDE = PKG.parent / "include"
 OUT = PKG / "libhdfe_b200.so"
 BUILD = PKG / "_build"
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
-FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr",
-         f"-I{INCLUDE}", f"-I{CSRC}"]
+# (-fno-gnu-unique: a template's statics -- the limits raised so far -- belong to
+# this copy of the library, as its kernels do, not to every copy in the process)
+FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC,-fno-gnu-unique",
+         "--expt-relaxed-constexpr", f"-I{INCLUDE}", f"-I{CSRC}"]
 
 
 def nvcc() -> str:
@@ -34,7 +36,7 @@ def nvcc() -> str:
 
 
 def _headers_mtime() -> float:
-    hs = list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h"))
+    hs = list(CSRC.glob("*.cuh")) + list(INCLUDE.glob("*.h")) + [Path(__file__)]
     return max((h.stat().st_mtime for h in hs), default=0.0)
 
 
