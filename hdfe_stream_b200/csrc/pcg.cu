@@ -101,16 +101,16 @@ struct Params {
     double *X, *R, *P, *AP;
     double *carry;      // (total warps, 2, K)
     double *part;       // (quantities, gridDim.x)
-    int64_t *wfirst;    // (total warps) row of each warp's first nonzero
+    int64_t *wfirst;    // (total warps) row of each warp's first nonzero (mixed_lane_kernel)
     uint8_t *cut;       // (L) row spans two or more warps
     unsigned *bar;
     hdfe_pcg_info *info;
 };
 
-// Workspace layout in bytes: R (L*K), P (L*KP), AP (L*K), carry, part,
-// wfirst, cut flags, then the barrier words.
+// Workspace layout in bytes: R (L*K), P (L*KP), AP (L*K), carry, part, the
+// warps' ranges, cut flags, then the barrier words.
 struct Layout {
-    int64_t r, p, ap, carry, part, wfirst, wlo, cut, bar, total;
+    int64_t r, p, ap, carry, part, wlo, cut, bar, total;
 };
 
 inline Layout layout(int64_t L, int k, int64_t blocks)
@@ -127,7 +127,6 @@ inline Layout layout(int64_t L, int k, int64_t blocks)
     // partials: p'Ap, ||R||^2, R'dinv R, ||B||^2 per column, then the dense
     // block's column sums (kSmall x k)
     o.part = take((4 + kSmall) * (int64_t)k * blocks * 8);
-    o.wfirst = take(warps * 8);
     o.wlo = take((warps + 1) * 8);
     o.cut = take(L);
     o.bar = take(64);
@@ -1198,12 +1197,13 @@ cudaError_t launch_rows(const Params &p, int blocks, int64_t rows, cudaStream_t 
 
 // ------------------------------------------------ one column per lane
 //
-// Wide blocks (the JLA's blocks of probe vectors: up to 32 columns) run with
-// one column per lane instead of K accumulators per thread.  The block is
-// padded to K = 8, 16 or 32 columns (padding columns are zero columns); a
-// row of a vector is then one coalesced load of 8K bytes, a thread holds one
-// accumulator, and all columns share one pass over S's indices and values
-// and one set of grid barriers per iteration.
+// Blocks of 5 to 32 columns (the JLA's blocks of probe vectors) run with their
+// columns over the lanes instead of K accumulators per thread.  The block is
+// padded to K = 8, 16 or 32 columns (padding columns are zero columns); a row
+// of a vector is then one coalesced load, and all columns share one pass over
+// S's indices and values and one set of grid barriers per iteration.  The FP64
+// kernel holds two columns a lane and gathers to registers (lane_kernel, below);
+// what follows to there is the mixed-precision kernel's form, one column a lane:
 //   SpMM: a warp streams its range of nonzeros 32 at a time, H = 32 / K
 //   nonzeros side by side (one per group of K lanes), the rows of V it needs
 //   staged in shared memory by asynchronous copies, several windows ahead.  Row
@@ -1219,8 +1219,8 @@ cudaError_t launch_rows(const Params &p, int blocks, int64_t rows, cudaStream_t 
 #ifndef HDFE_PCG_LANE_FROM
 #define HDFE_PCG_LANE_FROM 5            // blocks of at least this many columns
 #endif
-// CTA size per block width: the K = 32 kernel stages 24 KB of gathers per
-// warp, so it runs 8 warps per CTA; narrower ones run 16.
+// The mixed kernel's CTA per block width: at K = 32 it stages up to 24 KB of
+// gathers per warp, so it runs 8 warps per CTA; narrower ones run 16.
 __host__ __device__ constexpr int lane_threads(int K) { return K >= 32 ? 256 : 512; }
 __host__ __device__ constexpr int lane_ru(int K) { return K >= 32 ? 4 : 2; }  // vector elements per trip
 constexpr int kLaneStages = 3;          // windows of 32 nonzeros in flight per warp
@@ -1233,8 +1233,12 @@ constexpr int kLaneStages = 3;          // windows of 32 nonzeros in flight per 
 #ifndef HDFE_PCG_PAIR_WIDE
 #define HDFE_PCG_PAIR_WIDE 1000000
 #endif
+// A row's fixed cost in the warp split, in nonzeros.  us an iteration at 0, 4, 8, 16
+// and 32: with years (40,010 levels, 1.64M nonzeros) 85.1, 82.3, 80.6, 85.4, 97.4 at
+// 32 columns and 61.0, 59.4, 58.4, 56.7, 64.4 at 8; without (100,000 levels, 3.1M)
+// 148 to 150 and 103 to 104.
 #ifndef HDFE_PCG_PAIR_ROW_COST
-#define HDFE_PCG_PAIR_ROW_COST 8        // a row's fixed cost in the warp split, in nonzeros
+#define HDFE_PCG_PAIR_ROW_COST 8
 #endif
 constexpr uint8_t kRowCut = 1, kRowEmpty = 2;   // per-row flags
 // dynamic shared memory: per warp, kLaneStages x 32 gathered rows of K values
@@ -1252,7 +1256,7 @@ inline int pair_threads(int64_t L, int k)
 }
 
 struct LaneLayout {
-    int64_t r, p, ap, x, carry, part, wfirst, wlo, cut, bar, total;
+    int64_t r, p, ap, x, carry, part, wlo, cut, bar, total;
 };
 
 // R, P, AP (L, K); X (L, K) unless the caller's X has K columns already
@@ -1269,7 +1273,6 @@ inline LaneLayout lane_layout(int64_t L, int k, int64_t blocks)
     o.x = k == kw ? -1 : take(L * kw * 8);
     o.carry = take(warps * 2 * kw * 8);
     o.part = take(3 * (int64_t)kw * blocks * 8);
-    o.wfirst = take(warps * 8);
     o.wlo = take((warps + 1) * 8);
     o.cut = take(L);
     o.bar = take(64);
@@ -1992,7 +1995,6 @@ int solve_lanes(const int64_t *indptr, const int32_t *indices, const double *dat
     p.AP = (double *)(ws + lay.ap);
     p.carry = (double *)(ws + lay.carry);
     p.part = (double *)(ws + lay.part);
-    p.wfirst = (int64_t *)(ws + lay.wfirst);
     p.wlo = (int64_t *)(ws + lay.wlo);
     p.cut = (uint8_t *)(ws + lay.cut);
     p.bar = (unsigned *)(ws + lay.bar);
@@ -2076,7 +2078,6 @@ int solve_registers(const int64_t *indptr, const int32_t *indices, const double 
     p.AP = (double *)(ws + lay.ap);
     p.carry = (double *)(ws + lay.carry);
     p.part = (double *)(ws + lay.part);
-    p.wfirst = (int64_t *)(ws + lay.wfirst);
     p.wlo = (int64_t *)(ws + lay.wlo);
     p.cut = (uint8_t *)(ws + lay.cut);
     p.bar = (unsigned *)(ws + lay.bar);
@@ -2217,7 +2218,7 @@ struct Mixed {
 };
 
 struct MixedLayout {
-    int64_t r, p, ap, d, ax, carry, part, wfirst, wlo, cut, bar, total;
+    int64_t r, p, ap, d, ax, carry, part, wlo, cut, bar, total;
 };
 
 inline MixedLayout mixed_layout(int64_t L, int k, int64_t blocks)
@@ -2234,7 +2235,6 @@ inline MixedLayout mixed_layout(int64_t L, int k, int64_t blocks)
     const int64_t warps = blocks * (threads_for(k) / 32);
     o.carry = take(warps * 2 * k * 8);
     o.part = take(4 * (int64_t)k * blocks * 8);
-    o.wfirst = take(warps * 8);
     o.wlo = take((warps + 1) * 8);
     o.cut = take(L);
     o.bar = take(64);
@@ -2499,7 +2499,7 @@ __global__ void __launch_bounds__(threads_for(K), 1) mixed_kernel(Params a, Mixe
 // ------------------------------------------- mixed precision, wide blocks
 //
 // The refined solve for blocks of 5 to 32 columns (the JLA's probe blocks),
-// one column per lane as in lane_kernel: the FP64 residual B - S X uses S's
+// one column per lane (see above): the FP64 residual B - S X uses S's
 // FP64 values and the FP64 iterate; the inner PCG runs on S's FP32 values and
 // FP32 vectors R, P, AP, D with FP32 products and updates (p'Ap, the norms and
 // r'z accumulated in FP64); X += D in FP64.  Per inner iteration the bytes are
@@ -2955,7 +2955,6 @@ extern "C" int hdfe_pcg_solve_mixed(const int64_t *indptr, const int32_t *indice
     p.X = X;
     p.carry = (double *)(ws + lay.carry);
     p.part = (double *)(ws + lay.part);
-    p.wfirst = (int64_t *)(ws + lay.wfirst);
     p.wlo = (int64_t *)(ws + lay.wlo);
     p.cut = (uint8_t *)(ws + lay.cut);
     p.bar = (unsigned *)(ws + lay.bar);
