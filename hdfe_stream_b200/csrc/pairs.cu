@@ -603,7 +603,8 @@ __global__ void __launch_bounds__(kThreads) k_single(uint8_t *alive, const int64
 // after the other, instead of to one warp: a warp takes some 1.5 us per 32
 // edges, so a vertex of tens of millions would hold the grid at a barrier for
 // longer than the barrier's limit.  A hub costs a barrier a level; below the
-// bound a warp's 32 vertices take 0.1 s at most.
+// bound a warp's 32 vertices take 0.1 s at most.  Rounds without one pay for the
+// test (the 1M-worker panel's two: 1.12 -> 1.16 ms).
 constexpr int64_t kHub = 1 << 16;
 
 struct CutArgs {

@@ -40,8 +40,8 @@ namespace hdfe {
 namespace sorting {
 
 constexpr int kThreads = 256;
-constexpr int kItems = 16;              // items per thread per tile (two CTAs' tiles
-                                        // and registers still give 4 CTAs an SM)
+constexpr int kItems = 16;              // items per thread per tile (the scatter's 48 KB
+                                        // tile and 11 KB of counts: three CTAs an SM)
 constexpr int kTile = kThreads * kItems;
 constexpr int kBins = 256;
 constexpr int kWarps = kThreads / 32;

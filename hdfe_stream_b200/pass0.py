@@ -95,7 +95,8 @@ def sort_pairs(keys, vals=None, key_bits: int = 64):
 
 
 # A range of ids up to this many values an id goes through the bitmap: its words
-# then stay within 4 bytes an id, half of one radix pass's keys, and in the L2.
+# then stay within 4 bytes an id, half of one radix pass's keys (16 with the words'
+# counts and ranks, which leave the L2 from some 8M ids on).
 RANGE_PER_ID = 32
 RANGE_FREE = 1 << 20
 
