@@ -8,9 +8,10 @@ namespace rows {
 
 // ------------------------------------------------------ Rademacher passes
 //
-// What bounds these passes is instruction issue, not memory: N x B hashes and
-// FP64 updates against N rows read once.  So per (row, draw) only what depends
-// on both is left.  A sub-warp of BP lanes (lane j: draw j) takes a window of
+// What bounds these passes is instruction issue (the centring pass: 71% of
+// cycles) and, in the projection, the latency of a window's chain at 20 warps an
+// SM (52%), not memory (3 and 6% of DRAM): N x B hashes and FP64 updates against
+// N rows read once.  So per (row, draw) only what depends on both is left.  A sub-warp of BP lanes (lane j: draw j) takes a window of
 // up to 32 rows made of whole groups, stages codes, covariates and weights
 // lane-parallel in shared memory, and keeps each draw's signs of the window as
 // one 32-bit word (bit q: row q).  Then, without weights, the sum of a run or a

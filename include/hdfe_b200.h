@@ -579,7 +579,7 @@ typedef struct hdfe_pcg_info {
 
 /* Largest k (right-hand-side columns per solve) hdfe_pcg_solve accepts.
  * Blocks of up to 4 columns keep each row's k values in one thread's
- * registers; wider blocks (the JLA's probe blocks) run one column per lane,
+ * registers; wider blocks (the JLA's probe blocks) run two columns per lane,
  * padded to 8, 16 or 32 columns, so every column of the block shares one
  * pass over S per iteration. */
 #define HDFE_PCG_MAX_K 32
