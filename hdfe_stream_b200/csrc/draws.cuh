@@ -11,17 +11,18 @@ namespace rows {
 // What bounds these passes is instruction issue (the centring pass: 71% of
 // cycles) and, in the projection, the latency of a window's chain at 20 warps an
 // SM (52%), not memory (3 and 6% of DRAM): N x B hashes and FP64 updates against
-// N rows read once.  So per (row, draw) only what depends on both is left.  A sub-warp of BP lanes (lane j: draw j) takes a window of
-// up to 32 rows made of whole groups, stages codes, covariates and weights
-// lane-parallel in shared memory, and keeps each draw's signs of the window as
-// one 32-bit word (bit q: row q).  Then, without weights, the sum of a run or a
-// group is n - 2 popc(word & mask); the covariates' group sums are made once a
-// window by lane (group, covariate); and U's row of a run of equal codes is
-// gathered once, the window's first eight runs in flight during the hashing.
-// The projection stores r o per (row, draw) in a padded tile (P = (r o)^2 and
-// M = (1 - r o)^2 = (r - o)^2, r = +-1), and lane t then sums row t over the
-// draws in draw order: one flush per 32 rows rather than one per group, and
-// coalesced.  A group of more than 32 rows is walked in chunks of 32, twice.
+// N rows read once.  So per (row, draw) only what depends on both is left.  A
+// sub-warp of BP lanes (lane j: draw j) takes a window of up to 32 rows made of
+// whole groups, stages codes, covariates and weights lane-parallel in shared
+// memory, and keeps each draw's signs of the window as one 32-bit word (bit q:
+// row q).  Then, without weights, the sum of a run or a group is n - 2 popc(word
+// & mask); the covariates' group sums are made once a window by lane (group,
+// covariate); and U's row of a run of equal codes is gathered once, the window's
+// first eight runs in flight during the hashing. The projection stores r o per
+// (row, draw) in a padded tile (P = (r o)^2 and M = (1 - r o)^2 = (r - o)^2, r =
+// +-1), and lane t then sums row t over the draws in draw order: one flush per 32
+// rows rather than one per group, and coalesced.  A group of more than 32 rows is
+// walked in chunks of 32, twice.
 //
 // 1M-worker panel (8.5M rows, 2 covariates, 32 draws): center 2.15 -> 0.82 ms,
 // project with the five sums 5.30 -> 1.29 ms a block.

@@ -586,7 +586,7 @@ typedef struct hdfe_pcg_info {
 
 /* Largest k hdfe_pcg_solve_mixed accepts: blocks of up to 4 columns keep a
  * row's k values in one thread's registers, wider ones run one column per
- * lane (padded to 8, 16 or 32), as hdfe_pcg_solve does. */
+ * lane, padded to 8, 16 or 32. */
 #define HDFE_PCG_MIXED_MAX_K 32
 
 /* Device workspace bytes hdfe_pcg_solve needs (for the current device). */
