@@ -210,15 +210,23 @@ def ptr(t) -> int | None:
     return None if t is None else t.data_ptr()
 
 
+_torch_names = None         # what `is_plain` looks up in torch, bound at its first call
+
+
 def is_plain(t) -> bool:
     """Whether t is a dense tensor of values and nothing else -- no gradient to
     record, no forward derivative, no vmap level, no negation to be applied --,
     so that a kernel may take its address in place of torch operations."""
-    import torch
-    return type(t) is torch.Tensor and t.layout == torch.strided and \
-        not (t.requires_grad and torch.is_grad_enabled()) and \
-        not torch._C._functorch.is_functorch_wrapped_tensor(t) and \
-        torch.autograd.forward_ad.unpack_dual(t).tangent is None and not t.is_neg()
+    global _torch_names
+    if _torch_names is None:
+        import torch
+        _torch_names = (torch.Tensor, torch.strided, torch.is_grad_enabled,
+                        torch._C._functorch.is_functorch_wrapped_tensor,
+                        torch.autograd.forward_ad.unpack_dual)
+    Tensor, strided, recording, wrapped, unpack_dual = _torch_names
+    return type(t) is Tensor and t.layout is strided and \
+        not (t.requires_grad and recording()) and not wrapped(t) and \
+        unpack_dual(t).tangent is None and not t.is_neg()
 
 
 def stream_handle(stream=None) -> int:

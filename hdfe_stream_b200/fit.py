@@ -270,9 +270,10 @@ def solve_setup(cells: DeviceCells, stream=None):
     diag, rhs, raw_ss = cells.diag, cells.rhs, cells.raw_ss
     L, m = rhs.shape
     dev = rhs.device
-    if not all(_lib.is_plain(t) and t.dtype == torch.float64 and t.device == dev and t.is_cuda
-               and tuple(t.shape) == shape
-               for t, shape in ((diag, (L,)), (rhs, (L, m)), (raw_ss, (m,)))):
+    f64, plain = torch.float64, _lib.is_plain
+    if not (rhs.is_cuda and diag.dtype is f64 and rhs.dtype is f64 and raw_ss.dtype is f64
+            and diag.device == dev and raw_ss.device == dev and diag.shape == (L,)
+            and raw_ss.shape == (m,) and plain(diag) and plain(rhs) and plain(raw_ss)):
         # other types, sizes or devices than pass 1's: torch's rules
         scale = torch.sqrt(torch.clamp(raw_ss, min=0.0))
         zero = torch.linalg.vector_norm(rhs, dim=0) <= RHS_ZERO_TOL * scale

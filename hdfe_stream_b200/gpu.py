@@ -260,16 +260,13 @@ class BlockSolver:
             Xj = torch.empty_like(Bj) if k > width else X
             X0j = None if X0 is None else X0[:, j0:j1].to(self.dev, torch.float64).contiguous()
             zj = None if zero is None else zero[j0:j1]
-            if on_device:
-                go = lambda: self._launch(Bj, zj.data_ptr(), X0j, Xj)
-            else:
-                go = lambda: self.launch(Bj, zj, X0j, Xj)
+            go, flags = (self._launch, zj.data_ptr()) if on_device else (self.launch, zj)
             timer = getattr(self, "timer", None)
             if timer is not None:
                 with timer("pcg_kernel"):
-                    go()
+                    go(Bj, flags, X0j, Xj)
             else:
-                go()
+                go(Bj, flags, X0j, Xj)
             it, c, r = self.read_info()
             if k > width:
                 X[:, j0:j1] = Xj
