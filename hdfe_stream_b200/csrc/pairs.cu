@@ -603,8 +603,7 @@ __global__ void __launch_bounds__(kThreads) k_single(uint8_t *alive, const int64
 // after the other, instead of to one warp: a warp takes some 1.5 us per 32
 // edges, so a vertex of tens of millions would hold the grid at a barrier for
 // longer than the barrier's limit.  A hub costs a barrier a level; below the
-// bound a warp's 32 vertices take 0.1 s at most.  Rounds without one pay for the
-// test (the 1M-worker panel's two: 1.12 -> 1.16 ms).
+// bound a warp's 32 vertices take 0.1 s at most.
 constexpr int64_t kHub = 1 << 16;
 
 struct CutArgs {
@@ -615,11 +614,11 @@ struct CutArgs {
     int32_t *order;         // (n) reached vertices by depth
     int32_t *lvl;           // (n + 1) where each depth begins in order
     int32_t *hubs;          // (n + 1) reached vertices of kHub neighbours or more
-    // zeroed before the launch: three queue counters, the root's key, three hub
-    // counters
+    // zeroed before the launch: three levels' counters of queued vertices and of
+    // hubs, side by side (every warp reads both after a level's barrier; two
+    // addresses cost 2 us a level more: 1.16 ms for two rounds against 1.11), and the root's key
     unsigned *queue;
     int *root_key;          // n - the smallest alive vertex
-    unsigned *hub_queue;
     unsigned long long *removed;
     int64_t *levels;
 };
@@ -733,12 +732,12 @@ __global__ void __launch_bounds__(kCoop, 1) k_cut_round(CutArgs a)
     unsigned n_hubs = 0;                        // on the levels so far
     int level = 0;
     for (;; level++) {
-        unsigned *tail = a.queue + (level + 1) % 3, *more = a.hub_queue + (level + 1) % 3;
+        unsigned *tail = a.queue + 2 * ((level + 1) % 3);
         int32_t *next = a.order + start + count;
         if (t0 == 0) {
             a.lvl[level] = (int32_t)start;
-            a.queue[(level + 2) % 3] = 0;       // last read before the previous barrier
-            a.hub_queue[(level + 2) % 3] = 0;
+            // (last read before the previous barrier)
+            *reinterpret_cast<unsigned long long *>(a.queue + 2 * ((level + 2) % 3)) = 0;
         }
         int held = 0;
         auto flush = [&]() {
@@ -761,18 +760,21 @@ __global__ void __launch_bounds__(kCoop, 1) k_cut_round(CutArgs a)
             held += __popc(m);
             if (held >= kFull) flush();
         };
-        walk_edges(a, a.order + start, count, a.hubs + n_hubs, more, claim);
+        walk_edges(a, a.order + start, count, a.hubs + n_hubs, tail + 1, claim);
         if (held) flush();
         if (!g.sync()) return;
-        const unsigned found = *(volatile unsigned *)more;
+        const unsigned long long counts = *(volatile unsigned long long *)tail;
+        const unsigned found = (unsigned)(counts >> 32);
+        unsigned reached = (unsigned)counts;
         if (found) {                            // the same in every CTA
             walk_hubs(a, a.hubs + n_hubs, found, claim);
             if (held) flush();
             n_hubs += found;
             if (!g.sync()) return;
+            reached = *(volatile unsigned *)tail;
         }
         start += count;
-        count = *(volatile unsigned *)tail;
+        count = reached;
         if (count == 0) break;
     }
     if (t0 == 0) a.lvl[level + 1] = (int32_t)start;
@@ -955,10 +957,10 @@ struct Ctx {
     int32_t *parent;
     pairs::Graph g;
     // scalars (8 bytes each): P, ncomp, status, changed, rows kept, components before,
-    // single observations; from 8 a round's own (queue counters and root key, workers
-    // removed, the tree's depth, hub counters); at 16 the grid barrier
+    // single observations; from 8 a round's own (root key, at 10 workers removed, the
+    // tree's depth, the queue's counters); at 16 the grid barrier
     int64_t *P, *ncomp, *removed, *levels, *kept, *before, *single;
-    unsigned *status, *changed, *queue, *hub_queue;
+    unsigned *status, *changed, *queue;
     int *root_key;
     int launches = 0;
 
@@ -983,11 +985,10 @@ struct Ctx {
         kept = sc + 4;
         before = sc + 5;
         single = sc + 6;
-        queue = (unsigned *)(sc + 8);
-        root_key = (int *)(queue + 3);
+        root_key = (int *)(sc + 8);
         removed = sc + 10;
         levels = sc + 11;
-        hub_queue = (unsigned *)(sc + 12);
+        queue = (unsigned *)(sc + 12);
         g.pa = pa;
         g.pb = pb;
         g.count = count;
@@ -1177,10 +1178,10 @@ extern "C" int hdfe_leave_one_out(const uint32_t *a, const uint32_t *b, int64_t 
     // done with by then)
     CutArgs ca{c.g,  indptr, indices, depth,   tpar,    size,       pre,       low,
                high, aux,    cut,     order, (int32_t *)crow, (int32_t *)crow + n + 1, c.queue,
-               c.root_key, c.hub_queue, reinterpret_cast<unsigned long long *>(c.removed),
+               c.root_key, reinterpret_cast<unsigned long long *>(c.removed),
                c.levels};
     for (;;) {
-        HDFE_CUDA_TRY(cudaMemsetAsync(c.queue, 0, 48, s));      // through hub_queue
+        HDFE_CUDA_TRY(cudaMemsetAsync(c.root_key, 0, 56, s));   // through the queue's counters
         void *args[] = {&ca};
         if ((st = c.coop((const void *)k_cut_round, args)) != HDFE_OK) return st;
         int64_t h[2];                       // workers removed, the tree's depth
