@@ -615,8 +615,9 @@ struct CutArgs {
     int32_t *lvl;           // (n + 1) where each depth begins in order
     int32_t *hubs;          // (n + 1) reached vertices of kHub neighbours or more
     // zeroed before the launch: three levels' counters of queued vertices and of
-    // hubs, side by side (every warp reads both after a level's barrier; two
-    // addresses cost 2 us a level more: 1.16 ms for two rounds against 1.11), and the root's key
+    // hubs, side by side (every warp reads both after a level's barrier; at two
+    // addresses that cost 2 us a level: 1.16 ms for two rounds, 1.11 at one), and
+    // the root's key
     unsigned *queue;
     int *root_key;          // n - the smallest alive vertex
     unsigned long long *removed;

@@ -352,11 +352,10 @@ class InverseOperator:
     def _plain(self, levels, streamed):
         """Whether the blocks are (L, B) and (G, B) FP64 values on the
         operator's device."""
-        torch = _torch()
-        return all(_lib.is_plain(t) and t.dtype == torch.float64 and t.device == self.dev
-                   and t.dim() == 2 and t.shape[0] == n
-                   for t, n in ((levels, self.L), (streamed, self.G))) and \
-            levels.shape[1] == streamed.shape[1] > 0
+        f64, B = _torch().float64, levels.shape[-1] if levels.dim() else 0
+        return B > 0 and levels.shape == (self.L, B) and streamed.shape == (self.G, B) \
+            and levels.dtype is f64 and streamed.dtype is f64 and levels.device == self.dev \
+            and streamed.device == self.dev and _lib.is_plain(levels) and _lib.is_plain(streamed)
 
     def _drop_null_dense(self, levels, streamed):
         qs, ql = self.null_space()
